@@ -4,7 +4,7 @@
 //
 // GB300 shape of the V-cycle:
 //   * Fine levels: ONE launch per level on the way down and one on the way up.
-//     Each CTA loads its tile plus a halo into shared memory and runs all of
+//     Each CTA loads its tile plus a halo into registers and runs all of
 //     the level's red-black half-sweeps there (temporal blocking: half-sweep s
 //     is valid on the region shrunk by s+1 cells, so a halo of 2*pairs+1
 //     leaves the tile and a one-cell ring valid after the last sweep). The
@@ -107,37 +107,6 @@ __global__ void k_coarsen_labels(int fnx, int fny, const uint8_t* __restrict__ f
   coarse[I + (long)J * cnx] = air ? AIR : (fluid ? FLUID : SOLID);
 }
 
-// The red-black update of one cell from shared memory (pressureRedBlack.ts:
-// 52-66 with sum order +x, -x, +y, -y).
-__device__ __forceinline__ void rb_update(float* xs, const float* bs, uint8_t c, int s, int sw, float scale,
-                                          float omega) {
-  if ((c & 3u) != FLUID) return;
-  const int cnt = code_count(c);
-  if (cnt == 0) return;
-  float sum = 0.0f;
-  if (c & LINK_XP) sum += xs[s + 1];
-  if (c & LINK_XM) sum += xs[s - 1];
-  if (c & LINK_YP) sum += xs[s + sw];
-  if (c & LINK_YM) sum += xs[s - sw];
-  const float pgs = (sum - scale * bs[s]) / (float)cnt;
-  xs[s] = (1.0f - omega) * xs[s] + omega * pgs;
-}
-
-// r = b - (count*x - sum), 0 off-fluid (pressureMultigrid.ts:117-151).
-__device__ __forceinline__ float residual_at(const float* xs, const float* bs, uint8_t c, int s, int sw, bool& counted) {
-  counted = false;
-  if ((c & 3u) != FLUID) return 0.0f;
-  const int cnt = code_count(c);
-  if (cnt == 0) return 0.0f;
-  float sum = 0.0f;
-  if (c & LINK_XP) sum += xs[s + 1];
-  if (c & LINK_XM) sum += xs[s - 1];
-  if (c & LINK_YP) sum += xs[s + sw];
-  if (c & LINK_YM) sum += xs[s - sw];
-  counted = true;
-  return bs[s] - ((float)cnt * xs[s] - sum);
-}
-
 struct SmoothArgs {
   int nx, ny;
   const float* xin;
@@ -151,6 +120,7 @@ struct SmoothArgs {
   const float* ec;  // POST: coarse correction
   StepAccum* acc;   // POST: residual norm accumulation (may be null)
   int x_is_zero;    // PRE on a coarse level: x starts at zero (pressureMultigrid.ts:175)
+  int pairs, halo;  // sweep pairs, and the region's halo (smooth_halo)
 };
 
 // (sum - scale*b) / count with count in 1..4: a multiply by the exact
@@ -171,269 +141,337 @@ __device__ __forceinline__ float div3(float s) {
   return (s == 0.0f || fabsf(s) == __int_as_float(0x7f800000)) ? q0 : q1;
 }
 
-__device__ __forceinline__ float over_count(float s, int cnt) {
-  const float third = div3(s);
-  return cnt == 3 ? third : s * (cnt == 4 ? 0.25f : (cnt == 2 ? 0.5f : 1.0f));
+// s / count for rc = (RN(1 / count), -count), count 1..4, without a branch or
+// a test of the count: div3's steps for every count. For 1, 2 and 4 the first
+// product is the quotient, the remainder 0 and the second step changes
+// nothing. An infinite s has a NaN remainder, which fmaxf turns into a finite
+// number: the quotient then stays infinite. Equals IEEE division for every
+// float but for the sign of a zero.
+__device__ __forceinline__ float over_links(float s, float2 rc) {
+  const float q0 = __fmul_rn(s, rc.x);
+  const float r = fmaxf(__fmaf_rn(rc.y, q0, s), -3.402823466e+38f);
+  return __fmaf_rn(r, rc.x, q0);
 }
 
-// Temporally blocked red-black smoother. One 1024-thread CTA owns a 64x64
-// region: its tile plus a halo of H = 2*pairs (+1 when a residual follows).
-// Thread (tx, ty) owns the cells (2tx, ty), (2tx+1, ty), (2tx, ty+32),
-// (2tx+1, ty+32) — one of each colour per row — and keeps their stencil
-// code, rhs and value in registers for the whole launch. Neighbour values go
-// through shared memory split by local parity, xs[(li+lj)&1][lj][li>>1], so
-// a warp's reads and writes are unit-stride. Every half-sweep updates every
-// region cell of its colour except the region's outer ring: half-sweep s is
-// correct on the region shrunk by s+1 cells, so after 2*pairs half-sweeps the
-// tile (and, with the +1, a ring around it) holds exactly the values the
-// sequential sweeps produce; outer cells hold finite values nobody uses.
-// The region side R is 64 (1024 threads) on large levels and 32 (256
-// threads, more CTAs for levels too small to fill the GPU with 64^2 regions).
-template <int P, int MODE, int R>
-struct Tile {
-  static constexpr int H = (MODE == MODE_PLAIN) ? 2 * P : 2 * P + 1;
-  static constexpr int T = R - 2 * H;  // tile side, even
+// Temporally blocked red-black smoother. One CTA of NW warps owns a region of
+// 64 columns x NW * RW rows: its tile plus a halo of H cells all round (H
+// even). Lane l of a warp owns the columns 2l and 2l + 1 of the warp's RW
+// rows, value and rhs in registers for the whole launch. A cell's vertical
+// neighbours are then the same lane's registers, one horizontal neighbour is
+// the lane's other column and the other one shuffle away; only the first and
+// last row of each warp go through shared memory, one value a lane and
+// half-sweep (edge[c]: colour c's cells of those rows, written by the
+// half-sweeps of colour c and read by those of the other colour, so one
+// barrier a half-sweep orders both). The region starts at even coordinates:
+// the colour-c cell of row r is column (c + r) & 1 of the pair in every lane,
+// known at compile time, and the 2 x 2 children of a coarse cell belong to
+// one lane.
+//
+// Every half-sweep updates every updatable cell of its colour. Half-sweep s
+// is correct on the region shrunk by s + 1 cells (beyond the region's border
+// a cell sees some finite value), so a halo of 2 pairs leaves the tile with
+// exactly the values that the sequential sweeps produce, and 2 pairs + 1 a
+// ring around it for the residual (rounded up to even). From x = 0 the first
+// half-sweep sees nothing but zeros, inside the region and beyond: it is
+// correct everywhere, and 2 pairs serve the residual too (smooth_halo).
+//
+// Bound by instruction issue and, where a level has few regions, by the
+// latency of one region (load, 2 pairs half-sweeps of ~150 to 250 cycles,
+// residual). With x in shared memory instead (four loads, a store and a
+// barrier of 32 warps for every update, 4 cells a thread) the 1024^2 PRE
+// launch executed 8.9 M warp instructions, three quarters of them set-up.
+// Launches chained in a graph, before -> now: V(3,3) PRE from zero / POST at
+// 2048^2 44.3 / 45.8 -> 14.8 / 17.4 us, 1024^2 12.0 / 12.5 -> 5.8 / 6.2,
+// 512^2 4.5 / 4.7 -> 3.2 / 3.7, 256^2 3.4 / 3.5 -> 2.6 / 3.1, 64^2 2.9 / 3.1
+// -> 2.5 / 3.0; four SOR pairs at 1024^2 with obstacles 16.6 -> 8.9.
+//
+// The shapes: 8 warps of 8 rows (a 64 x 64 region) spend the fewest
+// instructions a cell; 16 warps of 2 rows (64 x 32) have the shortest chain
+// of updates a warp, for levels whose 64 x 64 regions would leave SMs idle or
+// give a few of them a second one (SMOOTH_SMALL regions): PRE at 512^2 (100
+// regions) 4.2 against 3.2 us, 640^2 (169) 4.9 against 4.2, 704^2 (196) 4.9
+// against 4.9, POST 5.4 against 5.8, 1024^2 (400) 6.1 against 7.7. 8 x 4 and
+// 16 x 4 lay between.
+constexpr long SMOOTH_SMALL = 176;
+
+template <int NW, int RW>
+struct SmoothShared {
+  float edge[2][NW + 2][2][32];        // [colour][warp + 1][first / last row][lane]; beyond the region: 0
+  float2 rc[2 * RW][32 * NW];          // (RN(1 / count), -count) of a cell's links, (0, 0) where it is not updated
+  float2 lut[64];                      // that pair for each code
 };
 
-// Loads of data an earlier phase of the same launch may have written (the
-// persistent solve): through L2 only, so that no stale L1 line is read.
-// Otherwise plain loads, and the read-only path for the coarse correction.
-template <bool COH>
-__device__ __forceinline__ float ld_coherent(const float* p) {
-  if constexpr (COH) return __ldcg(p);
-  return *p;
-}
-template <bool COH>
-__device__ __forceinline__ float ld_ro(const float* p) {
-  if constexpr (COH) return __ldcg(p);
-  return __ldg(p);
-}
+// One region of the smoother, region (bx, by) of the level; called by one
+// whole block (every thread, in step).
+template <int MODE, int NW, int RW>
+__device__ __forceinline__ void smooth_tile(const SmoothArgs& a, int bx, int by, SmoothShared<NW, RW>& sh) {
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int nx = a.nx, ny = a.ny, H = a.halo;
+  const int TX = 64 - 2 * H, TY = RW * NW - 2 * H;
+  const int col = bx * TX - H + 2 * lane;      // even
+  const int row = by * TY - H + RW * w;        // even
+  // rows of an even width start at multiples of 8 bytes, so a lane's pair is
+  // one 8-byte access (the levels' buffers come from cudaMalloc)
+  const bool pair = (nx & 1) == 0;
+  constexpr unsigned OUTSIDE2 = CODE_OUTSIDE | (unsigned)CODE_OUTSIDE << 8;
+  constexpr unsigned FULL2 = 0x3c3cu;  // two fluid cells with four links each
 
-// One region of the temporally blocked smoother, region (bx, by) of the
-// level; called by one whole block (every thread, in step).
-template <int P, int MODE, int R, bool COH>
-__device__ __forceinline__ void smooth_tile(const SmoothArgs& a, int bx, int by) {
-  constexpr int RGN = R;
-  constexpr int RGN_T = R / 2;
-  constexpr int H = Tile<P, MODE, R>::H;
-  constexpr int T = Tile<P, MODE, R>::T;
-  static_assert(T % 2 == 0 && T > 0, "tile must be even");
-  __shared__ float xs[2][RGN][RGN / 2];
-  __shared__ float rs[MODE == MODE_PRE ? RGN : 1][MODE == MODE_PRE ? RGN : 1];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int X0 = bx * T, Y0 = by * T;
-  const int GX = X0 - H, GY = Y0 - H;
-  const int nx = a.nx, ny = a.ny;
-
-  uint8_t cd[2][2];
-  float bb[2][2], xx[2][2];
+  float x[RW][2], b[RW][2];
+  unsigned cd[RW];  // the two cells' codes
 #pragma unroll
-  for (int r = 0; r < 2; r++) {
-    const int lj = ty + RGN_T * r;
-    const int gj = GY + lj;
-#pragma unroll
-    for (int o = 0; o < 2; o++) {
-      const int li = 2 * tx + o;
-      const int gi = GX + li;
-      if ((unsigned)gi < (unsigned)nx && (unsigned)gj < (unsigned)ny) {
-        // 32-bit offsets: a level holds fewer than 2^31 cells (the engine's
-        // grid limits)
-        const int k = gi + gj * nx;
-        cd[r][o] = a.code[k];
-        bb[r][o] = ld_coherent<COH>(a.b + k);
-        xx[r][o] = a.x_is_zero ? 0.0f : ld_coherent<COH>(a.xin + k);
+  for (int r = 0; r < RW; r++) {
+    const int gj = row + r;
+    cd[r] = OUTSIDE2;
+    x[r][0] = x[r][1] = b[r][0] = b[r][1] = 0.0f;
+    if ((unsigned)gj < (unsigned)ny) {
+      const int k = col + gj * nx;  // 32-bit offsets: a level holds fewer than 2^31 cells
+      if (pair) {
+        if ((unsigned)col < (unsigned)nx) {
+          cd[r] = *reinterpret_cast<const unsigned short*>(a.code + k);
+          const float2 q = *reinterpret_cast<const float2*>(a.b + k);
+          b[r][0] = q.x;
+          b[r][1] = q.y;
+          if (!a.x_is_zero) {
+            const float2 p = *reinterpret_cast<const float2*>(a.xin + k);
+            x[r][0] = p.x;
+            x[r][1] = p.y;
+          }
+        }
       } else {
-        cd[r][o] = CODE_OUTSIDE;
-        bb[r][o] = 0.0f;
-        xx[r][o] = 0.0f;
+#pragma unroll
+        for (int o = 0; o < 2; o++)
+          if ((unsigned)(col + o) < (unsigned)nx) {
+            cd[r] = (cd[r] & (o ? 0x00ffu : 0xff00u)) | (unsigned)a.code[k + o] << (8 * o);
+            b[r][o] = a.b[k + o];
+            if (!a.x_is_zero) x[r][o] = a.xin[k + o];
+          }
       }
     }
-    if constexpr (MODE == MODE_POST) {
-      // pressureMultigrid.ts:192-207 — a fluid cell's x += 9/16, 3/16, 3/16,
-      // 1/16 of e at coarse columns (I, I2) and rows (J, J2), I = i >> 1, I2
-      // = I + 1 (odd i, clamped) or I - 1 (even i, clamped). The row's two
-      // cells are the odd column GX + 2tx (H is odd, T even) and the even one
-      // after it, so both read coarse columns A = max(I, 0) and B = min(I +
-      // 1, cnx - 1) of I = (GX + 2tx - 1) / 2: the odd cell as (I, I2) =
-      // (A, B), the even one as (B, A). Four loads serve the two cells.
-      // The loads do not wait for the codes: on rows inside the grid they
-      // run for every pair, at columns clamped into the coarse level (the
-      // clamps change nothing for a pair with a cell in the grid).
-      static_assert(H % 2 == 1, "the prolongation pairs an odd column with the even one after it");
-      if ((unsigned)gj < (unsigned)ny) {
-        const int I = (GX + 2 * tx - 1) / 2;
-        const int A = min(max(I, 0), a.cnx - 1), B = max(min(I + 1, a.cnx - 1), 0);
-        const int J = gj >> 1;
-        const int J2 = (gj & 1) ? min(J + 1, a.cny - 1) : max(J - 1, 0);
-        const float* e = a.ec;
-        const int cs = a.cnx;
-        const float eAJ = ld_ro<COH>(e + A + J * cs), eBJ = ld_ro<COH>(e + B + J * cs);
-        const float eAJ2 = ld_ro<COH>(e + A + J2 * cs), eBJ2 = ld_ro<COH>(e + B + J2 * cs);
-        if ((cd[r][0] & 3u) == FLUID) xx[r][0] += 0.5625f * eAJ + 0.1875f * (eBJ + eAJ2) + 0.0625f * eBJ2;
-        if ((cd[r][1] & 3u) == FLUID) xx[r][1] += 0.5625f * eBJ + 0.1875f * (eAJ + eBJ2) + 0.0625f * eAJ2;
-      }
+  }
+  if constexpr (MODE == MODE_POST) {
+    // pressureMultigrid.ts:192-207 — a fluid cell's x += 9/16, 3/16, 3/16,
+    // 1/16 of e at coarse columns (I, I2) and rows (J, J2), I = i >> 1, I2 =
+    // I + 1 (odd i) or I - 1 (even i), clamped. The pair of columns 2m, 2m+1
+    // reads coarse columns m-1, m, m+1: each lane loads its m, the others
+    // come by shuffle (the first and last lane load theirs). The 8 rows read
+    // 6 coarse rows. The clamps change nothing for a cell in the grid.
+    const int m = col >> 1, J0 = row >> 1;
+    const int cm = min(max(m, 0), a.cnx - 1);
+    const int ce = min(max(lane == 0 ? m - 1 : m + 1, 0), a.cnx - 1);
+    const bool end = lane == 0 || lane == 31;
+    float eL[RW / 2 + 2], eM[RW / 2 + 2], eR[RW / 2 + 2];  // coarse rows J0 - 1 .. J0 + RW / 2
+#pragma unroll
+    for (int q = 0; q < RW / 2 + 2; q++) {
+      const float* e = a.ec + min(max(J0 - 1 + q, 0), a.cny - 1) * a.cnx;
+      eM[q] = __ldg(e + cm);
+      eL[q] = end ? __ldg(e + ce) : 0.0f;
     }
 #pragma unroll
-    for (int o = 0; o < 2; o++) {
-      // Solid cells (and cells outside the grid) are exactly the neighbours
-      // no link points to; they hold +0.0 in shared memory (their own value
-      // stays in xx), so that a sweep can add all four neighbours without a
-      // test: an unlinked one adds +0.0, which leaves the sum's bits
-      // unchanged (a sum that starts at +0.0 never becomes -0.0).
-      xs[(2 * tx + o + lj) & 1][lj][tx] = (cd[r][o] & 3u) == SOLID ? 0.0f : xx[r][o];
+    for (int q = 0; q < RW / 2 + 2; q++) {
+      const float l = __shfl_up_sync(0xffffffffu, eM[q], 1), r = __shfl_down_sync(0xffffffffu, eM[q], 1);
+      eR[q] = lane == 31 ? eL[q] : r;
+      eL[q] = lane == 0 ? eL[q] : l;
     }
+#pragma unroll
+    for (int r = 0; r < RW; r++) {
+      const int q = 1 + r / 2, f = (r & 1) ? q + 1 : q - 1;  // an even row leans on the coarse row below, an odd one above
+      const float p0 = 0.5625f * eM[q] + 0.1875f * (eL[q] + eM[f]) + 0.0625f * eL[f];
+      const float p1 = 0.5625f * eM[q] + 0.1875f * (eR[q] + eM[f]) + 0.0625f * eR[f];
+      const float x0 = x[r][0] + p0, x1 = x[r][1] + p1;
+      x[r][0] = (cd[r] & 3u) == FLUID ? x0 : x[r][0];
+      x[r][1] = (cd[r] & 0x300u) == 0u ? x1 : x[r][1];
+    }
+  }
+
+  // code -> (RN(1 / count), -count) (pressureRedBlack.ts:52-66 updates fluid
+  // cells with a link only)
+  if (tid < 64) {
+    const int cnt = code_count((uint8_t)tid);
+    const bool on = (tid & 3) == FLUID && cnt > 0;
+    sh.lut[tid] = make_float2(on ? 1.0f / (float)cnt : 0.0f, on ? -(float)cnt : 0.0f);
+  }
+  if (w == 0) {
+    sh.edge[0][0][1][lane] = sh.edge[1][0][1][lane] = 0.0f;
+    sh.edge[0][NW + 1][0][lane] = sh.edge[1][NW + 1][0][lane] = 0.0f;
   }
   __syncthreads();
 
-  const float scale = a.scale_dev ? *a.scale_dev : a.scale, omega = a.omega, keep = 1.0f - omega;
-  {
-    // Colour view of the thread's cells: in row r the colour-c cell is
-    // column 2tx + oc[c] (the same for both rows), kept in registers with
-    // what its updates need precomputed once: whether it is updated at all
-    // (fluid, linked, off the region's outer ring), scale*b, the exact
-    // reciprocal of its link count (0 marks a count of 3: true division).
-    const int g = (GX + GY) & 1;
-    int oc[2];
-    oc[0] = (g + ty) & 1;
-    oc[1] = 1 - oc[0];
-    bool act[2][2];
-    float sb[2][2], rc[2][2], xc[2][2];
+  // the warp's form: every cell fluid with four links, or not (then its
+  // cells' link counts go to shared memory, and the update has no branches:
+  // a lane-divergent one in each of its cells cost ~100 cycles an update)
+  unsigned odd = 0u;
 #pragma unroll
-    for (int r = 0; r < 2; r++)
+  for (int r = 0; r < RW; r++) odd |= cd[r] ^ FULL2;
+  const bool full = __all_sync(0xffffffffu, odd == 0u);
+  if (!full) {
 #pragma unroll
-      for (int c = 0; c < 2; c++) {
-        const int o = oc[c];
-        const int lj = ty + RGN_T * r, li = 2 * tx + o;
-        const uint8_t code = o ? cd[r][1] : cd[r][0];
-        const int cnt = code_count(code);
-        act[r][c] = li != 0 && li != RGN - 1 && lj != 0 && lj != RGN - 1 && (code & 3u) == FLUID && cnt > 0;
-        sb[r][c] = scale * (o ? bb[r][1] : bb[r][0]);
-        rc[r][c] = cnt == 4 ? 0.25f : (cnt == 2 ? 0.5f : (cnt == 1 ? 1.0f : 0.0f));
-        xc[r][c] = o ? xx[r][1] : xx[r][0];
-      }
-    // With omega = 1 (the multigrid's relaxation) the blend (1 - omega) x +
-    // omega pGS is pGS for every finite x, up to the sign of an exact zero
-    // (0 x + (-0) is +0), which compares equal: the sweeps then skip it.
-    auto sweeps = [&](auto unit) {
-      constexpr bool UNIT = decltype(unit)::value;
-#pragma unroll
-      for (int hs = 0; hs < 2 * P; hs++) {
-        const int c = hs & 1;
-        const int q = c ^ g;  // local parity plane of colour c
-        const float(*xo)[RGN / 2] = xs[1 - q];
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-          if (!act[r][c]) continue;
-          const int lj = ty + RGN_T * r;
-          const int o = oc[c];
-          float sum = 0.0f;
-          sum += xo[lj][tx + o];
-          sum += xo[lj][tx + o - 1];
-          sum += xo[lj + 1][tx];
-          sum += xo[lj - 1][tx];
-          const float d = sum - sb[r][c];
-          const float third = div3(d);
-          const float pgs = rc[r][c] != 0.0f ? d * rc[r][c] : third;
-          const float nv = UNIT ? pgs : keep * xc[r][c] + omega * pgs;
-          xc[r][c] = nv;
-          xs[q][lj][tx] = nv;
-        }
-        __syncthreads();
-      }
-    };
-    if (omega == 1.0f)
-      sweeps(std::true_type{});
-    else
-      sweeps(std::false_type{});
-#pragma unroll
-    for (int r = 0; r < 2; r++) {
-      xx[r][0] = oc[0] == 0 ? xc[r][0] : xc[r][1];
-      xx[r][1] = oc[0] == 0 ? xc[r][1] : xc[r][0];
-    }
-  }
-
-  if (MODE == MODE_PRE || (MODE == MODE_POST && a.acc != nullptr)) {
-    double rsq = 0.0;
-    unsigned long long rn = 0;
-#pragma unroll
-    for (int r = 0; r < 2; r++) {
-      const int lj = ty + RGN_T * r;
+    for (int r = 0; r < RW; r++)
 #pragma unroll
       for (int o = 0; o < 2; o++) {
-        const int li = 2 * tx + o;
-        if ((unsigned)(li - H) >= (unsigned)T || (unsigned)(lj - H) >= (unsigned)T) continue;
-        const uint8_t c = cd[r][o];
-        float res = 0.0f;
-        if ((c & 3u) == FLUID) {
-          const int cnt = code_count(c);
-          if (cnt > 0) {
-            // r = b - (count*x - sum), sum order +x, -x, +y, -y (pressureMultigrid.ts:117-151);
-            // every neighbour read, an unlinked one being +0.0 (as in the sweeps)
-            const float(*xq)[RGN / 2] = xs[1 - ((li + lj) & 1)];
-            float sum = 0.0f;
-            sum += xq[lj][tx + o];
-            sum += xq[lj][tx + o - 1];
-            sum += xq[lj + 1][tx];
-            sum += xq[lj - 1][tx];
-            res = bb[r][o] - ((float)cnt * xx[r][o] - sum);
-            rsq = fma(f2d_exact(res), f2d_exact(res), rsq);
+        const unsigned c = cd[r] >> (8 * o) & 0x3fu;
+        sh.rc[2 * r + o][tid] = sh.lut[c];
+        // Solid cells (and cells outside the grid) are exactly the
+        // neighbours no link points to: they hold +0.0, so that a sum adds
+        // all four neighbours without a test (x + 0.0 is x, but for the sign
+        // of an exact zero). A solid cell's own value is written back from xin.
+        x[r][o] = (c & 3u) == SOLID ? 0.0f : x[r][o];
+      }
+  }
+  const float scale = MODE == MODE_PLAIN && a.scale_dev ? *a.scale_dev : a.scale;
+  if constexpr (MODE == MODE_PLAIN) {
+#pragma unroll
+    for (int r = 0; r < RW; r++) {
+      b[r][0] = scale * b[r][0];
+      b[r][1] = scale * b[r][1];
+    }
+  }
+  // colour c in the warp's first row (even) is column c, in its last (odd) column 1 - c
+  auto publish = [&](int c) {
+    sh.edge[c][w + 1][0][lane] = x[0][c];
+    sh.edge[c][w + 1][1][lane] = x[RW - 1][1 - c];
+  };
+  publish(0);
+  publish(1);
+  __syncthreads();
+
+  const float omega = a.omega, keep = 1.0f - omega;
+  // With omega = 1 (the multigrid's relaxation) the blend (1 - omega) x +
+  // omega pGS is pGS for every finite x, up to the sign of an exact zero
+  // (0 x + (-0) is +0), which compares equal: the sweeps then skip it.
+  auto half_sweep = [&](auto unit, auto colour) {
+    constexpr bool UNIT = decltype(unit)::value;
+    constexpr int c = decltype(colour)::value;
+    const float above = sh.edge[1 - c][w + 2][0][lane], below = sh.edge[1 - c][w][1][lane];
+    // pressureRedBlack.ts:52-66, sum order +x, -x, +y, -y
+    auto rhs = [&](int r, int o) {
+      const float own = x[r][1 - o];
+      const float far = o == 0 ? __shfl_up_sync(0xffffffffu, own, 1) : __shfl_down_sync(0xffffffffu, own, 1);
+      float sum = o == 0 ? own + far : far + own;
+      sum += r < RW - 1 ? x[r + 1][o] : above;
+      sum += r > 0 ? x[r - 1][o] : below;
+      // the multigrid's scale is -1: sum - (-1) b
+      return MODE == MODE_PLAIN ? sum - b[r][o] : sum + b[r][o];
+    };
+    if (full) {
+#pragma unroll
+      for (int r = 0; r < RW; r++) {
+        const int o = (c + r) & 1;
+        const float pgs = rhs(r, o) * 0.25f;
+        x[r][o] = UNIT ? pgs : keep * x[r][o] + omega * pgs;
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < RW; r++) {
+        const int o = (c + r) & 1;
+        const float2 rc = sh.rc[2 * r + o][tid];
+        const float pgs = over_links(rhs(r, o), rc);
+        const float nv = UNIT ? pgs : keep * x[r][o] + omega * pgs;
+        x[r][o] = rc.x != 0.0f ? nv : x[r][o];
+      }
+    }
+    publish(c);
+    __syncthreads();
+  };
+  auto sweeps = [&](auto unit) {
+#pragma unroll 1
+    for (int k = 0; k < a.pairs; k++) {
+      half_sweep(unit, std::integral_constant<int, 0>{});
+      half_sweep(unit, std::integral_constant<int, 1>{});
+    }
+  };
+  if (omega == 1.0f)
+    sweeps(std::true_type{});
+  else
+    sweeps(std::false_type{});
+
+  // the tile's cells of this thread: all columns of the pair, rows lo..hi-1
+  const bool mine = lane >= H / 2 && lane < 32 - H / 2;
+  const int lo = max(H - RW * w, 0), hi = min(min(RW * NW - H - RW * w, RW), ny - row);
+
+  if (MODE == MODE_PRE || (MODE == MODE_POST && a.acc != nullptr)) {
+    // r = b - (count*x - sum), 0 off-fluid (pressureMultigrid.ts:117-151), as
+    // b + (-count*x + sum): every operation the negation of the same rounding
+    double rsq = 0.0;
+    unsigned long long rn = 0;
+    auto residuals = [&](auto four) {
+      constexpr bool FOUR = decltype(four)::value;
+      [[maybe_unused]] float even = 0.0f;  // the even row's two residuals, summed
+#pragma unroll
+      for (int r = 0; r < RW; r++) {
+        float res[2];
+        const float left = __shfl_up_sync(0xffffffffu, x[r][1], 1), right = __shfl_down_sync(0xffffffffu, x[r][0], 1);
+#pragma unroll
+        for (int o = 0; o < 2; o++) {
+          float sum = o == 0 ? x[r][1] + left : right + x[r][0];
+          sum += r < RW - 1 ? x[r + 1][o] : sh.edge[o][w + 2][0][lane];
+          sum += r > 0 ? x[r - 1][o] : sh.edge[1 - o][w][1][lane];
+          const float n = FOUR ? -4.0f : sh.rc[2 * r + o][tid].y;
+          const float v = b[r][o] + (n * x[r][o] + sum);
+          res[o] = FOUR || n != 0.0f ? v : 0.0f;
+          if (MODE == MODE_POST && (FOUR || n != 0.0f) && mine && r >= lo && r < hi) {
+            const double d = f2d_exact(res[o]);
+            rsq = fma(d, d, rsq);
             rn += 1;
           }
         }
-        if (MODE == MODE_PRE) rs[lj][li] = res;
-      }
-    }
-    if (MODE == MODE_PRE) {
-      __syncthreads();
-      // pressureMultigrid.ts:156-178: coarse b = sum of the children's
-      // residuals; tiles start at even coordinates, so all children of the
-      // tile's coarse cells are tile cells.
-      const int t = tx + RGN_T * ty;
-      if (t < (T / 2) * (T / 2)) {
-        const int cj = t / (T / 2), ci = t - cj * (T / 2);
-        const int I = (X0 >> 1) + ci, J = (Y0 >> 1) + cj;
-        if (I < a.cnx && J < a.cny) {
-          float sum = 0.0f;
-          for (int dj = 0; dj < 2; dj++)
-            for (int di = 0; di < 2; di++) {
-              const int i = 2 * I + di, j = 2 * J + dj;
-              if (i < nx && j < ny) sum += rs[j - GY][i - GX];
-            }
-          a.bc[I + J * a.cnx] = sum;
+        if constexpr (MODE == MODE_PRE) {
+          // pressureMultigrid.ts:156-178: coarse b = sum of the children's
+          // residuals (a child outside the grid is 0)
+          if ((r & 1) == 0) {
+            even = res[0] + res[1];
+          } else {
+            const float sum = (even + res[0]) + res[1];
+            const int I = col >> 1, J = (row + r) >> 1;
+            if (mine && r >= lo && r - 1 < hi && I < a.cnx) a.bc[I + J * a.cnx] = sum;
+          }
         }
       }
-    } else {
+    };
+    if (full)
+      residuals(std::true_type{});
+    else
+      residuals(std::false_type{});
+    if constexpr (MODE == MODE_POST) {
       __shared__ double red[32];
       __shared__ unsigned long long redn[32];
       const double bsum = block_sum(rsq, red);
       const unsigned long long bn = block_sum_u64(rn, redn);
-      if (tx == 0 && ty == 0) {
+      if (tid == 0) {
         atomicAdd(&a.acc->res_sq, bsum);
         atomicAdd(&a.acc->n_res, bn);
       }
     }
   }
 
-  if (a.xout != nullptr) {
+  if (a.xout == nullptr || !mine) return;
 #pragma unroll
-    for (int r = 0; r < 2; r++) {
-      const int lj = ty + RGN_T * r;
-      const int gj = GY + lj;
-      if (lj < H || lj >= H + T || gj >= ny) continue;
+  for (int r = 0; r < RW; r++) {
+    if (r < lo || r >= hi) continue;
+    const int k = col + (row + r) * nx;
+    if (!full && !a.x_is_zero) {
 #pragma unroll
-      for (int o = 0; o < 2; o++) {
-        const int li = 2 * tx + o;
-        const int gi = GX + li;
-        if (li < H || li >= H + T || gi >= nx) continue;
-        a.xout[gi + gj * nx] = xx[r][o];
-      }
+      for (int o = 0; o < 2; o++)
+        if ((cd[r] >> (8 * o) & 3u) == SOLID && col + o < nx) x[r][o] = a.xin[k + o];
+    }
+    if (pair) {
+      if (col < nx) *reinterpret_cast<float2*>(a.xout + k) = make_float2(x[r][0], x[r][1]);
+    } else {
+      if (col < nx) a.xout[k] = x[r][0];
+      if (col + 1 < nx) a.xout[k + 1] = x[r][1];
     }
   }
 }
 
-template <int P, int MODE, int R>
-__global__ void __launch_bounds__(R* R / 4, R == 64 ? 1 : 4) k_smooth(SmoothArgs a) {
-  smooth_tile<P, MODE, R, false>(a, blockIdx.x, blockIdx.y);
+// The halo (even) that leaves the tile correct: see smooth_tile.
+__host__ __device__ static int smooth_halo(int mode, int pairs, bool x_is_zero, bool residual) {
+  if (mode == MODE_PRE && x_is_zero) return 2 * pairs;
+  return mode == MODE_PRE || residual ? 2 * pairs + 2 : 2 * pairs;
+}
+
+template <int MODE, int NW, int RW>
+__global__ void __launch_bounds__(32 * NW, RW == 8 ? 24 / NW : 32 / NW) k_smooth(SmoothArgs a) {
+  __shared__ SmoothShared<NW, RW> sh;
+  smooth_tile<MODE, NW, RW>(a, blockIdx.x, blockIdx.y, sh);
 }
 
 // ----------------------------------------------------- single-CTA coarse tail
@@ -1186,43 +1224,20 @@ __global__ void k_rb_halfsweep(int nx, int ny, float* __restrict__ p, const floa
 
 // ------------------------------------------------------------- host side
 
-template <int P, int MODE, int R>
-static void launch_smooth_r(cudaStream_t s, const SmoothArgs& a) {
-  constexpr int T = Tile<P, MODE, R>::T;
-  dim3 blk(R / 2, R / 2);
-  dim3 grd((a.nx + T - 1) / T, (a.ny + T - 1) / T);
-  k_smooth<P, MODE, R><<<grd, blk, 0, s>>>(a);
+template <int MODE, int NW, int RW>
+static void launch_smooth_nw(cudaStream_t s, const SmoothArgs& a) {
+  const int tx = 64 - 2 * a.halo, ty = RW * NW - 2 * a.halo;
+  k_smooth<MODE, NW, RW><<<dim3((a.nx + tx - 1) / tx, (a.ny + ty - 1) / ty), 32 * NW, 0, s>>>(a);
 }
 
-// 64^2 regions unless they would leave most SMs idle: below 64 such CTAs
-// (levels of about 400^2 and smaller) the 32^2 regions' extra CTAs win over
-// their larger halo share (measured: 256^2 and 128^2 faster, 512^2 slower).
-template <int P, int MODE>
-static void launch_smooth_t(cudaStream_t s, const SmoothArgs& a) {
-  constexpr int T = Tile<P, MODE, 64>::T;
-  const long blocks64 = (long)((a.nx + T - 1) / T) * ((a.ny + T - 1) / T);
-  if (blocks64 < 64)
-    launch_smooth_r<P, MODE, 32>(s, a);
-  else
-    launch_smooth_r<P, MODE, 64>(s, a);
-}
-
-template <int MODE>
-static bool launch_smooth_p(cudaStream_t s, const SmoothArgs& a, int pairs) {
-  switch (pairs) {
-    case 0: if (MODE != MODE_PLAIN) { launch_smooth_t<0, MODE>(s, a); return true; } return false;
-    case 1: launch_smooth_t<1, MODE>(s, a); return true;
-    case 2: launch_smooth_t<2, MODE>(s, a); return true;
-    case 3: launch_smooth_t<3, MODE>(s, a); return true;
-    case 4: launch_smooth_t<4, MODE>(s, a); return true;
-    default: return false;
-  }
-}
-
-static bool launch_smooth(cudaStream_t s, const SmoothArgs& a, int pairs, int mode) {
-  if (mode == MODE_PLAIN) return launch_smooth_p<MODE_PLAIN>(s, a, pairs);
-  if (mode == MODE_PRE) return launch_smooth_p<MODE_PRE>(s, a, pairs);
-  return launch_smooth_p<MODE_POST>(s, a, pairs);
+static void launch_smooth(cudaStream_t s, SmoothArgs a, int pairs, int mode) {
+  a.pairs = pairs;
+  a.halo = smooth_halo(mode, pairs, a.x_is_zero, a.acc != nullptr);
+  const int t = 64 - 2 * a.halo;
+  const bool small = (long)((a.nx + t - 1) / t) * ((a.ny + t - 1) / t) < SMOOTH_SMALL;
+  if (mode == MODE_PLAIN) small ? launch_smooth_nw<MODE_PLAIN, 16, 2>(s, a) : launch_smooth_nw<MODE_PLAIN, 8, 8>(s, a);
+  else if (mode == MODE_PRE) small ? launch_smooth_nw<MODE_PRE, 16, 2>(s, a) : launch_smooth_nw<MODE_PRE, 8, 8>(s, a);
+  else small ? launch_smooth_nw<MODE_POST, 16, 2>(s, a) : launch_smooth_nw<MODE_POST, 8, 8>(s, a);
 }
 
 void launch_build_codes(cudaStream_t s, int nx, int ny, const uint8_t* label, uint8_t* code, const int* only_if) {
@@ -1608,6 +1623,7 @@ struct BatchSolve {
   int* lists = nullptr;          // device: base, count, act_scene, act_pre, act_n, act_total
   BatchPlan plan{};
   std::vector<int> max_items;    // per cycle phase: all scenes' items (the grid's bound)
+  std::vector<char> small;       // per cycle phase: its smoother items are the 64 x 32 regions
   std::pair<int, int> init_ph{0, 0}, zero_ph{0, 0};  // prologue defect pass, p = 0 fill: every scene
 };
 
@@ -1659,8 +1675,9 @@ __device__ void batch_compact(const BatchPlan& P) {
   }
 }
 
-template <int P, int MODE>
-__global__ void __launch_bounds__(1024, 1) k_batch_smooth(BatchPlan plan, int ph) {
+template <int MODE, int NW, int RW>
+__global__ void __launch_bounds__(32 * NW, RW == 8 ? 24 / NW : 32 / NW) k_batch_smooth(BatchPlan plan, int ph, int pairs) {
+  __shared__ SmoothShared<NW, RW> sh;
   for (int i = blockIdx.x;; i += gridDim.x) {
     BatchItem it;
     if (!batch_item(plan, ph, i, it)) return;  // the same for the whole block
@@ -1690,7 +1707,9 @@ __global__ void __launch_bounds__(1024, 1) k_batch_smooth(BatchPlan plan, int ph
       a.ec = C.x0;
       a.acc = l == 0 && !S.mixed ? S.acc : nullptr;
     }
-    smooth_tile<P, MODE, 64, false>(a, it.bx, it.by);
+    a.pairs = pairs;
+    a.halo = smooth_halo(MODE, pairs, a.x_is_zero, a.acc != nullptr);
+    smooth_tile<MODE, NW, RW>(a, it.bx, it.by, sh);
     __syncthreads();  // the next region reuses the shared tiles
   }
 }
@@ -1834,11 +1853,42 @@ BatchSolve* batch_solve_create(const std::vector<Engine*>& es_in, std::string& w
     count[(size_t)ph * n + k] = (int)items.size() - base[(size_t)ph * n + k];
     b->max_items[ph] += count[(size_t)ph * n + k];
   };
-  auto smooth_items = [&](int k, int l, int halo) {
-    const int T = 64 - 2 * halo;
-    const BatchLevel& L = hs[k].lv[l];
-    for (int by = 0; by < (L.ny + T - 1) / T; by++)
-      for (int bx = 0; bx < (L.nx + T - 1) / T; bx++) items.push_back(BatchItem{k, l, bx, by});
+  // the level scene k smooths in phase ph (-1: none) and its region's halo;
+  // PRE: level lc_k - depth + d at phase d (the tails aligned); POST: level
+  // lc_k - 1 - d at phase depth + 1 + d
+  auto smooth_level = [&](int ph, int k, int* halo) {
+    const bool pre = ph < depth;
+    const int l = pre ? hs[k].lc - depth + ph : hs[k].lc - 1 - (ph - depth - 1);
+    *halo = pre ? smooth_halo(MODE_PRE, b->pre, l > 0 || hs[k].mixed, false)
+                : smooth_halo(MODE_POST, b->post, false, l == 0 && !hs[k].mixed);
+    return l;
+  };
+  auto regions = [&](int k, int l, int halo, int rows, int* gx, int* gy) {
+    const int tx = 64 - 2 * halo, ty = rows - 2 * halo;
+    *gx = (hs[k].lv[l].nx + tx - 1) / tx;
+    *gy = (hs[k].lv[l].ny + ty - 1) / ty;
+  };
+  // a phase's regions as launch_smooth chooses them, for all its scenes together
+  b->small.assign(nph, 0);
+  for (int ph = 0; ph < 2 * depth + 1; ph++) {
+    if (ph == depth) continue;
+    long total = 0;
+    for (int k = 0; k < n; k++) {
+      int halo, gx, gy;
+      const int l = smooth_level(ph, k, &halo);
+      if (l < 0) continue;
+      regions(k, l, halo, 64, &gx, &gy);
+      total += (long)gx * gy;
+    }
+    b->small[ph] = total < SMOOTH_SMALL;
+  }
+  auto smooth_items = [&](int ph, int k) {
+    int halo, gx, gy;
+    const int l = smooth_level(ph, k, &halo);
+    if (l < 0) return;
+    regions(k, l, halo, b->small[ph] ? 32 : 64, &gx, &gy);
+    for (int by = 0; by < gy; by++)
+      for (int bx = 0; bx < gx; bx++) items.push_back(BatchItem{k, l, bx, by});
   };
   auto defect_items = [&](int k) {
     const BatchLevel& L = hs[k].lv[0];
@@ -1847,17 +1897,9 @@ BatchSolve* batch_solve_create(const std::vector<Engine*>& es_in, std::string& w
       for (int bx = 0; bx < (L.nx + 29) / 30; bx++) items.push_back(BatchItem{k, 0, bx, by});
   };
   for (int k = 0; k < n; k++) {
-    // PRE: level lc_k - depth + d at phase d (the tails aligned); POST: level
-    // lc_k - 1 - d at phase depth + 1 + d
-    for (int d = 0; d < depth; d++) {
-      const int l = hs[k].lc - depth + d;
-      if (l >= 0) add(d, k, [&] { smooth_items(k, l, 2 * b->pre + 1); });
-    }
+    for (int ph = 0; ph < depth; ph++) add(ph, k, [&] { smooth_items(ph, k); });
     add(depth, k, [&] { items.push_back(BatchItem{k, hs[k].lc, 0, 0}); });
-    for (int d = 0; d < depth; d++) {
-      const int l = hs[k].lc - 1 - d;
-      if (l >= 0) add(depth + 1 + d, k, [&] { smooth_items(k, l, 2 * b->post + 1); });
-    }
+    for (int ph = depth + 1; ph < 2 * depth + 1; ph++) add(ph, k, [&] { smooth_items(ph, k); });
     if (hs[k].mixed) add(2 * depth + 1, k, [&] { defect_items(k); });
   }
   b->init_ph.first = (int)items.size();
@@ -1922,14 +1964,10 @@ static unsigned phase_grid(const BatchSolve& b, int ph, int per_sm) {
 template <int MODE>
 static void launch_batch_smooth(cudaStream_t s, const BatchSolve& b, int pairs, int ph) {
   if (b.max_items[ph] == 0) return;
-  const dim3 blk(32, 32), g(phase_grid(b, ph, 1));
-  switch (pairs) {
-    case 0: k_batch_smooth<0, MODE><<<g, blk, 0, s>>>(b.plan, ph); break;
-    case 1: k_batch_smooth<1, MODE><<<g, blk, 0, s>>>(b.plan, ph); break;
-    case 2: k_batch_smooth<2, MODE><<<g, blk, 0, s>>>(b.plan, ph); break;
-    case 3: k_batch_smooth<3, MODE><<<g, blk, 0, s>>>(b.plan, ph); break;
-    default: k_batch_smooth<4, MODE><<<g, blk, 0, s>>>(b.plan, ph); break;
-  }
+  if (b.small[ph])
+    k_batch_smooth<MODE, 16, 2><<<phase_grid(b, ph, 2), 512, 0, s>>>(b.plan, ph, pairs);
+  else
+    k_batch_smooth<MODE, 8, 8><<<phase_grid(b, ph, 3), 256, 0, s>>>(b.plan, ph, pairs);
 }
 
 // The whole batched solve, enqueued on `s` while it is being captured: the
