@@ -52,7 +52,7 @@ struct Engine {
 
   std::vector<Level> levels;  // levels[0].x[0] is the resident pressure
   int coarse_level = 0;       // first level solved inside the single-CTA kernel
-  size_t coarse_smem = 0;
+  uint16_t* tail_codes = nullptr;  // its levels' codes in the order its lanes read them
 
   // float64 pressure of the defect-correction solve (fl_params.mixed):
   // p64[ctl->par] is the pressure, r32 the float residual fed to each V-cycle.
@@ -281,8 +281,7 @@ void launch_rb_sweeps(cudaStream_t s, int nx, int ny, const float* x_in, float* 
                       const uint8_t* code, float scale, float omega, int pairs, const float* scale_dev = nullptr);
 void launch_rms_remaining(cudaStream_t s, int nx, int ny, const float* p, const float* div, const uint8_t* code,
                           float scale, StepAccum* acc);
-void launch_build_codes(cudaStream_t s, int nx, int ny, const uint8_t* label, uint8_t* code,
-                        const int* only_if = nullptr);
+void launch_build_codes(cudaStream_t s, int nx, int ny, const uint8_t* label, uint8_t* code);
 // cur = in, raising *flag when any of the n labels changed
 void launch_label_sync(cudaStream_t s, const uint8_t* in, uint8_t* cur, long n, int* flag);
 // the conditional `h` = (*flag != 0), then *flag = 0

@@ -20,7 +20,6 @@
 //   * Labels become one byte per cell of stencil links (fl_common.cuh), built
 //     per level when labels change (pressureMultigrid.ts:302-310 rebuilt them
 //     every solve; stepGpu.ts:498 only on change, as here).
-#include <mutex>
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -35,20 +34,42 @@ constexpr int MAX_LEVELS = 24;
 
 // ------------------------------------------------------------ label codes
 
-// only_if (when set): the kernel does nothing unless *only_if is nonzero
-__global__ void k_build_codes(int nx, int ny, const uint8_t* __restrict__ label, uint8_t* __restrict__ code,
-                              const int* only_if) {
-  if (only_if != nullptr && *only_if == 0) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= nx || j >= ny) return;
-  const long k = i + (long)j * nx;
-  uint8_t c = label[k] & 3u;
+// The stencil code of cell (i, j) of a level.
+__device__ __forceinline__ unsigned cell_code(const uint8_t* label, int nx, int ny, int i, int j) {
+  const int k = i + j * nx;
+  unsigned c = label[k] & 3u;
   if (i + 1 < nx && label[k + 1] != SOLID) c |= LINK_XP;
   if (i > 0 && label[k - 1] != SOLID) c |= LINK_XM;
   if (j + 1 < ny && label[k + nx] != SOLID) c |= LINK_YP;
   if (j > 0 && label[k - nx] != SOLID) c |= LINK_YM;
-  code[k] = c;
+  return c;
+}
+
+// pressureMultigrid.ts:92-110 (multigrid.wgsl:259-286): the coarse label of
+// the 2 x 2 cells from (i, j) on (even), Air > Fluid > Solid.
+__device__ __forceinline__ uint8_t coarse_label(const uint8_t* label, int nx, int ny, int i, int j) {
+  bool air = false, fluid = false;
+  for (int dj = 0; dj < 2; dj++)
+    for (int di = 0; di < 2; di++) {
+      if (i + di >= nx || j + dj >= ny) continue;
+      const uint8_t l = label[i + di + (j + dj) * nx];
+      air = air || l == AIR;
+      fluid = fluid || l == FLUID;
+    }
+  return air ? AIR : (fluid ? FLUID : SOLID);
+}
+
+// A level's stencil codes and, where `coarse` is set, the next level's labels.
+// only_if (when set): the kernel does nothing unless *only_if is nonzero
+__global__ void k_build_codes(int nx, int ny, const uint8_t* __restrict__ label, uint8_t* __restrict__ code,
+                              uint8_t* __restrict__ coarse, const int* only_if) {
+  if (only_if != nullptr && *only_if == 0) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  if (i >= nx || j >= ny) return;
+  code[i + j * nx] = (uint8_t)cell_code(label, nx, ny, i, j);  // 32-bit offsets: a level holds fewer than 2^31 cells
+  if (coarse != nullptr && ((i | j) & 1) == 0)
+    coarse[(i >> 1) + (j >> 1) * ((nx + 1) / 2)] = coarse_label(label, nx, ny, i, j);
 }
 
 // The uploaded labels against the current ones: copies the cells that
@@ -88,25 +109,6 @@ void launch_label_sync(cudaStream_t s, const uint8_t* in, uint8_t* cur, long n, 
 
 void launch_label_cond(cudaStream_t s, int* flag, cudaGraphConditionalHandle h) { k_label_cond<<<1, 1, 0, s>>>(flag, h); }
 
-// pressureMultigrid.ts:92-110 (multigrid.wgsl:259-286): Air > Fluid > Solid.
-__global__ void k_coarsen_labels(int fnx, int fny, const uint8_t* __restrict__ fine, int cnx, int cny,
-                                 uint8_t* __restrict__ coarse, const int* only_if) {
-  if (only_if != nullptr && *only_if == 0) return;
-  const int I = blockIdx.x * blockDim.x + threadIdx.x;
-  const int J = blockIdx.y * blockDim.y + threadIdx.y;
-  if (I >= cnx || J >= cny) return;
-  bool air = false, fluid = false;
-  for (int dj = 0; dj < 2; dj++)
-    for (int di = 0; di < 2; di++) {
-      const int i = 2 * I + di, j = 2 * J + dj;
-      if (i >= fnx || j >= fny) continue;
-      const uint8_t l = fine[i + (long)j * fnx];
-      air = air || l == AIR;
-      fluid = fluid || l == FLUID;
-    }
-  coarse[I + (long)J * cnx] = air ? AIR : (fluid ? FLUID : SOLID);
-}
-
 struct SmoothArgs {
   int nx, ny;
   const float* xin;
@@ -123,34 +125,27 @@ struct SmoothArgs {
   int pairs, halo;  // sweep pairs, and the region's halo (smooth_halo)
 };
 
-// (sum - scale*b) / count with count in 1..4: a multiply by the exact
-// reciprocal for 1, 2 and 4 (the same float as the division, since scaling by
-// a power of two is exact) and a true division for 3.
-//
-// The division by 3 is the correctly rounded quotient formed with two FMAs
-// (the correction step for a divisor known in advance: Markstein; Brisebarre,
-// Muller and Raina, IEEE Trans. Computers 2004): q0 = RN(s * RN(1/3)),
-// r = s - 3 q0 (exact), q = RN(q0 + r * RN(1/3)); zero and infinities take
-// q0. It equals IEEE s / 3 for every float (checked exhaustively), at a
-// fraction of the division's latency.
-__device__ __forceinline__ float div3(float s) {
-  const float y = 0x1.555556p-2f;  // RN(1/3)
-  const float q0 = __fmul_rn(s, y);
-  const float r = __fmaf_rn(-3.0f, q0, s);
-  const float q1 = __fmaf_rn(r, y, q0);
-  return (s == 0.0f || fabsf(s) == __int_as_float(0x7f800000)) ? q0 : q1;
-}
-
 // s / count for rc = (RN(1 / count), -count), count 1..4, without a branch or
-// a test of the count: div3's steps for every count. For 1, 2 and 4 the first
-// product is the quotient, the remainder 0 and the second step changes
-// nothing. An infinite s has a NaN remainder, which fmaxf turns into a finite
-// number: the quotient then stays infinite. Equals IEEE division for every
-// float but for the sign of a zero.
+// a test of the count: the correctly rounded quotient formed with two FMAs
+// (the correction step for a divisor known in advance: Markstein; Brisebarre,
+// Muller and Raina, IEEE Trans. Computers 2004): q0 = RN(s * RN(1 / count)),
+// r = s - count q0 (exact), q = RN(q0 + r * RN(1 / count)). For 1, 2 and 4 q0
+// is the quotient, r is 0 and the second step changes nothing. An infinite s
+// has a NaN remainder, which fmaxf turns into a finite number: the quotient
+// then stays infinite. Equals IEEE division for every float (for 3 checked
+// exhaustively) but for the sign of a zero.
 __device__ __forceinline__ float over_links(float s, float2 rc) {
   const float q0 = __fmul_rn(s, rc.x);
   const float r = fmaxf(__fmaf_rn(rc.y, q0, s), -3.402823466e+38f);
   return __fmaf_rn(r, rc.x, q0);
+}
+
+// over_links' factors of a cell with this code: (0, 0) unless it is fluid
+// with a link, which the sweeps update (pressureRedBlack.ts:52-66).
+__device__ __forceinline__ float2 link_factors(int code) {
+  const int cnt = code_count((uint8_t)code);
+  const bool on = (code & 3) == FLUID && cnt > 0;
+  return make_float2(on ? 1.0f / (float)cnt : 0.0f, on ? -(float)cnt : 0.0f);
 }
 
 // Temporally blocked red-black smoother. One CTA of NW warps owns a region of
@@ -283,13 +278,7 @@ __device__ __forceinline__ void smooth_tile(const SmoothArgs& a, int bx, int by,
     }
   }
 
-  // code -> (RN(1 / count), -count) (pressureRedBlack.ts:52-66 updates fluid
-  // cells with a link only)
-  if (tid < 64) {
-    const int cnt = code_count((uint8_t)tid);
-    const bool on = (tid & 3) == FLUID && cnt > 0;
-    sh.lut[tid] = make_float2(on ? 1.0f / (float)cnt : 0.0f, on ? -(float)cnt : 0.0f);
-  }
+  if (tid < 64) sh.lut[tid] = link_factors(tid);
   if (w == 0) {
     sh.edge[0][0][1][lane] = sh.edge[1][0][1][lane] = 0.0f;
     sh.edge[0][NW + 1][0][lane] = sh.edge[1][NW + 1][0][lane] = 0.0f;
@@ -476,30 +465,44 @@ __global__ void __launch_bounds__(32 * NW, RW == 8 ? 24 / NW : 32 / NW) k_smooth
 
 // ----------------------------------------------------- single-CTA coarse tail
 
-// The coarsest levels (both sides <= fl_params.mg_tail_side, 32 by default,
-// at most 64) run in ONE 1024-thread CTA, entirely in shared memory (a zero
-// word first, then per level x split by parity, xs[(i+j)&1][j][i>>1] with a
-// power-of-two row stride, b and the stencil codes row-major). The CTA is bound by how
-// many instructions its warps issue, so each level is owned by as few warps
-// as hold its cells: a row of colour-c cells gets LPR = 2^lsh lanes (the
-// power of two >= ceil(nx/2)), a warp covers 32/LPR rows, and only the first
-// `nwarps` warps (at most 32; a 64-row level gives each of them two row
-// groups) take part in that level's phases, synchronising on the level's own
-// named barrier. Coarser levels are owned by a subset of the finer level's
-// warps, so the barrier that ends a phase on a level also orders it before
-// every coarser-level phase.
-struct CoarseLevel {
-  int nx, ny;
-  const uint8_t* code;
-  int off_x, off_b, off_c;  // shared-memory offsets: floats, floats, bytes
-  int lsh;                  // log2 of the lanes per row
-  int nwarps;               // owner warps
-  int slots;                // row groups per warp: 2 when the level has more than 32 groups
-};
+// The coarsest levels (both sides <= fl_params.mg_tail_side, at most 64) run
+// in ONE CTA. Each level lies in a square frame of a power-of-two side F (the
+// tail's first level in the smallest frame that holds it, the next in half of
+// that, and so on; cells beyond the level are coded outside), so that every
+// index is known at compile time. A lane owns a pair of columns (2i, 2i + 1)
+// of one row: one cell of each colour. A row takes F / 2 lanes, a warp 64 / F
+// rows, and the frame's first F^2 / 64 warps (at most 32; at F = 64 each of
+// them has two row groups) take part in a level's phases, synchronising on the
+// frame's own named barrier. A pair's index in its frame, row * F / 2 + i, is
+// then the thread's index (+ 1024 in its second row group).
+//
+// The CTA is one chain of dependent phases, so their latency is all that
+// counts. A level's values, rhs and codes stay in its owners' registers from
+// the pre-smoothing to the post-smoothing. In a half-sweep a cell's one
+// horizontal neighbour is the lane's other value, the other one shuffle away,
+// the vertical ones two shared-memory loads, or two shuffles in a frame that
+// one warp holds, which then needs no shared memory and no barrier. An
+// unlinked neighbour is masked to +0.0 (which leaves a sum's bits unchanged
+// but for the sign of an exact zero), and over_links divides without a branch.
+// The fine level's owners write their residuals by column into an exchange
+// buffer, from which the coarse level's owners sum them (two 16-byte loads a
+// pair); the coarse level's result comes back through its own.
+//
+// Coarser levels are owned by a subset of the finer level's warps, so the
+// barrier that ends a phase on a level also orders it before every
+// coarser-level phase.
+//
+// Measured, 32^2 to 8^2 with V(3,3) and 16 coarsest pairs, launches chained in
+// a graph: 6.0 us, against 16.1 with the values, codes and geometry in shared
+// memory and fetched again in every phase. From 64^2 on: 13.3 us, hardly less
+// than with the 64^2 level's own two launches (14.1), and 1024^2 V-cycles 45.0
+// against 45.6: the tail stays at 32^2.
+constexpr int TAIL_LEVELS = 7;  // at most 64 a side
 
 struct CoarseArgs {
-  int nlev;
-  CoarseLevel lv[MAX_LEVELS];
+  int nx, ny, nlev;       // of the tail's first level; levels
+  int frame;              // its frame's side
+  const uint16_t* codes;  // every frame's codes (k_tail_codes)
   const float* b_top;
   float* x_top;
   int x_is_zero;
@@ -509,284 +512,267 @@ struct CoarseArgs {
 };
 
 // Default first level of the single-CTA tail (fl_params.mg_tail_side = 0):
-// levels with both sides <= 32. Measured on the 1024^2 plume: 1641 steps/s
-// from 32, 1570 from 64, 1636 from 16, 1626 from 8 (below 32 the extra
-// launches cost more than the tail's shorter barrier chain saves).
+// levels with both sides <= 32.
 constexpr int TAIL_SIDE_DEFAULT = 32;
 
-struct CoarseView {
-  float* xs;  // 2 * ny * rs floats
-  float* bs;
-  const uint8_t* cs;
-  int nx, ny, rs;
-  __device__ float& x(int i, int j) const { return xs[((i + j) & 1) * ny * rs + j * rs + (i >> 1)]; }
+template <int F>
+struct Frame {
+  static constexpr int LPR = F > 1 ? F / 2 : 1;                       // lanes a row
+  static constexpr int PAIRS = F * LPR;
+  static constexpr int NP = PAIRS < 32 ? 32 : PAIRS;                  // with the warp's idle lanes
+  static constexpr int WARPS = NP > 1024 ? 32 : NP / 32;
+  static constexpr int SLOTS = NP > 1024 ? 2 : 1;
+  static constexpr bool ONE = WARPS == 1;
+  static constexpr int BAR = F == 64 ? 1 : F == 32 ? 2 : 3;           // named barrier (64, 32 and 16)
+  // shared memory, in floats: the frames one after the other, smallest first;
+  // the exchange buffer (a float2 a pair, by column), then the values by
+  // colour, a row of lanes before and after each
+  static constexpr int OFF = Frame<F / 2>::OFF + Frame<F / 2>::FLOATS;
+  static constexpr int FLOATS = 2 * NP + (ONE ? 0 : 2 * (NP + 2 * LPR));
+  static constexpr int CODES = Frame<F / 2>::CODES + Frame<F / 2>::NP;  // offset of the frame's codes
+};
+template <>
+struct Frame<0> {
+  static constexpr int NP = 0, OFF = 0, FLOATS = 0, CODES = 0;
+};
+constexpr int TAIL_CODES = Frame<64>::CODES + Frame<64>::NP;
+
+// What a lane keeps of one pair, by colour.
+struct TailPair {
+  float x[2], b[2];
+  unsigned code;  // byte c: colour c's
 };
 
-__device__ __forceinline__ CoarseView coarse_view(unsigned char* smem, const CoarseLevel& L) {
-  float* fs = reinterpret_cast<float*>(smem);
-  CoarseView v;
-  v.xs = fs + L.off_x;
-  v.bs = fs + L.off_b;
-  v.cs = smem + L.off_c;
-  v.nx = L.nx;
-  v.ny = L.ny;
-  v.rs = 1 << L.lsh;
-  return v;
-}
+__device__ __forceinline__ float masked(float v, int m) { return __int_as_float(__float_as_int(v) & m); }
 
-// The cell of colour c in row group w + 32 s owned by `lane`.
-__device__ __forceinline__ void tail_cell(const CoarseLevel& L, int w, int lane, int s, int c, int& i, int& j) {
-  j = ((w + 32 * s) << (5 - L.lsh)) + (lane >> L.lsh);
-  i = 2 * (lane & ((1 << L.lsh) - 1)) + ((c + j) & 1);
-}
+template <int F>
+struct TailLevel {
+  using G = Frame<F>;
+  float2* r;       // exchange buffer
+  float* v[2];     // values by colour
+  int tid, lane;
+  TailPair q[G::SLOTS];
 
-// Named barrier `l + 1` over the owner warps of tail level l (a warp
-// barrier when one warp owns the level).
-__device__ __forceinline__ void tail_bar(int l, int nwarps) {
-  if (nwarps == 1) {
-    __syncwarp();
+  __device__ __forceinline__ TailLevel(float* smem, int tid_) : tid(tid_), lane(tid_ & 31) {
+    r = reinterpret_cast<float2*>(smem + G::OFF);
+    v[0] = smem + G::OFF + 2 * G::NP + G::LPR;
+    v[1] = v[0] + G::NP + 2 * G::LPR;
+  }
+  __device__ __forceinline__ int pair(int s) const { return tid + 1024 * s; }
+  __device__ __forceinline__ int row(int s) const { return pair(s) / G::LPR; }
+  __device__ __forceinline__ void bar() const {
+    if (G::ONE)
+      __syncwarp();
+    else
+      asm volatile("bar.sync %0, %1;" ::"n"(G::BAR), "n"(32 * G::WARPS) : "memory");
+  }
+  // the neighbour sum of pair s's colour-c cell, order +x, -x, +y, -y (the
+  // first two commute)
+  __device__ __forceinline__ float sum(int s, int c) const {
+    const unsigned k = q[s].code >> (8 * c);
+    const int o = (c + row(s)) & 1;  // the pair's column of colour c
+    const int xp = -(int)(k >> 2 & 1u), xm = -(int)(k >> 3 & 1u);
+    const float own = q[s].x[1 - c];
+    const float far = __shfl_sync(0xffffffffu, own, lane + (o ? 1 : -1));
+    float up, dn;
+    if constexpr (G::ONE) {
+      up = __shfl_sync(0xffffffffu, own, lane + G::LPR);
+      dn = __shfl_sync(0xffffffffu, own, lane - G::LPR);
+    } else {
+      up = v[1 - c][pair(s) + G::LPR];
+      dn = v[1 - c][pair(s) - G::LPR];
+    }
+    return ((masked(own, o ? xm : xp) + masked(far, o ? xp : xm)) + masked(up, -(int)(k >> 4 & 1u))) +
+           masked(dn, -(int)(k >> 5 & 1u));
+  }
+  __device__ __forceinline__ void publish(int s, int c) const {
+    if constexpr (!G::ONE) v[c][pair(s)] = q[s].x[c];
+  }
+  __device__ __forceinline__ void publish_all() const {
+#pragma unroll
+    for (int s = 0; s < G::SLOTS; s++) publish(s, 0), publish(s, 1);
+    bar();
+  }
+  __device__ __forceinline__ void exchange(int s, float c0, float c1) const {
+    r[pair(s)] = (row(s) & 1) ? make_float2(c1, c0) : make_float2(c0, c1);  // odd rows: colour 0 is column 1
+  }
+  __device__ __forceinline__ float2 factors(const float2* lut, int s, int c) const {
+    return lut[q[s].code >> (8 * c) & 0x3fu];
+  }
+  // r = b - (count*x - sum), 0 where the cell is not updated (pressureMultigrid.ts:117-151)
+  __device__ __forceinline__ float residual(const float2* lut, int s, int c) const {
+    const float2 rc = factors(lut, s, c);
+    const float res = q[s].b[c] + (rc.y * q[s].x[c] + sum(s, c));
+    return rc.x != 0.0f ? res : 0.0f;
+  }
+  // `pairs` red-black sweep pairs; from_zero: the values are 0 and not yet
+  // published, so the first half-sweep has no neighbours to add.
+  __device__ __forceinline__ void sweeps(const float2* lut, int pairs, float omega, bool from_zero) {
+    float2 rc[G::SLOTS][2];
+#pragma unroll
+    for (int s = 0; s < G::SLOTS; s++)
+#pragma unroll
+      for (int c = 0; c < 2; c++) rc[s][c] = factors(lut, s, c);
+    const float keep = 1.0f - omega;
+    auto run = [&](auto unit) {
+      constexpr bool UNIT = decltype(unit)::value;  // omega = 1: pGS itself (see smooth_tile)
+#pragma unroll 1
+      for (int k = 0; k < pairs; k++) {
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+#pragma unroll
+          for (int s = 0; s < G::SLOTS; s++) {
+            float t = q[s].b[c];
+            if (c == 1 || k > 0 || !from_zero) t = sum(s, c) + t;
+            const float pgs = over_links(t, rc[s][c]);
+            const float nv = UNIT ? pgs : keep * q[s].x[c] + omega * pgs;
+            q[s].x[c] = rc[s][c].x != 0.0f ? nv : q[s].x[c];
+            publish(s, c);
+          }
+          if (!G::ONE) bar();
+        }
+      }
+    };
+    if (omega == 1.0f)
+      run(std::true_type{});
+    else
+      run(std::false_type{});
+  }
+};
+
+// The V-cycle from frame F down (frames larger than the tail's first one pass
+// the call on); rsq, rn: the residual norm of the first level when a.acc asks
+// for it.
+template <int F>
+__device__ __forceinline__ void tail_frame(const CoarseArgs& a, float* smem, const float2* lut, const unsigned* code,
+                                           int tid, double& rsq, unsigned long long& rn) {
+  using G = Frame<F>;
+  if (F > a.frame) {
+    if constexpr (F > 1) tail_frame<F / 2>(a, smem, lut, code, tid, rsq, rn);
     return;
   }
-  asm volatile("bar.sync %0, %1;" ::"r"(l + 1), "r"(nwarps * 32) : "memory");
-}
-
-// r = b - (count*x - sum), 0 off-fluid (pressureMultigrid.ts:117-151).
-// Branch-free for the same reason as tail_smooth: every neighbour is read
-// (an unlinked one at the cell itself) and an unlinked one adds +0.0.
-__device__ __forceinline__ float coarse_residual(const CoarseView& v, int i, int j, bool& counted) {
-  const int k = i + j * v.nx;
-  const uint8_t c = v.cs[k];
-  const int cnt = code_count(c);
-  counted = (c & 3u) == FLUID && cnt > 0;
-  const int pl = v.ny * v.rs;
-  const int own = ((i + j) & 1) * pl + j * v.rs + (i >> 1);
-  const int oth = (1 - ((i + j) & 1)) * pl + j * v.rs;
-  const float x0 = v.xs[own];
-  const float vxp = v.xs[(c & LINK_XP) ? oth + ((i + 1) >> 1) : own];
-  const float vxm = v.xs[(c & LINK_XM) ? oth + ((i - 1) >> 1) : own];
-  const float vyp = v.xs[(c & LINK_YP) ? oth + v.rs + (i >> 1) : own];
-  const float vym = v.xs[(c & LINK_YM) ? oth - v.rs + (i >> 1) : own];
-  float sum = 0.0f;
-  sum += (c & LINK_XP) ? vxp : 0.0f;
-  sum += (c & LINK_XM) ? vxm : 0.0f;
-  sum += (c & LINK_YP) ? vyp : 0.0f;
-  sum += (c & LINK_YM) ? vym : 0.0f;
-  const float r = v.bs[k] - ((float)cnt * x0 - sum);
-  return counted ? r : 0.0f;
-}
-
-// `pairs` red-black sweep pairs on tail level l by its owner warps; ends
-// with the level's barrier (also when pairs is 0). Each thread keeps its
-// cells' rhs, value, link mask and the shared-memory addresses of their
-// four neighbours in registers. The update has no branches: on these small
-// levels most warps hold boundary cells, and a lane-divergent branch around
-// each neighbour load serialised the warp (measured: a one-warp half-sweep
-// took ~630 cycles that way, ~270 with unconditional loads). An unlinked
-// neighbour is read at the zero word that starts shared memory and adds
-// +0.0, which leaves the sum's bits unchanged: a running sum that starts at
-// +0.0 never becomes -0.0.
-__device__ __forceinline__ float lds_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-  return v;
-}
-__device__ __forceinline__ void sts_f32(uint32_t addr, float v) {
-  asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-
-__device__ void tail_smooth(unsigned char* smem, const CoarseLevel& L, int l, int pairs, float omega, int w,
-                            int lane) {
-  if (w >= L.nwarps) return;
-  float* xs = reinterpret_cast<float*>(smem) + L.off_x;
-  const uint32_t sm_sh = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-  const float* bs = reinterpret_cast<const float*>(smem) + L.off_b;
-  const uint8_t* cs = smem + L.off_c;
-  // row stride: the lanes per row (a power of two), so that the rows a warp
-  // covers fall in distinct shared-memory banks
-  const int rs = 1 << L.lsh;
-  const int plane = L.ny * rs;
-  bool upd[2][2];  // the cell is updated
-  int own[2][2], nb[2][2][4];
-  float bq[2][2], xq[2][2], rc[2][2];
+  if (tid >= 32 * G::WARPS) return;
+  TailLevel<F> L(smem, tid);
+  const int depth = __popc(a.frame - 1) - __popc(F - 1);  // the level below the tail's first
+  const bool last = depth == a.nlev - 1, top = depth == 0;
+  const int nx = ((a.nx - 1) >> depth) + 1, ny = ((a.ny - 1) >> depth) + 1;
+  constexpr int LOG = F == 64 ? 6 : F == 32 ? 5 : F == 16 ? 4 : F == 8 ? 3 : F == 4 ? 2 : F == 2 ? 1 : 0;
 #pragma unroll
-  for (int s = 0; s < 2; s++)
-#pragma unroll
-    for (int c = 0; c < 2; c++) {
-      int i, j;
-      tail_cell(L, w, lane, s, c, i, j);
-      const bool ok = i < L.nx && j < L.ny;
-      const uint8_t code = ok ? cs[i + j * L.nx] : (uint8_t)CODE_OUTSIDE;
-      const int cnt = code_count(code);
-      const bool act = ok && (code & 3u) == FLUID && cnt > 0;
-      // float indices from the start of shared memory; an unlinked
-      // neighbour (and every neighbour of a cell outside the level) is the
-      // zero word at index 0
-      const int ow = L.off_x + (ok ? c * plane + j * rs + (i >> 1) : 0);
-      const int o = L.off_x + (1 - c) * plane + j * rs + (i >> 1), d = i & 1;
-      own[s][c] = ow;
-      nb[s][c][0] = (ok && (code & LINK_XP)) ? o + d : 0;
-      nb[s][c][1] = (ok && (code & LINK_XM)) ? o + d - 1 : 0;
-      nb[s][c][2] = (ok && (code & LINK_YP)) ? o + rs : 0;
-      nb[s][c][3] = (ok && (code & LINK_YM)) ? o - rs : 0;
-      upd[s][c] = act;
-      rc[s][c] = cnt == 4 ? 0.25f : (cnt == 2 ? 0.5f : (cnt == 1 ? 1.0f : 0.0f));
-      bq[s][c] = ok ? bs[i + j * L.nx] : 0.0f;
-      xq[s][c] = ok ? xs[ow - L.off_x] : 0.0f;
-    }
-  // shared-space byte addresses (explicit ld/st.shared)
-#pragma unroll
-  for (int s = 0; s < 2; s++)
-#pragma unroll
-    for (int c = 0; c < 2; c++) {
-      own[s][c] = (int)(sm_sh + 4u * (uint32_t)own[s][c]);
-#pragma unroll
-      for (int k = 0; k < 4; k++) nb[s][c][k] = (int)(sm_sh + 4u * (uint32_t)nb[s][c][k]);
-    }
-  const bool two = L.slots == 2;
-  const float keep = 1.0f - omega;
-  // omega = 1: pGS itself (see smooth_tile)
-  auto sweeps = [&](auto unit) {
-    constexpr bool UNIT = decltype(unit)::value;
-#pragma unroll 1
-    for (int hs = 0; hs < 2 * pairs; hs += 2) {
-#pragma unroll
-      for (int c = 0; c < 2; c++) {
-#pragma unroll
-        for (int s = 0; s < 2; s++) {
-          if (s == 1 && !two) continue;  // warp-uniform: the level has one row group per warp
-          const float v0 = lds_f32((uint32_t)nb[s][c][0]), v1 = lds_f32((uint32_t)nb[s][c][1]);
-          const float v2 = lds_f32((uint32_t)nb[s][c][2]), v3 = lds_f32((uint32_t)nb[s][c][3]);
-          float sum = 0.0f;
-          sum += v0;
-          sum += v1;
-          sum += v2;
-          sum += v3;
-          const float dv = sum - (-1.0f) * bq[s][c];
-          const float third = div3(dv);
-          const float pgs = rc[s][c] != 0.0f ? dv * rc[s][c] : third;
-          const float nv = UNIT ? pgs : keep * xq[s][c] + omega * pgs;
-          if (upd[s][c]) {
-            xq[s][c] = nv;
-            sts_f32((uint32_t)own[s][c], nv);
-          }
-        }
-        tail_bar(l, L.nwarps);
-      }
-    }
-  };
-  if (omega == 1.0f)
-    sweeps(std::true_type{});
-  else
-    sweeps(std::false_type{});
-  if (pairs <= 0) tail_bar(l, L.nwarps);
-}
-
-// The whole tail, run by one 1024-thread block over `smem` (the layout of
-// coarse_smem_bytes).
-__device__ __forceinline__ void mg_coarse_body(const CoarseArgs& a, unsigned char* smem) {
-  const int tid = threadIdx.x + 32 * threadIdx.y;
-  const int lane = tid & 31, w = tid >> 5;
-  if (tid == 0) reinterpret_cast<float*>(smem)[0] = 0.0f;  // the zero word tail_smooth's unlinked neighbours read
-  for (int l = 0; l < a.nlev; l++) {
-    const CoarseLevel& L = a.lv[l];
-    const int n = L.nx * L.ny;
-    uint8_t* c = smem + L.off_c;
-    for (int k = tid; k < n; k += 1024) c[k] = L.code[k];
-  }
-  const CoarseLevel& TL = a.lv[0];
-  const CoarseView T = coarse_view(smem, TL);
-  if (w < TL.nwarps) {
-#pragma unroll
-    for (int s = 0; s < 2; s++)
-#pragma unroll
-      for (int c = 0; c < 2; c++) {
-        int i, j;
-        tail_cell(TL, w, lane, s, c, i, j);
-        if (i < T.nx && j < T.ny) {
-          const int k = i + j * T.nx;
-          T.bs[k] = a.b_top[k];
-          T.x(i, j) = a.x_is_zero ? 0.0f : a.x_top[k];
+  for (int s = 0; s < G::SLOTS; s++) {
+    TailPair& q = L.q[s];
+    q.code = code[s == 1 ? 7 : LOG];
+    q.x[0] = q.x[1] = 0.0f;
+    float2 b = make_float2(0.0f, 0.0f);  // by column
+    const int j = L.row(s), i = 2 * (L.pair(s) & (G::LPR - 1));
+    if (top) {
+      if (j < ny && i < nx) {
+        const int k = i + j * nx;
+        b.x = a.b_top[k];
+        if (i + 1 < nx) b.y = a.b_top[k + 1];
+        if (!a.x_is_zero) {
+          const float x0 = a.x_top[k], x1 = i + 1 < nx ? a.x_top[k + 1] : 0.0f;
+          q.x[0] = (j & 1) ? x1 : x0;
+          q.x[1] = (j & 1) ? x0 : x1;
         }
       }
+    } else if (F < 64 && L.pair(s) < G::PAIRS) {
+      // the coarse rhs: the sum of the children's residuals
+      // (pressureMultigrid.ts:156-178; those outside the level are 0)
+      constexpr int FF = F < 64 ? 2 * F : 64;
+      const float2* f = reinterpret_cast<const float2*>(smem + Frame<FF>::OFF) + 2 * j * Frame<FF>::LPR + i;
+      const float2 lo = f[0], hi = f[Frame<FF>::LPR];
+      b.x = ((lo.x + lo.y) + hi.x) + hi.y;
+      if (F > 1) {
+        const float2 lo2 = f[1], hi2 = f[Frame<FF>::LPR + 1];
+        b.y = ((lo2.x + lo2.y) + hi2.x) + hi2.y;
+      }
+    }
+    q.b[0] = (j & 1) ? b.y : b.x;
+    q.b[1] = (j & 1) ? b.x : b.y;
   }
+  const int sweeps = last ? a.coarse_sweeps : a.pre;
+  const bool from_zero = !top || a.x_is_zero;
+  if (!from_zero || sweeps == 0) L.publish_all();
+  L.sweeps(lut, sweeps, a.omega, from_zero);
+  if constexpr (F > 1) {
+    if (!last) {
+#pragma unroll
+      for (int s = 0; s < G::SLOTS; s++) L.exchange(s, L.residual(lut, s, 0), L.residual(lut, s, 1));
+      L.bar();
+      tail_frame<F / 2>(a, smem, lut, code, tid, rsq, rn);
+      L.bar();  // the coarse level's owners are done with it
+      // prolongation (9/16, 3/16, 3/16, 1/16, pressureMultigrid.ts:192-207)
+      const float* e = smem + Frame<F / 2>::OFF;
+      constexpr int ES = 2 * Frame<F / 2>::LPR;
+      const int cx = (nx + 1) / 2 - 1, cy = (ny + 1) / 2 - 1;
+#pragma unroll
+      for (int s = 0; s < G::SLOTS; s++) {
+        TailPair& q = L.q[s];
+        const int j = L.row(s), I = min(L.pair(s) & (G::LPR - 1), cx);
+        const int J = min(j >> 1, cy), J2 = (j & 1) ? min(J + 1, cy) : max(J - 1, 0);
+        const int left = max(I - 1, 0), right = min(I + 1, cx);
+        const float m1 = e[J * ES + I], l1 = e[J * ES + left], r1 = e[J * ES + right];
+        const float m2 = e[J2 * ES + I], l2 = e[J2 * ES + left], r2 = e[J2 * ES + right];
+        const float add0 = 0.5625f * m1 + 0.1875f * (l1 + m2) + 0.0625f * l2;
+        const float add1 = 0.5625f * m1 + 0.1875f * (r1 + m2) + 0.0625f * r2;
+        const float x0 = q.x[0] + ((j & 1) ? add1 : add0), x1 = q.x[1] + ((j & 1) ? add0 : add1);
+        q.x[0] = (q.code & 3u) == FLUID ? x0 : q.x[0];
+        q.x[1] = (q.code >> 8 & 3u) == FLUID ? x1 : q.x[1];
+      }
+      if (!G::ONE || a.post == 0) L.publish_all();
+      L.sweeps(lut, a.post, a.omega, false);
+    }
+  }
+  if (!top) {
+#pragma unroll
+    for (int s = 0; s < G::SLOTS; s++) L.exchange(s, L.q[s].x[0], L.q[s].x[1]);
+    return;
+  }
+#pragma unroll
+  for (int s = 0; s < G::SLOTS; s++) {
+    const TailPair& q = L.q[s];
+    if (a.acc != nullptr)
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        const double d = f2d_exact(L.residual(lut, s, c));  // 0 where not counted
+        rsq = fma(d, d, rsq);
+        rn += L.factors(lut, s, c).x != 0.0f;
+      }
+    const int j = L.row(s), i = 2 * (L.pair(s) & (G::LPR - 1));
+    if (j < ny && i < nx) a.x_top[i + j * nx] = (j & 1) ? q.x[1] : q.x[0];
+    if (j < ny && i + 1 < nx) a.x_top[i + 1 + j * nx] = (j & 1) ? q.x[0] : q.x[1];
+  }
+}
+
+// The whole tail, run by one block of at least the first frame's warps (and
+// 64 threads).
+template <int TOP>
+struct TailShared {
+  float f[Frame<TOP>::OFF + Frame<TOP>::FLOATS];
+  float2 lut[64];  // code -> (RN(1 / count), -count)
+};
+
+template <int TOP>
+__device__ __forceinline__ void mg_coarse_body(const CoarseArgs& a, TailShared<TOP>& sh) {
+  const int tid = threadIdx.x;
+  // the codes of the thread's pair of every frame it has one in (7: its second of frame 64)
+  unsigned code[8];
+  auto load = [&](int q, int at, int np, int p) { code[q] = p < np ? __ldg(a.codes + at + p) : 0u; };
+  load(0, Frame<1>::CODES, Frame<1>::NP, tid);
+  load(1, Frame<2>::CODES, Frame<2>::NP, tid);
+  load(2, Frame<4>::CODES, Frame<4>::NP, tid);
+  load(3, Frame<8>::CODES, Frame<8>::NP, tid);
+  load(4, Frame<16>::CODES, Frame<16>::NP, tid);
+  load(5, Frame<32>::CODES, Frame<32>::NP, tid);
+  if (TOP == 64) {
+    load(6, Frame<64>::CODES, Frame<64>::NP, tid);
+    load(7, Frame<64>::CODES, Frame<64>::NP, tid + 1024);
+  }
+  if (tid < 64) sh.lut[tid] = link_factors(tid);
   __syncthreads();
-
-  // down: pre-smooth, then residual + restriction (by the coarse level's
-  // owners) with the coarse x set to 0
-  for (int l = 0; l < a.nlev - 1; l++) {
-    const CoarseLevel& FL = a.lv[l];
-    const CoarseLevel& CL = a.lv[l + 1];
-    tail_smooth(smem, FL, l, a.pre, a.omega, w, lane);
-    if (w >= CL.nwarps) continue;
-    const CoarseView F = coarse_view(smem, FL);
-    const CoarseView C = coarse_view(smem, CL);
-#pragma unroll
-    for (int s = 0; s < 2; s++)
-#pragma unroll
-      for (int c = 0; c < 2; c++) {
-        int I, J;
-        tail_cell(CL, w, lane, s, c, I, J);
-        if (I >= C.nx || J >= C.ny) continue;
-        float sum = 0.0f;
-        for (int dj = 0; dj < 2; dj++)
-          for (int di = 0; di < 2; di++) {
-            const int i = 2 * I + di, j = 2 * J + dj;
-            if (i < F.nx && j < F.ny) {
-              bool counted;
-              sum += coarse_residual(F, i, j, counted);
-            }
-          }
-        C.bs[I + J * C.nx] = sum;
-        C.x(I, J) = 0.0f;
-      }
-    tail_bar(l + 1, CL.nwarps);
-  }
-  tail_smooth(smem, a.lv[a.nlev - 1], a.nlev - 1, a.coarse_sweeps, a.omega, w, lane);
-  // up: prolongation (9/16, 3/16, 3/16, 1/16), then post-smooth
-  for (int l = a.nlev - 2; l >= 0; l--) {
-    const CoarseLevel& FL = a.lv[l];
-    if (w >= FL.nwarps) continue;
-    tail_bar(l, FL.nwarps);  // the coarse level's owners are done with it
-    const CoarseView F = coarse_view(smem, FL);
-    const CoarseView C = coarse_view(smem, a.lv[l + 1]);
-#pragma unroll
-    for (int s = 0; s < 2; s++)
-#pragma unroll
-      for (int c = 0; c < 2; c++) {
-        int i, j;
-        tail_cell(FL, w, lane, s, c, i, j);
-        if (i >= F.nx || j >= F.ny) continue;
-        if ((F.cs[i + j * F.nx] & 3u) != FLUID) continue;
-        const int I = i >> 1, J = j >> 1;
-        const int I2 = (i & 1) ? min(I + 1, C.nx - 1) : max(I - 1, 0);
-        const int J2 = (j & 1) ? min(J + 1, C.ny - 1) : max(J - 1, 0);
-        F.x(i, j) += 0.5625f * C.x(I, J) + 0.1875f * (C.x(I2, J) + C.x(I, J2)) + 0.0625f * C.x(I2, J2);
-      }
-    tail_bar(l, FL.nwarps);
-    tail_smooth(smem, FL, l, a.post, a.omega, w, lane);
-  }
-
   double rsq = 0.0;
   unsigned long long rn = 0;
-  if (w < TL.nwarps) {
-#pragma unroll
-    for (int s = 0; s < 2; s++)
-#pragma unroll
-      for (int c = 0; c < 2; c++) {
-        int i, j;
-        tail_cell(TL, w, lane, s, c, i, j);
-        if (i >= T.nx || j >= T.ny) continue;
-        if (a.acc != nullptr) {
-          bool counted;
-          const float res = coarse_residual(T, i, j, counted);
-          if (counted) {
-            rsq = fma(f2d_exact(res), f2d_exact(res), rsq);
-            rn += 1;
-          }
-        }
-        a.x_top[i + j * T.nx] = T.x(i, j);
-      }
-  }
+  tail_frame<TOP>(a, sh.f, sh.lut, code, tid, rsq, rn);
   if (a.acc != nullptr) {
     __shared__ double red[32];
     __shared__ unsigned long long redn[32];
@@ -799,9 +785,55 @@ __device__ __forceinline__ void mg_coarse_body(const CoarseArgs& a, unsigned cha
   }
 }
 
-__global__ void __launch_bounds__(1024, 1) k_mg_coarse(CoarseArgs a) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  mg_coarse_body(a, smem);
+// TOP 32: first levels of at most 32 a side, with twice the registers a thread
+template <int TOP>
+__global__ void __launch_bounds__(TOP == 64 ? 1024 : 512, 1) k_mg_coarse(CoarseArgs a) {
+  __shared__ TailShared<TOP> sh;
+  mg_coarse_body<TOP>(a, sh);
+}
+
+// The labels and codes of every level of the tail in one launch of one CTA:
+// from the first level's labels down, each level's codes, the next level's
+// labels, and the level's codes in its frame (the layout of Frame<F>::CODES; a
+// pair's low byte is its cell of colour 0; cells beyond the level are outside).
+struct TailLabels {
+  int nx, ny, nlev, frame;
+  uint8_t* label[TAIL_LEVELS];
+  uint8_t* code[TAIL_LEVELS];
+  uint16_t* out;
+};
+
+template <int F>
+__device__ __forceinline__ void tail_codes(const TailLabels& a, int l, int nx, int ny) {
+  using G = Frame<F>;
+  if (F == a.frame >> l) {
+    const uint8_t* label = a.label[l];
+    for (int p = threadIdx.x; p < G::NP; p += blockDim.x) {
+      const int j = p / G::LPR, i = 2 * (p & (G::LPR - 1));
+      unsigned c[2] = {CODE_OUTSIDE, CODE_OUTSIDE};
+      if (p < G::PAIRS && j < ny) {
+#pragma unroll
+        for (int o = 0; o < 2; o++)
+          if (i + o < nx) {
+            c[o] = cell_code(label, nx, ny, i + o, j);
+            a.code[l][i + o + j * nx] = (uint8_t)c[o];
+          }
+        if (l + 1 < a.nlev && i < nx && (j & 1) == 0)
+          a.label[l + 1][i / 2 + j / 2 * ((nx + 1) / 2)] = coarse_label(label, nx, ny, i, j);
+      }
+      a.out[G::CODES + p] = (uint16_t)((j & 1) ? (c[1] | c[0] << 8) : (c[0] | c[1] << 8));
+    }
+    __syncthreads();
+    if (++l == a.nlev) return;
+    nx = (nx + 1) / 2;
+    ny = (ny + 1) / 2;
+  }
+  if constexpr (F > 1) tail_codes<F / 2>(a, l, nx, ny);
+}
+
+__global__ void __launch_bounds__(1024) k_tail_labels(TailLabels a, const int* only_if) {
+  if (only_if != nullptr && *only_if == 0) return;
+  tail_codes<64>(a, 0, a.nx, a.ny);
 }
 
 // The float64 defect-correction pass (iterative refinement, solveMixed):
@@ -1240,9 +1272,14 @@ static void launch_smooth(cudaStream_t s, SmoothArgs a, int pairs, int mode) {
   else small ? launch_smooth_nw<MODE_POST, 16, 2>(s, a) : launch_smooth_nw<MODE_POST, 8, 8>(s, a);
 }
 
-void launch_build_codes(cudaStream_t s, int nx, int ny, const uint8_t* label, uint8_t* code, const int* only_if) {
+static void launch_level_codes(cudaStream_t s, int nx, int ny, const uint8_t* label, uint8_t* code, uint8_t* coarse,
+                               const int* only_if) {
   dim3 b(32, 8), g((nx + 31) / 32, (ny + 7) / 8);
-  k_build_codes<<<g, b, 0, s>>>(nx, ny, label, code, only_if);
+  k_build_codes<<<g, b, 0, s>>>(nx, ny, label, code, coarse, only_if);
+}
+
+void launch_build_codes(cudaStream_t s, int nx, int ny, const uint8_t* label, uint8_t* code) {
+  launch_level_codes(s, nx, ny, label, code, nullptr, nullptr);
 }
 
 void launch_rb_halfsweep(cudaStream_t s, int nx, int ny, float* p, const float* b, const uint8_t* code,
@@ -1338,34 +1375,11 @@ void launch_rms_remaining(cudaStream_t s, int nx, int ny, const float* p, const 
   k_rms_remaining<<<g, b, 0, s>>>(nx, ny, p, div, code, scale, acc);
 }
 
-// Shared-memory layout of the single-CTA tail for levels from..end.
-// log2 of the lanes a tail level gives one row of one colour: the power of
-// two >= ceil(nx / 2); also the row stride of its parity planes.
-static int tail_lsh(int nx) {
-  int lpr = 1, lsh = 0;
-  while (lpr < (nx + 1) / 2) {
-    lpr <<= 1;
-    lsh++;
-  }
-  return lsh;
-}
-
-static size_t coarse_smem_bytes(const Engine& e, int from, int* off_x, int* off_b, int* off_c) {
-  size_t floats = 4;  // 16 bytes: the zero word
-  for (int l = from; l < (int)e.levels.size(); l++) {
-    const long n = (long)e.levels[l].nx * e.levels[l].ny;
-    if (off_x) off_x[l - from] = (int)floats;
-    floats += 2 * ((size_t)1 << tail_lsh(e.levels[l].nx)) * (size_t)e.levels[l].ny;
-    if (off_b) off_b[l - from] = (int)floats;
-    floats += n;
-  }
-  size_t bytes = floats * sizeof(float);
-  for (int l = from; l < (int)e.levels.size(); l++) {
-    const long n = (long)e.levels[l].nx * e.levels[l].ny;
-    if (off_c) off_c[l - from] = (int)bytes;
-    bytes += (size_t)((n + 15) / 16) * 16;
-  }
-  return bytes;
+// The side of the frame that holds an nx x ny level of the tail.
+static int tail_frame_side(int nx, int ny) {
+  int f = 1;
+  while (f < nx || f < ny) f *= 2;
+  return f;
 }
 
 void mg_free(Engine& e) {
@@ -1376,20 +1390,9 @@ void mg_free(Engine& e) {
     if (&L != &e.levels[0]) cudaFree(L.label);
     cudaFree(L.code);
   }
+  cudaFree(e.tail_codes);
+  e.tail_codes = nullptr;
   e.levels.clear();
-}
-
-// The dynamic shared-memory limit of k_mg_coarse is a per-device property
-// of the function, shared by every engine in the process: it only ever grows
-// to the largest tail any engine on the device needs (an engine with a
-// smaller tail must not lower it under another engine's launches).
-static void raise_coarse_smem_limit(int device, size_t bytes) {
-  static std::mutex mu;
-  static size_t limit[256] = {};
-  std::lock_guard<std::mutex> lock(mu);
-  if (device < 0 || device >= 256 || bytes <= limit[device]) return;
-  if (cudaFuncSetAttribute(k_mg_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess)
-    limit[device] = bytes;
 }
 
 void mg_setup(Engine& e) {
@@ -1427,20 +1430,33 @@ void mg_setup(Engine& e) {
       break;
     }
   e.coarse_level = lc;
-  e.coarse_smem = coarse_smem_bytes(e, lc, nullptr, nullptr, nullptr);
-  raise_coarse_smem_limit(e.device, e.coarse_smem);
+  cudaMalloc(&e.tail_codes, TAIL_CODES * sizeof(uint16_t));
   e.codes_valid = false;
 }
 
-void mg_build_codes(Engine& e) {
-  cudaStream_t s = e.stream;
-  for (size_t l = 1; l < e.levels.size(); l++) {
-    const Level& F = e.levels[l - 1];
-    const Level& C = e.levels[l];
-    dim3 b(32, 8), g((C.nx + 31) / 32, (C.ny + 7) / 8);
-    k_coarsen_labels<<<g, b, 0, s>>>(F.nx, F.ny, F.label, C.nx, C.ny, C.label, nullptr);
+// Every level's labels and codes on stream s: one launch a level above the
+// tail, one for the tail's levels together.
+static void enqueue_build_codes(const Engine& e, cudaStream_t s, const int* only_if) {
+  const int lc = e.coarse_level, n = (int)e.levels.size();
+  for (int l = 0; l < lc; l++) {
+    const Level& L = e.levels[l];
+    launch_level_codes(s, L.nx, L.ny, L.label, L.code, e.levels[l + 1].label, only_if);
   }
-  for (const Level& L : e.levels) launch_build_codes(s, L.nx, L.ny, L.label, L.code);
+  TailLabels a{};
+  a.nx = e.levels[lc].nx;
+  a.ny = e.levels[lc].ny;
+  a.nlev = n - lc;
+  a.frame = tail_frame_side(a.nx, a.ny);
+  for (int l = lc; l < n; l++) {
+    a.label[l - lc] = e.levels[l].label;
+    a.code[l - lc] = e.levels[l].code;
+  }
+  a.out = e.tail_codes;
+  k_tail_labels<<<1, 1024, 0, s>>>(a, only_if);
+}
+
+void mg_build_codes(Engine& e) {
+  enqueue_build_codes(e, e.stream, nullptr);
   e.codes_valid = true;
 }
 
@@ -1450,13 +1466,7 @@ __global__ void k_clear_flag(int* flag) { *flag = 0; }
 // *flag is set (the label compare's result), then the flag cleared: a
 // plain graph's worth of launches where an IF node would otherwise decide.
 void mg_build_codes_if(Engine& e, cudaStream_t s, int* flag) {
-  for (size_t l = 1; l < e.levels.size(); l++) {
-    const Level& F = e.levels[l - 1];
-    const Level& C = e.levels[l];
-    dim3 b(32, 8), g((C.nx + 31) / 32, (C.ny + 7) / 8);
-    k_coarsen_labels<<<g, b, 0, s>>>(F.nx, F.ny, F.label, C.nx, C.ny, C.label, flag);
-  }
-  for (const Level& L : e.levels) launch_build_codes(s, L.nx, L.ny, L.label, L.code, flag);
+  enqueue_build_codes(e, s, flag);
   k_clear_flag<<<1, 1, 0, s>>>(flag);
 }
 
@@ -1469,22 +1479,20 @@ void mg_vcycle(Engine& e, StepAccum* acc) { mg_vcycle_on(e, e.levels[0].b, false
 // One V-cycle with level 0's rhs `b0`; with `zero_start` the level-0 unknown
 // starts from 0 (the correction equation of the defect-correction loop)
 // instead of the warm start in levels[0].x[0].
+// The threads of a frame's warps, at least 64.
+static int tail_threads(int frame) { return std::min(1024, std::max(64, frame * frame / 2)); }
+
 // The single-CTA tail's arguments for a V-cycle on b0 (the finest level's
 // rhs when the tail starts there), from zero when zero_start, accumulating
 // the finest residual into acc when the tail holds the finest level.
 static CoarseArgs coarse_args(const Engine& e, const float* b0, bool zero_start, StepAccum* acc) {
   const int lc = e.coarse_level;
   CoarseArgs a{};
-  int ox[MAX_LEVELS], ob[MAX_LEVELS], oc[MAX_LEVELS];
-  coarse_smem_bytes(e, lc, ox, ob, oc);
   a.nlev = (int)e.levels.size() - lc;
-  for (int l = 0; l < a.nlev; l++) {
-    const Level& L = e.levels[lc + l];
-    const int lsh = tail_lsh(L.nx);
-    const int rows_per_warp = 32 >> lsh;
-    const int groups = (L.ny + rows_per_warp - 1) / rows_per_warp;
-    a.lv[l] = CoarseLevel{L.nx, L.ny, L.code, ox[l], ob[l], oc[l], lsh, std::min(32, groups), groups > 32 ? 2 : 1};
-  }
+  a.nx = e.levels[lc].nx;
+  a.ny = e.levels[lc].ny;
+  a.frame = tail_frame_side(a.nx, a.ny);
+  a.codes = e.tail_codes;
   a.b_top = lc == 0 ? b0 : e.levels[lc].b;
   a.x_top = e.levels[lc].x[0];
   a.x_is_zero = lc > 0 || zero_start;
@@ -1527,7 +1535,10 @@ void mg_vcycle_on(Engine& e, const float* b0, bool zero_start, StepAccum* acc) {
     double bytes = (lc == 0 ? 4.0 : 0.0) * cells(lc) + 8.0 * cells(lc);
     for (int l = lc; l < (int)e.levels.size(); l++) bytes += cells(l);
     const CoarseArgs a = coarse_args(e, b0, zero_start, acc);
-    k_mg_coarse<<<1, dim3(32, 32), e.coarse_smem, s>>>(a);
+    if (a.frame == 64)
+      k_mg_coarse<64><<<1, tail_threads(a.frame), 0, s>>>(a);
+    else
+      k_mg_coarse<32><<<1, tail_threads(a.frame), 0, s>>>(a);
     prof_end(e, tok, bytes, 1);
   }
   for (int l = lc - 1; l >= 0; l--) {
@@ -1617,7 +1628,7 @@ struct BatchSolve {
   int n = 0, depth = 0, sms = 0;
   int pre = 0, post = 0;
   bool any_mixed = false;
-  size_t tail_smem = 0;
+  int tail_threads = 64;
   BatchScene* scenes = nullptr;  // device, largest scene first
   BatchItem* items = nullptr;    // device
   int* lists = nullptr;          // device: base, count, act_scene, act_pre, act_n, act_total
@@ -1714,12 +1725,13 @@ __global__ void __launch_bounds__(32 * NW, RW == 8 ? 24 / NW : 32 / NW) k_batch_
   }
 }
 
-__global__ void __launch_bounds__(1024, 1) k_batch_tail(BatchPlan plan, int ph) {
-  extern __shared__ __align__(16) unsigned char smem[];
+template <int TOP>
+__global__ void __launch_bounds__(TOP == 64 ? 1024 : 512, 1) k_batch_tail(BatchPlan plan, int ph) {
+  __shared__ TailShared<TOP> sh;
   for (int i = blockIdx.x;; i += gridDim.x) {
     BatchItem it;
     if (!batch_item(plan, ph, i, it)) return;
-    mg_coarse_body(plan.sc[it.scene].tail, smem);
+    mg_coarse_body<TOP>(plan.sc[it.scene].tail, sh);
     __syncthreads();
   }
 }
@@ -1839,7 +1851,7 @@ BatchSolve* batch_solve_create(const std::vector<Engine*>& es_in, std::string& w
     S.ctl = e.ctl;
     S.acc = e.acc;
     b->any_mixed = b->any_mixed || mixed;
-    b->tail_smem = std::max(b->tail_smem, e.coarse_smem);
+    b->tail_threads = std::max(b->tail_threads, tail_threads(S.tail.frame));
     b->depth = std::max(b->depth, S.lc);
   }
   const int n = b->n, depth = b->depth, nph = 2 * depth + 2;
@@ -1926,8 +1938,6 @@ BatchSolve* batch_solve_create(const std::vector<Engine*>& es_in, std::string& w
     err = cudaMemcpy(b->lists, base.data(), base.size() * sizeof(int), cudaMemcpyHostToDevice);
   if (err == cudaSuccess)
     err = cudaMemcpy(b->lists + base.size(), count.data(), count.size() * sizeof(int), cudaMemcpyHostToDevice);
-  if (err == cudaSuccess && b->tail_smem > 48 * 1024)
-    err = cudaFuncSetAttribute(k_batch_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->tail_smem);
   if (err != cudaSuccess) {
     why = cudaGetErrorString(err);
     batch_solve_destroy(b);
@@ -2001,7 +2011,10 @@ cudaError_t batch_solve_enqueue(const BatchSolve& b, cudaStream_t s, cudaStream_
   if (err != cudaSuccess) return err;
   const int D = b.depth;
   for (int d = 0; d < D; d++) launch_batch_smooth<MODE_PRE>(body, b, b.pre, d);
-  k_batch_tail<<<phase_grid(b, D, 1), dim3(32, 32), b.tail_smem, body>>>(b.plan, D);
+  if (b.tail_threads > 512)
+    k_batch_tail<64><<<phase_grid(b, D, 1), b.tail_threads, 0, body>>>(b.plan, D);
+  else
+    k_batch_tail<32><<<phase_grid(b, D, 1), b.tail_threads, 0, body>>>(b.plan, D);
   for (int d = 0; d < D; d++) launch_batch_smooth<MODE_POST>(body, b, b.post, D + 1 + d);
   if (b.max_items[2 * D + 1] > 0)
     k_batch_defect<<<phase_grid(b, 2 * D + 1, 8), 32 * UR_WARPS, 0, body>>>(b.plan, 2 * D + 1);

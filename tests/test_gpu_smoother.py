@@ -57,3 +57,25 @@ def test_multigrid_regions(o32, nx, ny, pre, post):
     same(exp, p, "%dx%d, V(%d,%d)" % (nx, ny, pre, post))
     # a sum of float squares in another order of float64 additions
     assert abs(rr.value - rr32) <= 1e-9 * rr32
+
+
+@pytest.mark.parametrize("nx,ny", [(2, 2), (3, 5), (8, 8), (9, 16), (17, 32), (32, 31), (33, 2), (64, 3), (3, 64),
+                                   (63, 40), (64, 64), (100, 77)])
+@pytest.mark.parametrize("side,coarsest,sweeps,pre,post", [(0, 8, 16, 3, 3), (64, 4, 8, 2, 2), (64, 1, 3, 0, 1),
+                                                           (16, 2, 0, 1, 0), (64, 64, 5, 1, 1)])
+def test_tail_frames(o32, nx, ny, side, coarsest, sweeps, pre, post):
+    """The single-CTA tail: levels that fill their frame or not, in both
+    directions, first level finest or not, one level or several, no sweeps."""
+    label, div, p0 = problem(nx, ny)
+    prm = native.default_params(mg_pre=pre, mg_post=post, mg_coarse_sweeps=sweeps, mg_coarsest=coarsest,
+                                mg_tail_side=side)
+    eng = native.Engine(nx, ny, params=prm)
+    try:
+        p, used, rr = p0.copy(), native.ctypes.c_int(), native.ctypes.c_double()
+        eng.call("fl_mg_solve", ptr(p), ptr(div), ptr(label), 0.02, 2, 1e-30, native.ctypes.byref(used),
+                 native.ctypes.byref(rr))
+    finally:
+        eng.close()
+    exp, _, rr32 = o32.mg_solve(nx, ny, p0, div, label, 0.02, 2, 1e-30, pre, post, sweeps, coarsest)
+    same(exp, p, "%dx%d" % (nx, ny))
+    assert used.value == 2 and abs(rr.value - rr32) <= 1e-9 * rr32
