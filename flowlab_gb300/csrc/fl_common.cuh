@@ -232,6 +232,16 @@ __device__ __forceinline__ bool solid_cell(const uint8_t* __restrict__ label, in
   return (unsigned)i < (unsigned)nx && (unsigned)j < (unsigned)ny && __ldg(label + i + j * nx) == SOLID;
 }
 
+// Programmatic dependent launch: a kernel launched with launch_dependent
+// (fl_internal.h) may start while the kernel before it drains. dep_wait blocks
+// until that kernel has completed and its results are visible (at once in a
+// kernel launched otherwise); before it, a kernel reads only what kernels
+// further back wrote. dep_trigger, after it, lets the next kernel start
+// likewise: so whoever runs ahead of its dep_wait has only its immediate
+// predecessor still running.
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dep_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Block-wide reductions (thread count a multiple of 32, <= 1024); the result
 // is valid in the block's first thread.
 __device__ inline double block_sum(double v, double* shm32) {

@@ -508,7 +508,7 @@ void enqueue_rb_fixed(Engine* e, cudaStream_t s) {
     const int chunk = std::min(per, iters - k);
     const int tok = prof_begin(*e, FL_PH_RB_SWEEPS);
     launch_rb_sweeps(s, L.nx, L.ny, L.x[src], L.x[1 - src], L.b, L.code, 0.0f, (float)e->prm.omega, chunk,
-                     &e->sc->scale);
+                     &e->sc->scale, k > 0);
     prof_end(*e, tok, 13.0 * e->cells(), 1);
     src = 1 - src;
     k += chunk;
@@ -569,7 +569,8 @@ int rb_solve_device(Engine* e, float scale, int iterations, float omega, double 
     int chunk = std::min(per, iterations - k);
     if (target >= 0) chunk = std::min(chunk, 12 - (k % 12));
     const int tok = prof_begin(*e, FL_PH_RB_SWEEPS);
-    launch_rb_sweeps(e->stream, L.nx, L.ny, L.x[src], L.x[1 - src], L.b, L.code, scale, omega, chunk);
+    launch_rb_sweeps(e->stream, L.nx, L.ny, L.x[src], L.x[1 - src], L.b, L.code, scale, omega, chunk, nullptr,
+                     k > 0 && !(target >= 0 && k % 12 == 0));
     prof_end(*e, tok, 13.0 * e->cells(), 1);
     TRY(check_launch(e, "red-black sweeps"));
     src = 1 - src;

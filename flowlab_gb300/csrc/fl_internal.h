@@ -185,6 +185,26 @@ void prof_end(Engine& e, int token, double bytes, int launches);
 // fl_engine.cu.
 void set_global_error(const char* fmt, ...);
 
+// A launch that may start while the kernel before it on the stream drains
+// (dep_wait, fl_common.cuh): only where that is a kernel, in the stream or the
+// captured graph, and only for kernels that call dep_wait. early = false: an
+// ordinary launch. Measured, V-cycles in a graph: 256^2 24.7 -> 20.5 us,
+// 1024^2 45.5 -> 40.9, 2048^2 82 -> 74.
+template <class... P, class... A>
+inline cudaError_t launch_dependent(bool early, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s,
+                                    const A&... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // ------------------------------------------------------------- launchers
 
 // fl_advect.cu
@@ -277,8 +297,9 @@ void launch_update_resid64(cudaStream_t s, int nx, int ny, double* p64a, double*
 void launch_solve_begin(cudaStream_t s, StepAccum* acc, SolveCtl* ctl, bool use_cond, cudaGraphConditionalHandle h);
 void launch_solve_check(cudaStream_t s, StepAccum* acc, SolveCtl* ctl, bool use_cond, cudaGraphConditionalHandle h);
 void launch_zero_if(cudaStream_t s, const SolveCtl* ctl, float* p32, double* p64a, double* p64b, long n);
+// early: the kernel before it on the stream is another of these launches
 void launch_rb_sweeps(cudaStream_t s, int nx, int ny, const float* x_in, float* x_out, const float* b,
-                      const uint8_t* code, float scale, float omega, int pairs, const float* scale_dev = nullptr);
+                      const uint8_t* code, float scale, float omega, int pairs, const float* scale_dev, bool early);
 void launch_rms_remaining(cudaStream_t s, int nx, int ny, const float* p, const float* div, const uint8_t* code,
                           float scale, StepAccum* acc);
 void launch_build_codes(cudaStream_t s, int nx, int ny, const uint8_t* label, uint8_t* code);

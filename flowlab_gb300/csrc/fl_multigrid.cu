@@ -213,35 +213,62 @@ __device__ __forceinline__ void smooth_tile(const SmoothArgs& a, int bx, int by,
 
   float x[RW][2], b[RW][2];
   unsigned cd[RW];  // the two cells' codes
-#pragma unroll
-  for (int r = 0; r < RW; r++) {
-    const int gj = row + r;
+  auto load_codes = [&](int r) {
+    const int gj = row + r, k = col + gj * nx;  // 32-bit offsets: a level holds fewer than 2^31 cells
     cd[r] = OUTSIDE2;
-    x[r][0] = x[r][1] = b[r][0] = b[r][1] = 0.0f;
-    if ((unsigned)gj < (unsigned)ny) {
-      const int k = col + gj * nx;  // 32-bit offsets: a level holds fewer than 2^31 cells
-      if (pair) {
-        if ((unsigned)col < (unsigned)nx) {
-          cd[r] = *reinterpret_cast<const unsigned short*>(a.code + k);
-          const float2 q = *reinterpret_cast<const float2*>(a.b + k);
-          b[r][0] = q.x;
-          b[r][1] = q.y;
-          if (!a.x_is_zero) {
-            const float2 p = *reinterpret_cast<const float2*>(a.xin + k);
-            x[r][0] = p.x;
-            x[r][1] = p.y;
-          }
-        }
-      } else {
+    if ((unsigned)gj >= (unsigned)ny) return;
+    if (pair) {
+      if ((unsigned)col < (unsigned)nx) cd[r] = *reinterpret_cast<const unsigned short*>(a.code + k);
+    } else {
 #pragma unroll
-        for (int o = 0; o < 2; o++)
-          if ((unsigned)(col + o) < (unsigned)nx) {
-            cd[r] = (cd[r] & (o ? 0x00ffu : 0xff00u)) | (unsigned)a.code[k + o] << (8 * o);
-            b[r][o] = a.b[k + o];
-            if (!a.x_is_zero) x[r][o] = a.xin[k + o];
-          }
-      }
+      for (int o = 0; o < 2; o++)
+        if ((unsigned)(col + o) < (unsigned)nx)
+          cd[r] = (cd[r] & (o ? 0x00ffu : 0xff00u)) | (unsigned)a.code[k + o] << (8 * o);
     }
+  };
+  auto load_values = [&](int r) {
+    const int gj = row + r, k = col + gj * nx;
+    x[r][0] = x[r][1] = b[r][0] = b[r][1] = 0.0f;
+    if ((unsigned)gj >= (unsigned)ny) return;
+    if (pair) {
+      if ((unsigned)col < (unsigned)nx) {
+        const float2 q = *reinterpret_cast<const float2*>(a.b + k);
+        b[r][0] = q.x;
+        b[r][1] = q.y;
+        if (!a.x_is_zero) {
+          const float2 p = *reinterpret_cast<const float2*>(a.xin + k);
+          x[r][0] = p.x;
+          x[r][1] = p.y;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int o = 0; o < 2; o++)
+        if ((unsigned)(col + o) < (unsigned)nx) {
+          b[r][o] = a.b[k + o];
+          if (!a.x_is_zero) x[r][o] = a.xin[k + o];
+        }
+    }
+  };
+  // Before dep_wait: the codes (built long before), and on the way up b and x,
+  // which this level's PRE launch and the finer one's wrote; only the coarse
+  // correction comes from the launch before. On the way down b does.
+#pragma unroll
+  for (int r = 0; r < RW; r++) load_codes(r);
+  if (MODE == MODE_POST) {
+#pragma unroll
+    for (int r = 0; r < RW; r++) load_values(r);
+  }
+  if (tid < 64) sh.lut[tid] = link_factors(tid);
+  if (w == 0) {
+    sh.edge[0][0][1][lane] = sh.edge[1][0][1][lane] = 0.0f;
+    sh.edge[0][NW + 1][0][lane] = sh.edge[1][NW + 1][0][lane] = 0.0f;
+  }
+  dep_wait();
+  dep_trigger();
+  if (MODE != MODE_POST) {
+#pragma unroll
+    for (int r = 0; r < RW; r++) load_values(r);
   }
   if constexpr (MODE == MODE_POST) {
     // pressureMultigrid.ts:192-207 — a fluid cell's x += 9/16, 3/16, 3/16,
@@ -258,8 +285,8 @@ __device__ __forceinline__ void smooth_tile(const SmoothArgs& a, int bx, int by,
 #pragma unroll
     for (int q = 0; q < RW / 2 + 2; q++) {
       const float* e = a.ec + min(max(J0 - 1 + q, 0), a.cny - 1) * a.cnx;
-      eM[q] = __ldg(e + cm);
-      eL[q] = end ? __ldg(e + ce) : 0.0f;
+      eM[q] = e[cm];
+      eL[q] = end ? e[ce] : 0.0f;
     }
 #pragma unroll
     for (int q = 0; q < RW / 2 + 2; q++) {
@@ -278,11 +305,6 @@ __device__ __forceinline__ void smooth_tile(const SmoothArgs& a, int bx, int by,
     }
   }
 
-  if (tid < 64) sh.lut[tid] = link_factors(tid);
-  if (w == 0) {
-    sh.edge[0][0][1][lane] = sh.edge[1][0][1][lane] = 0.0f;
-    sh.edge[0][NW + 1][0][lane] = sh.edge[1][NW + 1][0][lane] = 0.0f;
-  }
   __syncthreads();
 
   // the warp's form: every cell fluid with four links, or not (then its
@@ -770,6 +792,8 @@ __device__ __forceinline__ void mg_coarse_body(const CoarseArgs& a, TailShared<T
   }
   if (tid < 64) sh.lut[tid] = link_factors(tid);
   __syncthreads();
+  dep_wait();
+  dep_trigger();
   double rsq = 0.0;
   unsigned long long rn = 0;
   tail_frame<TOP>(a, sh.f, sh.lut, code, tid, rsq, rn);
@@ -1257,19 +1281,29 @@ __global__ void k_rb_halfsweep(int nx, int ny, float* __restrict__ p, const floa
 // ------------------------------------------------------------- host side
 
 template <int MODE, int NW, int RW>
-static void launch_smooth_nw(cudaStream_t s, const SmoothArgs& a) {
+static void launch_smooth_nw(cudaStream_t s, const SmoothArgs& a, bool early) {
   const int tx = 64 - 2 * a.halo, ty = RW * NW - 2 * a.halo;
-  k_smooth<MODE, NW, RW><<<dim3((a.nx + tx - 1) / tx, (a.ny + ty - 1) / ty), 32 * NW, 0, s>>>(a);
+  launch_dependent(early, k_smooth<MODE, NW, RW>, dim3((a.nx + tx - 1) / tx, (a.ny + ty - 1) / ty), dim3(32 * NW), s, a);
 }
 
-static void launch_smooth(cudaStream_t s, SmoothArgs a, int pairs, int mode) {
+template <int MODE>
+static void launch_smooth_mode(cudaStream_t s, const SmoothArgs& a, bool early) {
+  const int t = 64 - 2 * a.halo;
+  if ((long)((a.nx + t - 1) / t) * ((a.ny + t - 1) / t) < SMOOTH_SMALL)
+    launch_smooth_nw<MODE, 16, 2>(s, a, early);
+  else
+    launch_smooth_nw<MODE, 8, 8>(s, a, early);
+}
+
+static void launch_smooth(cudaStream_t s, SmoothArgs a, int pairs, int mode, bool early) {
   a.pairs = pairs;
   a.halo = smooth_halo(mode, pairs, a.x_is_zero, a.acc != nullptr);
-  const int t = 64 - 2 * a.halo;
-  const bool small = (long)((a.nx + t - 1) / t) * ((a.ny + t - 1) / t) < SMOOTH_SMALL;
-  if (mode == MODE_PLAIN) small ? launch_smooth_nw<MODE_PLAIN, 16, 2>(s, a) : launch_smooth_nw<MODE_PLAIN, 8, 8>(s, a);
-  else if (mode == MODE_PRE) small ? launch_smooth_nw<MODE_PRE, 16, 2>(s, a) : launch_smooth_nw<MODE_PRE, 8, 8>(s, a);
-  else small ? launch_smooth_nw<MODE_POST, 16, 2>(s, a) : launch_smooth_nw<MODE_POST, 8, 8>(s, a);
+  if (mode == MODE_PLAIN)
+    launch_smooth_mode<MODE_PLAIN>(s, a, early);
+  else if (mode == MODE_PRE)
+    launch_smooth_mode<MODE_PRE>(s, a, early);
+  else
+    launch_smooth_mode<MODE_POST>(s, a, early);
 }
 
 static void launch_level_codes(cudaStream_t s, int nx, int ny, const uint8_t* label, uint8_t* code, uint8_t* coarse,
@@ -1289,7 +1323,7 @@ void launch_rb_halfsweep(cudaStream_t s, int nx, int ny, float* p, const float* 
 }
 
 void launch_rb_sweeps(cudaStream_t s, int nx, int ny, const float* x_in, float* x_out, const float* b,
-                      const uint8_t* code, float scale, float omega, int pairs, const float* scale_dev) {
+                      const uint8_t* code, float scale, float omega, int pairs, const float* scale_dev, bool early) {
   SmoothArgs a{};
   a.scale_dev = scale_dev;
   a.nx = nx;
@@ -1300,7 +1334,7 @@ void launch_rb_sweeps(cudaStream_t s, int nx, int ny, const float* x_in, float* 
   a.code = code;
   a.scale = scale;
   a.omega = omega;
-  launch_smooth(s, a, pairs, MODE_PLAIN);
+  launch_smooth(s, a, pairs, MODE_PLAIN, early);
 }
 
 template <bool UPDATE>
@@ -1527,7 +1561,7 @@ void mg_vcycle_on(Engine& e, const float* b0, bool zero_start, StepAccum* acc) {
     a.cnx = C.nx;
     a.cny = C.ny;
     a.x_is_zero = l > 0 || zero_start;
-    launch_smooth(s, a, e.prm.mg_pre, MODE_PRE);
+    launch_smooth(s, a, e.prm.mg_pre, MODE_PRE, l > 0);
     prof_end(e, tok, (l == 0 ? 13.0 : 9.0) * cells(l) + 4.0 * cells(l + 1), 1);
   }
   {
@@ -1535,10 +1569,9 @@ void mg_vcycle_on(Engine& e, const float* b0, bool zero_start, StepAccum* acc) {
     double bytes = (lc == 0 ? 4.0 : 0.0) * cells(lc) + 8.0 * cells(lc);
     for (int l = lc; l < (int)e.levels.size(); l++) bytes += cells(l);
     const CoarseArgs a = coarse_args(e, b0, zero_start, acc);
-    if (a.frame == 64)
-      k_mg_coarse<64><<<1, tail_threads(a.frame), 0, s>>>(a);
-    else
-      k_mg_coarse<32><<<1, tail_threads(a.frame), 0, s>>>(a);
+    // (lc == 0: the V-cycle's first launch)
+    launch_dependent(lc > 0, a.frame == 64 ? k_mg_coarse<64> : k_mg_coarse<32>, dim3(1), dim3(tail_threads(a.frame)), s,
+                     a);
     prof_end(e, tok, bytes, 1);
   }
   for (int l = lc - 1; l >= 0; l--) {
@@ -1559,7 +1592,7 @@ void mg_vcycle_on(Engine& e, const float* b0, bool zero_start, StepAccum* acc) {
     a.cnx = C.nx;
     a.cny = C.ny;
     a.acc = l == 0 ? acc : nullptr;
-    launch_smooth(s, a, e.prm.mg_post, MODE_POST);
+    launch_smooth(s, a, e.prm.mg_post, MODE_POST, true);
     prof_end(e, tok, 13.0 * cells(l) + 4.0 * cells(l + 1), 1);
   }
 }
