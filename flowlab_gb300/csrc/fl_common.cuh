@@ -330,6 +330,34 @@ __device__ __forceinline__ double f2d_exact(float f) {
   return f2d_slow(f);
 }
 
+static __device__ __noinline__ double fsum_slow(float a, float b) { return (double)a + (double)b; }
+
+// (double)a + (double)b on the integer pipe where b is the rounding error of a
+// rounded to float (|b| at most half a unit of a's last place, so the sum is
+// exact and stays within a binade of a): adding k units in the last place of a
+// double is adding k to its bits, 2 k below a power of two. Other cases (a or
+// b zero, subnormal, infinite or NaN; exponents less than 24 or more than 52
+// apart, or b's bits beyond the sum's last place) take the addition. Equal to
+// it in every case but for the sign of a zero sum.
+__device__ __forceinline__ double sum_exact(float a, float b) {
+  const unsigned ua = __float_as_uint(a), ub = __float_as_uint(b);
+  const int ea = (int)(ua >> 23 & 0xffu), eb = (int)(ub >> 23 & 0xffu), sh = 29 - (ea - eb);
+  const unsigned mb = (ub & 0x7fffffu) | 0x800000u;
+  const bool fast = ea != 0xff && eb != 0 && sh <= 5 && sh > -23 && (sh >= 0 || (mb & ((1u << (-sh & 31)) - 1u)) == 0u);
+  if (fast) {
+    unsigned k = sh >= 0 ? mb << (sh & 31) : mb >> (-sh & 31);
+    const bool minus = (ua ^ ub) >> 31;
+    if (minus && (ua & 0x7fffffu) == 0u) k += k;
+    const long long d = minus ? -(long long)k : (long long)k;
+    const unsigned long long bits = (unsigned long long)(ua >> 31) << 63 | ((unsigned long long)(ea + 896) << 52) |
+                                    ((unsigned long long)(ua & 0x7fffffu) << 29);
+    return dfrom_opaque(bits + (unsigned long long)d);
+  }
+  if ((ub & 0x7fffffffu) == 0u && ea != 0xff && ea != 0)  // b is 0: a itself
+    return f2d_exact(a);
+  return fsum_slow(a, b);
+}
+
 // x * 2^k (k = 1, 2) by an exponent increment when x is normal and the
 // product stays normal; zero returns itself (as x * 2^k does); otherwise
 // the multiply. Equal to x * 2^k in every case.
@@ -393,14 +421,12 @@ __device__ __forceinline__ float2 df_add_f(float2 x, float f) {
   const float e = __fadd_rn(s.y, x.y);
   return df_fast_two_sum(s.x, e);
 }
-// count * x for a link count 1..4 (2 and 4 scale exactly)
-__device__ __forceinline__ float2 df_mul_count(float2 x, int count) {
-  if (count == 4) return make_float2(__fmul_rn(4.0f, x.x), __fmul_rn(4.0f, x.y));
-  if (count == 2) return make_float2(__fmul_rn(2.0f, x.x), __fmul_rn(2.0f, x.y));
-  if (count == 1) return x;
-  const float p = __fmul_rn(3.0f, x.x);
-  float e = __fmaf_rn(3.0f, x.x, -p);
-  e = __fmaf_rn(3.0f, x.y, e);
+// count * x for a link count 0..4, without a branch: the product by one exact
+// FMA; a count that is a power of two leaves the pair as it is, scaled.
+__device__ __forceinline__ float2 df_mul_count(float2 x, float count) {
+  const float p = __fmul_rn(count, x.x);
+  float e = __fmaf_rn(count, x.x, -p);
+  e = __fmaf_rn(count, x.y, e);
   return df_fast_two_sum(p, e);
 }
 __device__ __forceinline__ float df_round(float2 x) { return __fadd_rn(x.x, x.y); }

@@ -860,98 +860,122 @@ __global__ void __launch_bounds__(1024) k_tail_labels(TailLabels a, const int* o
   tail_codes<64>(a, 0, a.nx, a.ny);
 }
 
-// The float64 defect-correction pass (iterative refinement, solveMixed):
-// p64' = p64 + e (when `update`), then r = b - (count*p64' - sum) in double
-// with the neighbour sum in the order +x, -x, +y, -y, r32 = float(r), and
-// the squared norm of r accumulated. GB300 issues float64 arithmetic at about
-// 1.6 lanes per clock per SM (measured; 32-bit integer adds: ~100), so this
-// pass is bound by its float64 instructions, not by memory, and spends them
-// only where the result needs them: each p64' is formed once and handed to
-// its neighbours in registers (the rows above and below) and by warp
-// shuffles (left and right); the exact float -> double widenings, the first
-// addition to 0.0, the products by 2 and 4 and the rounding of r to float
-// run on the integer pipe with identical results (fl_common.cuh), with their
-// rare cases out of line and their bit casts opaque, so that the compiler
-// neither predicates nor re-forms float64 instructions into every cell.
-// A warp owns 30 interior columns (lanes 1..30; lanes 0 and 31 are the halo
-// columns, formed redundantly) and walks UR_ROWS rows as a rolling window
-// (row above, row, row below), the raw values of the row two below loaded one
-// iteration ahead of their use.
-// 16 rows per warp, 4 warps per block (measured at 1024^2, per step of 5
-// passes: 128.5 us against 131.1 with 8 x 8 and 156 with 32-row warps, whose
-// grid leaves too few warps to cover the float64 latency)
-constexpr int UR_ROWS = 16;
-constexpr int UR_WARPS = 4;
+// ----------------------------------------------------- the defect-correction pass
+//
+// p' = p + e (when `update`), r = b - (count*p' - sum) in extended precision
+// with the neighbour sum in the order +x, -x, +y, -y, r32 = float(r), and the
+// squared norm of r accumulated: the finest level's part of a defect-
+// correction cycle (iterative refinement, solveMixed), in float64 or in
+// double-float pairs. A warp owns the interior columns of its lanes (the
+// first and last lane hold the halo) and RW rows; every load of its first rows is issued before any arithmetic,
+// all but e's before the launch waits for the smoother that writes e (e is not
+// restrict: its loads must not move above that wait). Each p'
+// is formed once a warp and handed to its neighbours in registers (the rows
+// above and below) and by shuffles (left and right).
+//
+// (the rows a warp: defect_rows).
+constexpr int DEFECT_WARPS = 4;
+// Columns a block owns.
+__host__ __device__ constexpr int defect_cols(bool df) { return df ? 60 : 30; }
 
-// One block's rows of the float64 pass: block (bx, by) of its grid.
-template <bool UPDATE>
+// Sums the block's norm in its first thread and adds it to the accumulators:
+// a warp's lanes by shuffles, then the first thread over the warps (a second
+// tree over 32 lanes for 4 values cost as much as the first).
+// n: the warp's count, the same in every lane.
+template <class T, class Add, class Wide>
+__device__ __forceinline__ void defect_norm(T v, int n, Add add, Wide wide, StepAccum* acc) {
+  __shared__ T part[DEFECT_WARPS];
+  __shared__ int parts[DEFECT_WARPS];
+  for (int o = 16; o > 0; o >>= 1) v = add(v, o);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (lane == 0) {
+    part[w] = v;
+    parts[w] = n;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = wide(part[0]);
+    int m = parts[0];
+    for (int k = 1; k < DEFECT_WARPS; k++) {
+      s += wide(part[k]);
+      m += parts[k];
+    }
+    atomicAdd(&acc->res_sq, s);
+    atomicAdd(&acc->n_res, (unsigned long long)m);
+  }
+}
+
+// The float64 pass. GB300 issues float64 arithmetic at about 2 lanes per
+// clock per SM (32-bit integer adds: ~100), so this pass is bound by its
+// float64 instructions, not by memory, and spends them only where the result
+// needs them: the exact float -> double widenings, b + b_lo, the first
+// addition to 0.0, the products by 2 and 4 and the rounding of r to float run
+// on the integer pipe with identical results (fl_common.cuh), with their rare
+// cases out of line and their bit casts opaque, so that the compiler neither
+// predicates nor re-forms float64 instructions into every cell.
+// One block's rows of the pass: block (bx, by) of its grid.
+template <bool UPDATE, int RW>
 __device__ __forceinline__ void update_resid64_tile(int nx, int ny, double* __restrict__ p64a,
                                                     double* __restrict__ p64b, const SolveCtl* ctl,
-                                                    const float* __restrict__ e, const float* __restrict__ b,
+                                                    const float* e, const float* __restrict__ b,
                                                     const float* __restrict__ b_lo,
                                                     const uint8_t* __restrict__ code, float* __restrict__ r32,
                                                     StepAccum* acc, int bx, int by) {
-  __shared__ double red[32];
-  __shared__ unsigned long long redn[32];
   const int par = ctl->par;
   const double* p_in = par ? p64b : p64a;
   double* p_out = par ? p64a : p64b;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int gx = bx * 30 - 1 + lane;
-  const int y0 = (by * UR_WARPS + w) * UR_ROWS;
+  const int y0 = (by * DEFECT_WARPS + w) * RW;
   const bool col = gx >= 0 && gx < nx;
   const bool own = col && lane != 0 && lane != 31;
 
-  // raw p64 and e of row y (zero outside the grid), and p64' formed from them
-  auto raw = [&](int y, double& rp, float& re) {
-    rp = 0.0;
-    re = 0.0f;
-    if (col && y >= 0 && y < ny) {
-      const int k = gx + y * nx;
-      rp = p_in[k];
-      if (UPDATE) re = e[k];
+  // rows y0-1 .. y0+RW of p and e, rows y0 .. y0+RW-1 of the rest; zero /
+  // outside where the grid ends. 32-bit offsets: a grid holds fewer than 2^31 cells
+  double P[RW + 2];
+  float E[RW + 2], B[RW], BL[RW];
+  uint8_t C[RW];
+#pragma unroll
+  for (int r = 0; r < RW + 2; r++) {
+    const int y = y0 - 1 + r;
+    P[r] = col && (unsigned)y < (unsigned)ny ? p_in[gx + y * nx] : 0.0;
+  }
+#pragma unroll
+  for (int r = 0; r < RW; r++) {
+    const int y = y0 + r;
+    const bool in = own && y < ny;
+    B[r] = in ? b[gx + y * nx] : 0.0f;
+    BL[r] = in ? b_lo[gx + y * nx] : 0.0f;
+    C[r] = in ? code[gx + y * nx] : (uint8_t)CODE_OUTSIDE;
+  }
+  dep_wait();
+  if (UPDATE) {
+#pragma unroll
+    for (int r = 0; r < RW + 2; r++) {
+      const int y = y0 - 1 + r;
+      E[r] = col && (unsigned)y < (unsigned)ny ? e[gx + y * nx] : 0.0f;
     }
-  };
-  auto form = [](double rp, float re) { return UPDATE ? rp + f2d_exact(re) : rp; };
-  double rp, rp0;
-  float re, re0;
-  raw(y0 - 1, rp0, re0);
-  raw(y0, rp, re);
-  double pm = form(rp0, re0), pc = form(rp, re);
-  raw(y0 + 1, rp, re);
-  float bnext = 0.0f, blnext = 0.0f;
-  uint8_t cnext = (uint8_t)CODE_OUTSIDE;
-  if (own && y0 < ny) {
-    const int k = gx + y0 * nx;
-    bnext = b[k];
-    blnext = b_lo[k];
-    cnext = code[k];
+#pragma unroll
+    for (int r = 0; r < RW + 2; r++) P[r] = P[r] + f2d_exact(E[r]);
   }
 
   double sq = 0.0;
-  unsigned long long n = 0;
-#pragma unroll 1
-  for (int t = 0; t < UR_ROWS; t++) {
+  int n = 0;
+#pragma unroll
+  for (int t = 0; t < RW; t++) {
     const int gy = y0 + t;
-    if (gy >= ny) break;  // the same for the whole warp
-    const double pp = form(rp, re);
-    raw(gy + 2, rp, re);
-    const float bv = bnext, blv = blnext;
-    const uint8_t c = cnext;
-    if (own && gy + 1 < ny && t + 1 < UR_ROWS) {
-      const int k = gx + (gy + 1) * nx;
-      bnext = b[k];
-      blnext = b_lo[k];
-      cnext = code[k];
-    }
+    const double pc = P[t + 1];
     const double left = __shfl_up_sync(0xffffffffu, pc, 1);
     const double right = __shfl_down_sync(0xffffffffu, pc, 1);
-    if (own) {
+    const uint8_t c = C[t];
+    const int cnt = code_count(c);
+    const bool on = (c & 3u) == FLUID && cnt > 0;
+    n += __popc(__ballot_sync(0xffffffffu, on));
+    if (own && gy < ny) {
       const int k = gx + gy * nx;
       if (UPDATE) p_out[k] = pc;
       float r = 0.0f;
-      const int cnt = code_count(c);
-      if ((c & 3u) == FLUID && cnt > 0) {
+      if (on) {
         // the first linked term enters as 0.0 + term
         double sum;
         bool first = true;
@@ -964,153 +988,207 @@ __device__ __forceinline__ void update_resid64_tile(int nx, int ny, double* __re
           first = false;
         }
         if (c & LINK_YP) {
-          sum = first ? zero_plus(pp) : sum + pp;
+          sum = first ? zero_plus(P[t + 2]) : sum + P[t + 2];
           first = false;
         }
-        if (c & LINK_YM) sum = first ? zero_plus(pm) : sum + pm;
+        if (c & LINK_YM) sum = first ? zero_plus(P[t]) : sum + P[t];
         const double cp = cnt == 4 ? scale_pow2(pc, 2)
                           : cnt == 2 ? scale_pow2(pc, 1)
                           : cnt == 1 ? pc
                                      : dmul_slow(pc, 3.0);
-        // b + b_lo is exact in double (at most 49 significant bits)
-        const double rd = (f2d_exact(bv) + f2d_exact(blv)) - (cp - sum);
+        const double rd = sum_exact(B[t], BL[t]) - (cp - sum);
         r = d2f_rn(rd);
         sq = fma(rd, rd, sq);
-        n += 1;
       }
       r32[k] = r;
     }
-    pm = pc;
-    pc = pp;
   }
-  const double bs = block_sum(sq, red);
-  const unsigned long long bn = block_sum_u64(n, redn);
-  if (threadIdx.x == 0) {
-    atomicAdd(&acc->res_sq, bs);
-    atomicAdd(&acc->n_res, bn);
-  }
+  defect_norm(
+      sq, n, [](double a, int o) { return a + __shfl_down_sync(0xffffffffu, a, o); },
+      [](double a) { return a; }, acc);
 }
 
 // The same pass with the double-float pressure (fl_params.mixed = 2): p' =
-// p + e per cell (df_add_f), then r = b - (count*p' - sum) in double-float
-// arithmetic, the neighbour sum in the order +x, -x, +y, -y starting from
-// the first linked neighbour, r32 = the pair rounded to float. All of it is
-// float32 arithmetic (~80 operations per cell), so unlike the float64 pass
-// this one is bound by memory, not by a pipe: a warp owns 30 interior
-// columns (lanes 1..30; lanes 0 and 31 load the halo columns) of DF_ROWS
-// rows and issues every load of its rows (DF_ROWS + 2 rows of p and e,
-// DF_ROWS of b and codes) before any arithmetic, so each warp waits for
-// memory once. The residual norm sums r32^2: each square is an exact pair
-// (the product and its FMA error), accumulated per thread as a double-float
-// and widened to double once per thread for the block reduction.
-// At 64 registers 8 blocks fit an SM, so a 1024^2 grid's 1120 blocks run
-// in one wave (at 72 registers, 7 per SM, the last 56 blocks made a second).
-constexpr int DF_ROWS = 8;
-constexpr int DF_WARPS = 4;
-
-// One block's rows of the double-float pass: block (bx, by) of its grid.
+// p + e per cell (df_add_f), then r in double-float arithmetic, the neighbour
+// sum starting from the first linked neighbour, r32 = the pair rounded to
+// float. All of it is float32 arithmetic (~100 operations per cell), which
+// bounds it. A lane owns a pair of columns (16-byte loads of p where the rows
+// allow it), so half of the horizontal neighbours are its own. A warp walks
+// its rows two at a time, the next two loaded before the arithmetic (unrolled
+// over 8 rows, the code outgrew the instruction cache: 2.6 of 8.9 stall cycles
+// an instruction). The residual norm sums r32^2: each
+// square is an exact pair (the product and its FMA error), accumulated as a
+// double-float and widened to double once a warp.
 template <bool UPDATE>
 __device__ __forceinline__ void update_resid_df_tile(int nx, int ny, float2* __restrict__ p2a,
                                                      float2* __restrict__ p2b, const SolveCtl* ctl,
-                                                     const float* __restrict__ e, const float* __restrict__ b,
+                                                     const float* e, const float* __restrict__ b,
                                                      const float* __restrict__ b_lo,
                                                      const uint8_t* __restrict__ code, float* __restrict__ r32,
-                                                     StepAccum* acc, int bx, int by) {
-  __shared__ double red[32];
-  __shared__ unsigned long long redn[32];
+                                                     StepAccum* acc, int bx, int by, int rows) {
   const int par = ctl->par;
   const float2* p_in = par ? p2b : p2a;
   float2* p_out = par ? p2a : p2b;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int gx = bx * 30 - 1 + lane;
-  const int y0 = (by * DF_WARPS + w) * DF_ROWS;
-  const bool col = gx >= 0 && gx < nx;
-  const bool own = col && lane != 0 && lane != 31;
+  const int gx = bx * 60 - 2 + 2 * lane;  // even: the lane's first column
+  const int y0 = (by * DEFECT_WARPS + w) * rows, y1 = min(y0 + rows, ny);
+  const bool pair = (nx & 1) == 0;  // rows start at multiples of 16 bytes of p: the lane's columns are in or out together
+  const bool in0 = (unsigned)gx < (unsigned)nx, in1 = (unsigned)(gx + 1) < (unsigned)nx;
+  const bool mine = lane != 0 && lane != 31;
+  constexpr unsigned OUTSIDE2 = CODE_OUTSIDE | (unsigned)CODE_OUTSIDE << 8;
+  // a neighbour where the link bit is set, else 0, which leaves a sum as it is
+  // (pairs are normalised): no lane-divergent branches
+  auto linked = [](float2 v, unsigned bit) {
+    const int m = -(int)(bit & 1u);
+    return make_float2(masked(v.x, m), masked(v.y, m));
+  };
 
-  // rows y0-1 .. y0+DF_ROWS of p (and e), rows y0 .. y0+DF_ROWS-1 of b and
-  // the codes; zero / outside where the grid ends
-  float2 P[DF_ROWS + 2];
-  float E[DF_ROWS + 2];
-  float B[DF_ROWS], BL[DF_ROWS];
-  uint8_t C[DF_ROWS];
-#pragma unroll
-  for (int r = 0; r < DF_ROWS + 2; r++) {
-    const int y = y0 - 1 + r;
-    P[r] = make_float2(0.0f, 0.0f);
-    E[r] = 0.0f;
-    if (col && y >= 0 && y < ny) {
-      const int k = gx + y * nx;  // 32-bit offsets: a grid holds fewer than 2^31 cells
-      P[r] = p_in[k];
-      if (UPDATE) E[r] = e[k];
+  // row y of the lane's pair (0 / outside beyond the grid); 32-bit offsets: a
+  // grid holds fewer than 2^31 cells
+  auto load2 = [&](const float* f, int y, bool ok) {
+    float2 v = make_float2(0.0f, 0.0f);
+    const int k = gx + y * nx;
+    if (pair) {
+      if (ok && in0) v = *reinterpret_cast<const float2*>(f + k);
+    } else {
+      if (ok && in0) v.x = f[k];
+      if (ok && in1) v.y = f[k + 1];
     }
-  }
-#pragma unroll
-  for (int r = 0; r < DF_ROWS; r++) {
-    const int y = y0 + r;
-    B[r] = 0.0f;
-    BL[r] = 0.0f;
-    C[r] = (uint8_t)CODE_OUTSIDE;
-    if (own && y < ny) {
-      const int k = gx + y * nx;
-      B[r] = b[k];
-      BL[r] = b_lo[k];
-      C[r] = code[k];
-    }
-  }
-  if (UPDATE) {
-#pragma unroll
-    for (int r = 0; r < DF_ROWS + 2; r++) P[r] = df_add_f(P[r], E[r]);
-  }
-
-  float2 acc2 = make_float2(0.0f, 0.0f);
-  unsigned long long n = 0;
-#pragma unroll
-  for (int t = 0; t < DF_ROWS; t++) {
-    const int gy = y0 + t;
-    const float2 pc = P[t + 1];
-    const float2 left = make_float2(__shfl_up_sync(0xffffffffu, pc.x, 1), __shfl_up_sync(0xffffffffu, pc.y, 1));
-    const float2 right =
-        make_float2(__shfl_down_sync(0xffffffffu, pc.x, 1), __shfl_down_sync(0xffffffffu, pc.y, 1));
-    if (own && gy < ny) {
-      const int k = gx + gy * nx;
-      if (UPDATE) p_out[k] = pc;
-      const uint8_t c = C[t];
-      float r = 0.0f;
-      const int cnt = code_count(c);
-      if ((c & 3u) == FLUID && cnt > 0) {
-        const float2 pp = P[t + 2], pm = P[t];
-        float2 sum = make_float2(0.0f, 0.0f);
-        bool first = true;
-        if (c & LINK_XP) {
-          sum = right;
-          first = false;
-        }
-        if (c & LINK_XM) {
-          sum = first ? left : df_add(sum, left);
-          first = false;
-        }
-        if (c & LINK_YP) {
-          sum = first ? pp : df_add(sum, pp);
-          first = false;
-        }
-        if (c & LINK_YM) sum = first ? pm : df_add(sum, pm);
-        const float2 d = df_add(df_mul_count(pc, cnt), df_neg(sum));
-        // (b + b_lo) - d: b_lo (the rhs's rounding error) joins the low parts
-        const float2 s = df_two_sum(B[t], -d.x);
-        r = __fadd_rn(s.x, __fadd_rn(s.y, __fsub_rn(BL[t], d.y)));
-        const float q = __fmul_rn(r, r);
-        acc2 = df_add(acc2, make_float2(q, __fmaf_rn(r, r, -q)));
-        n += 1;
+    return v;
+  };
+  auto load_p = [&](int y, float2* v) {
+    const int k = gx + y * nx;
+    const bool ok = (unsigned)y < (unsigned)ny;
+    v[0] = v[1] = make_float2(0.0f, 0.0f);
+    if (pair) {
+      if (ok && in0) {
+        const float4 q = *reinterpret_cast<const float4*>(p_in + k);
+        v[0] = make_float2(q.x, q.y);
+        v[1] = make_float2(q.z, q.w);
       }
-      r32[k] = r;
+    } else {
+      if (ok && in0) v[0] = p_in[k];
+      if (ok && in1) v[1] = p_in[k + 1];
+    }
+  };
+  auto load_code = [&](int y, bool ok) {
+    const int k = gx + y * nx;
+    unsigned c = OUTSIDE2;
+    if (pair) {
+      if (ok && in0) c = *reinterpret_cast<const unsigned short*>(code + k);
+    } else {
+      if (ok && in0) c = (c & 0xff00u) | code[k];
+      if (ok && in1) c = (c & 0x00ffu) | (unsigned)code[k + 1] << 8;
+    }
+    return c;
+  };
+  auto form = [](float2* v, float2 x) {
+    if (UPDATE) {
+      v[0] = df_add_f(v[0], x.x);
+      v[1] = df_add_f(v[1], x.y);
+    }
+  };
+
+  float2 P[4][2], N[2][2];  // rows y-1 .. y+2 of p', and the raw rows y+3, y+4
+  float2 E[2], B[2], BL[2];
+  unsigned C[2];
+#pragma unroll
+  for (int r = 0; r < 4; r++) load_p(y0 - 1 + r, P[r]);
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    const bool ok = mine && y0 + r < y1;
+    B[r] = load2(b, y0 + r, ok);
+    BL[r] = load2(b_lo, y0 + r, ok);
+    C[r] = load_code(y0 + r, ok);
+  }
+  dep_wait();
+  if (UPDATE) {
+    float2 e0[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) e0[r] = load2(e, y0 - 1 + r, (unsigned)(y0 - 1 + r) < (unsigned)ny);
+#pragma unroll
+    for (int r = 0; r < 4; r++) form(P[r], e0[r]);
+  }
+
+  float2 sq = make_float2(0.0f, 0.0f);
+  int n = 0;
+#pragma unroll 1
+  for (int y = y0; y < y1; y += 2) {
+    const bool more = y + 2 < y1;  // the same for the whole warp
+    float2 B1[2], BL1[2];
+    unsigned C1[2];
+    if (more) {
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        const bool ok = mine && y + 2 + r < y1;
+        load_p(y + 3 + r, N[r]);
+        if (UPDATE) E[r] = load2(e, y + 3 + r, y + 3 + r < ny);
+        B1[r] = load2(b, y + 2 + r, ok);
+        BL1[r] = load2(b_lo, y + 2 + r, ok);
+        C1[r] = load_code(y + 2 + r, ok);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+      const float2 p0 = P[t + 1][0], p1 = P[t + 1][1];
+      const float2 left = make_float2(__shfl_up_sync(0xffffffffu, p1.x, 1), __shfl_up_sync(0xffffffffu, p1.y, 1));
+      const float2 right =
+          make_float2(__shfl_down_sync(0xffffffffu, p0.x, 1), __shfl_down_sync(0xffffffffu, p0.y, 1));
+      float res[2];
+#pragma unroll
+      for (int o = 0; o < 2; o++) {
+        const float2 pc = o ? p1 : p0, xp = o ? right : p1, xm = o ? p0 : left, yp = P[t + 2][o], ym = P[t][o];
+        const unsigned c = C[t] >> (8 * o) & 0xffu;
+        const int cnt = code_count((uint8_t)c);
+        const bool on = (c & 3u) == FLUID && cnt > 0;
+        n += __popc(__ballot_sync(0xffffffffu, on));
+        const float2 sum = df_add(df_add(df_add(linked(xp, c >> 2), linked(xm, c >> 3)), linked(yp, c >> 4)),
+                                  linked(ym, c >> 5));
+        const float2 d = df_add(df_mul_count(pc, (float)cnt), df_neg(sum));
+        // (b + b_lo) - d: b_lo (the rhs's rounding error) joins the low parts
+        const float2 s = df_two_sum(o ? B[t].y : B[t].x, -d.x);
+        const float r = __fadd_rn(s.x, __fadd_rn(s.y, __fsub_rn(o ? BL[t].y : BL[t].x, d.y)));
+        res[o] = on ? r : 0.0f;
+        const float q = __fmul_rn(res[o], res[o]);
+        sq = df_add(sq, make_float2(q, __fmaf_rn(res[o], res[o], -q)));
+      }
+      const int gy = y + t, k = gx + gy * nx;
+      if (mine && gy < y1) {
+        if (pair) {
+          if (in0) {
+            if (UPDATE) *reinterpret_cast<float4*>(p_out + k) = make_float4(p0.x, p0.y, p1.x, p1.y);
+            *reinterpret_cast<float2*>(r32 + k) = make_float2(res[0], res[1]);
+          }
+        } else {
+          if (in0) {
+            if (UPDATE) p_out[k] = p0;
+            r32[k] = res[0];
+          }
+          if (in1) {
+            if (UPDATE) p_out[k + 1] = p1;
+            r32[k + 1] = res[1];
+          }
+        }
+      }
+    }
+    if (more) {
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        form(N[r], E[r]);
+        P[r][0] = P[r + 2][0], P[r][1] = P[r + 2][1];
+        P[r + 2][0] = N[r][0], P[r + 2][1] = N[r][1];
+        B[r] = B1[r];
+        BL[r] = BL1[r];
+        C[r] = C1[r];
+      }
     }
   }
-  const double bs = block_sum_df(acc2, reinterpret_cast<float2*>(red));
-  const unsigned long long bn = block_sum_u64(n, redn);
-  if (threadIdx.x == 0) {
-    atomicAdd(&acc->res_sq, bs);
-    atomicAdd(&acc->n_res, bn);
-  }
+  defect_norm(
+      sq, n,
+      [](float2 a, int o) {
+        return df_add(a, make_float2(__shfl_down_sync(0xffffffffu, a.x, o), __shfl_down_sync(0xffffffffu, a.y, o)));
+      },
+      [](float2 a) { return df_to_double(a); }, acc);
 }
 
 __device__ __forceinline__ double acc_rms(double sq, unsigned long long n) { return n ? sqrt(sq / (double)n) : 0.0; }
@@ -1337,31 +1415,63 @@ void launch_rb_sweeps(cudaStream_t s, int nx, int ny, const float* x_in, float* 
   launch_smooth(s, a, pairs, MODE_PLAIN, early);
 }
 
-template <bool UPDATE>
-__global__ void __launch_bounds__(32 * UR_WARPS) k_update_resid64(int nx, int ny, double* __restrict__ p64a,
-                                                                double* __restrict__ p64b,
-                                                                SolveCtl* ctl, const float* __restrict__ e,
-                                                                const float* __restrict__ b,
-                                                                const float* __restrict__ b_lo,
-                                                                const uint8_t* __restrict__ code,
-                                                                float* __restrict__ r32, StepAccum* acc, int test,
-                                                                int use_cond, cudaGraphConditionalHandle h) {
-  update_resid64_tile<UPDATE>(nx, ny, p64a, p64b, ctl, e, b, b_lo, code, r32, acc, blockIdx.x, blockIdx.y);
+template <bool UPDATE, int RW>
+__global__ void __launch_bounds__(32 * DEFECT_WARPS) k_update_resid64(int nx, int ny, double* __restrict__ p64a,
+                                                                     double* __restrict__ p64b, SolveCtl* ctl,
+                                                                     const float* e,
+                                                                     const float* __restrict__ b,
+                                                                     const float* __restrict__ b_lo,
+                                                                     const uint8_t* __restrict__ code,
+                                                                     float* __restrict__ r32, StepAccum* acc, int test,
+                                                                     int use_cond, cudaGraphConditionalHandle h) {
+  update_resid64_tile<UPDATE, RW>(nx, ny, p64a, p64b, ctl, e, b, b_lo, code, r32, acc, blockIdx.x, blockIdx.y);
   defect_pass_test(acc, ctl, test, use_cond, h);
 }
 
 template <bool UPDATE>
-__global__ void __launch_bounds__(32 * DF_WARPS, 8) k_update_resid_df(int nx, int ny, float2* __restrict__ p2a,
-                                                                   float2* __restrict__ p2b,
-                                                                   SolveCtl* ctl, const float* __restrict__ e,
-                                                                   const float* __restrict__ b,
-                                                                   const float* __restrict__ b_lo,
-                                                                   const uint8_t* __restrict__ code,
-                                                                   float* __restrict__ r32, StepAccum* acc,
-                                                                   int test, int use_cond,
-                                                                   cudaGraphConditionalHandle h) {
-  update_resid_df_tile<UPDATE>(nx, ny, p2a, p2b, ctl, e, b, b_lo, code, r32, acc, blockIdx.x, blockIdx.y);
+__global__ void __launch_bounds__(32 * DEFECT_WARPS) k_update_resid_df(int nx, int ny, float2* __restrict__ p2a,
+                                                                      float2* __restrict__ p2b, SolveCtl* ctl,
+                                                                      const float* e, const float* __restrict__ b,
+                                                                      const float* __restrict__ b_lo,
+                                                                      const uint8_t* __restrict__ code,
+                                                                      float* __restrict__ r32, StepAccum* acc, int rows,
+                                                                      int test, int use_cond,
+                                                                      cudaGraphConditionalHandle h) {
+  update_resid_df_tile<UPDATE>(nx, ny, p2a, p2b, ctl, e, b, b_lo, code, r32, acc, blockIdx.x, blockIdx.y, rows);
   defect_pass_test(acc, ctl, test, use_cond, h);
+}
+
+// The blocks of a pass over nx x ny cells with `rows` rows a warp.
+static long defect_blocks(int nx, int ny, bool df, int rows) {
+  const int c = defect_cols(df), r = DEFECT_WARPS * rows;
+  return (long)((nx + c - 1) / c) * ((ny + r - 1) / r);
+}
+
+// Rows a warp. A small grid's pass is the latency of one warp: as few rows as
+// there are SMs for; a large one's is throughput: more rows, so that fewer of
+// them are formed twice. blocks(rows): the pass's blocks.
+// float64 (2, 4 or 8): 256^2 2 rows 7.7 us, 4 rows 7.6, 8 rows 10.0; 512^2
+// 14.0 / 12.5 / 12.0; 1024^2 30.2 / 26.2 / 29.4; 2048^2 105 / 89 / 86.
+// Double-float (2, 4, 6 or 8): the fewest whose blocks are resident at once (6
+// an SM): 256^2 2 rows 6.2 us, 4 rows 7.1, 8 rows 9.3; 724^2 12.6 / 10.6 /
+// 11.3; 2048^2 57 / 42 / 36.
+// (Each after the POST launch it follows, that launch's time taken off, with
+// the cycle test; 8 rows unrolled and 4 warps a block before: float64 17.9 us
+// at 256^2, 27 at 1024^2, 94 at 2048^2; double-float 9.2, 13.8 and 49.)
+template <class Blocks>
+static int defect_rows(bool df, int sms, Blocks blocks) {
+  if (!df) return blocks(2) <= 2L * sms ? 2 : blocks(4) <= 26L * sms ? 4 : 8;
+  for (int r = 2; r < 8; r += 2)
+    if (blocks(r) <= 6L * sms) return r;
+  return 8;
+}
+
+// The device's SMs.
+static int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    n = 0;
+  return n > 0 ? n : 1;
 }
 
 void launch_update_resid64(cudaStream_t s, int nx, int ny, double* p64a, double* p64b, SolveCtl* ctl,
@@ -1369,24 +1479,20 @@ void launch_update_resid64(cudaStream_t s, int nx, int ny, double* p64a, double*
                            float* r32, StepAccum* acc, bool df, int test, bool use_cond,
                            cudaGraphConditionalHandle h) {
   const int uc = use_cond ? 1 : 0;
+  const int rows = defect_rows(df, sm_count(), [&](int r) { return defect_blocks(nx, ny, df, r); });
+  const int c = defect_cols(df), r = DEFECT_WARPS * rows;
+  const dim3 g((nx + c - 1) / c, (ny + r - 1) / r), t(32 * DEFECT_WARPS);
+  // the pass that updates follows the smoother that writes e
   if (df) {
     float2* a = reinterpret_cast<float2*>(p64a);
     float2* bb = reinterpret_cast<float2*>(p64b);
-    dim3 g((nx + 29) / 30, (ny + DF_WARPS * DF_ROWS - 1) / (DF_WARPS * DF_ROWS));
-    if (update)
-      k_update_resid_df<true><<<g, 32 * DF_WARPS, 0, s>>>(nx, ny, a, bb, ctl, e, b, b_lo, code, r32, acc, test, uc, h);
-    else
-      k_update_resid_df<false><<<g, 32 * DF_WARPS, 0, s>>>(nx, ny, a, bb, ctl, e, b, b_lo, code, r32, acc, test, uc,
-                                                           h);
+    launch_dependent(update, update ? k_update_resid_df<true> : k_update_resid_df<false>, g, t, s, nx, ny, a, bb, ctl, e,
+                     b, b_lo, code, r32, acc, rows, test, uc, h);
     return;
   }
-  dim3 g((nx + 29) / 30, (ny + UR_WARPS * UR_ROWS - 1) / (UR_WARPS * UR_ROWS));
-  if (update)
-    k_update_resid64<true><<<g, 32 * UR_WARPS, 0, s>>>(nx, ny, p64a, p64b, ctl, e, b, b_lo, code, r32, acc, test, uc,
-                                                       h);
-  else
-    k_update_resid64<false><<<g, 32 * UR_WARPS, 0, s>>>(nx, ny, p64a, p64b, ctl, e, b, b_lo, code, r32, acc, test,
-                                                        uc, h);
+  auto k = update ? (rows == 2 ? k_update_resid64<true, 2> : rows == 4 ? k_update_resid64<true, 4> : k_update_resid64<true, 8>)
+                  : (rows == 2 ? k_update_resid64<false, 2> : rows == 4 ? k_update_resid64<false, 4> : k_update_resid64<false, 8>);
+  launch_dependent(update, k, g, t, s, nx, ny, p64a, p64b, ctl, e, b, b_lo, code, r32, acc, test, uc, h);
 }
 
 void launch_solve_begin(cudaStream_t s, StepAccum* acc, SolveCtl* ctl, bool use_cond, cudaGraphConditionalHandle h) {
@@ -1667,6 +1773,7 @@ struct BatchSolve {
   int* lists = nullptr;          // device: base, count, act_scene, act_pre, act_n, act_total
   BatchPlan plan{};
   std::vector<int> max_items;    // per cycle phase: all scenes' items (the grid's bound)
+  int defect_rows[2] = {8, 8};   // the defect pass's rows a warp: float64 scenes, double-float scenes
   std::vector<char> small;       // per cycle phase: its smoother items are the 64 x 32 regions
   std::pair<int, int> init_ph{0, 0}, zero_ph{0, 0};  // prologue defect pass, p = 0 fill: every scene
 };
@@ -1769,35 +1876,39 @@ __global__ void __launch_bounds__(TOP == 64 ? 1024 : 512, 1) k_batch_tail(BatchP
   }
 }
 
-template <bool UPDATE>
-__device__ __forceinline__ void batch_defect_item(const BatchScene& S, const BatchItem& it) {
+// RW: the float64 scenes' rows a warp, rows_df: the double-float scenes'.
+template <bool UPDATE, int RW>
+__device__ __forceinline__ void batch_defect_item(const BatchScene& S, const BatchItem& it, int rows_df) {
   const BatchLevel& L0 = S.lv[0];
   const float* e = UPDATE ? L0.x0 : nullptr;
   if (S.mixed == MIXED_DF)
     update_resid_df_tile<UPDATE>(L0.nx, L0.ny, reinterpret_cast<float2*>(S.p64a), reinterpret_cast<float2*>(S.p64b),
-                                 S.ctl, e, L0.b, S.b_lo, L0.code, S.r32, S.acc, it.bx, it.by);
+                                 S.ctl, e, L0.b, S.b_lo, L0.code, S.r32, S.acc, it.bx, it.by, rows_df);
   else
-    update_resid64_tile<UPDATE>(L0.nx, L0.ny, S.p64a, S.p64b, S.ctl, e, L0.b, S.b_lo, L0.code, S.r32, S.acc, it.bx,
+    update_resid64_tile<UPDATE, RW>(L0.nx, L0.ny, S.p64a, S.p64b, S.ctl, e, L0.b, S.b_lo, L0.code, S.r32, S.acc, it.bx,
                                 it.by);
 }
 
 // The defect pass of the iterating scenes with a refined pressure: p += e
 // and the new residual.
-__global__ void __launch_bounds__(32 * UR_WARPS) k_batch_defect(BatchPlan plan, int ph) {
+template <int RW>
+__global__ void __launch_bounds__(32 * DEFECT_WARPS) k_batch_defect(BatchPlan plan, int ph, int rows_df) {
   for (int i = blockIdx.x;; i += gridDim.x) {
     BatchItem it;
     if (!batch_item(plan, ph, i, it)) return;
-    batch_defect_item<true>(plan.sc[it.scene], it);
+    batch_defect_item<true, RW>(plan.sc[it.scene], it, rows_df);
     __syncthreads();
   }
 }
 
 // The initial defect pass of every scene with a refined pressure (before
 // the loop), one item per block.
-__global__ void __launch_bounds__(32 * UR_WARPS) k_batch_defect_init(const BatchScene* __restrict__ sc,
-                                                                    const BatchItem* __restrict__ items) {
+template <int RW>
+__global__ void __launch_bounds__(32 * DEFECT_WARPS) k_batch_defect_init(const BatchScene* __restrict__ sc,
+                                                                         const BatchItem* __restrict__ items,
+                                                                         int rows_df) {
   const BatchItem it = items[blockIdx.x];
-  batch_defect_item<false>(sc[it.scene], it);
+  batch_defect_item<false, RW>(sc[it.scene], it, rows_df);
 }
 
 // Every scene's begin test, the compacted lists of the first cycle; the
@@ -1935,11 +2046,21 @@ BatchSolve* batch_solve_create(const std::vector<Engine*>& es_in, std::string& w
     for (int by = 0; by < gy; by++)
       for (int bx = 0; bx < gx; bx++) items.push_back(BatchItem{k, l, bx, by});
   };
+  // the defect pass's rows a warp, for all scenes of a kind together
+  auto defect_total = [&](bool df, int rows) {
+    long total = 0;
+    for (const BatchScene& S : hs)
+      if (S.mixed != 0 && (S.mixed == MIXED_DF) == df) total += defect_blocks(S.lv[0].nx, S.lv[0].ny, df, rows);
+    return total;
+  };
+  for (int df = 0; df < 2; df++)
+    b->defect_rows[df] = defect_rows(df, b->sms, [&](int r) { return defect_total(df, r); });
   auto defect_items = [&](int k) {
     const BatchLevel& L = hs[k].lv[0];
-    const int rows = hs[k].mixed == MIXED_DF ? DF_WARPS * DF_ROWS : UR_WARPS * UR_ROWS;
+    const bool df = hs[k].mixed == MIXED_DF;
+    const int cols = defect_cols(df), rows = DEFECT_WARPS * b->defect_rows[df];
     for (int by = 0; by < (L.ny + rows - 1) / rows; by++)
-      for (int bx = 0; bx < (L.nx + 29) / 30; bx++) items.push_back(BatchItem{k, 0, bx, by});
+      for (int bx = 0; bx < (L.nx + cols - 1) / cols; bx++) items.push_back(BatchItem{k, 0, bx, by});
   };
   for (int k = 0; k < n; k++) {
     for (int ph = 0; ph < depth; ph++) add(ph, k, [&] { smooth_items(ph, k); });
@@ -2018,8 +2139,10 @@ static void launch_batch_smooth(cudaStream_t s, const BatchSolve& b, int pairs, 
 // `body`) is one V-cycle of every iterating scene plus the defect pass and
 // the cycle tests, then the p = 0 fill of scenes whose rhs vanished.
 cudaError_t batch_solve_enqueue(const BatchSolve& b, cudaStream_t s, cudaStream_t body) {
+  const int rows = b.defect_rows[0];
   if (b.init_ph.second > 0)
-    k_batch_defect_init<<<b.init_ph.second, 32 * UR_WARPS, 0, s>>>(b.scenes, b.items + b.init_ph.first);
+    (rows == 2 ? k_batch_defect_init<2> : rows == 4 ? k_batch_defect_init<4> : k_batch_defect_init<8>)<<<
+        b.init_ph.second, 32 * DEFECT_WARPS, 0, s>>>(b.scenes, b.items + b.init_ph.first, b.defect_rows[1]);
   cudaStreamCaptureStatus cst;
   cudaGraph_t cap = nullptr;
   cudaError_t err = cudaStreamGetCaptureInfo(s, &cst, nullptr, &cap, nullptr, nullptr, nullptr);
@@ -2050,7 +2173,8 @@ cudaError_t batch_solve_enqueue(const BatchSolve& b, cudaStream_t s, cudaStream_
     k_batch_tail<32><<<phase_grid(b, D, 1), b.tail_threads, 0, body>>>(b.plan, D);
   for (int d = 0; d < D; d++) launch_batch_smooth<MODE_POST>(body, b, b.post, D + 1 + d);
   if (b.max_items[2 * D + 1] > 0)
-    k_batch_defect<<<phase_grid(b, 2 * D + 1, 8), 32 * UR_WARPS, 0, body>>>(b.plan, 2 * D + 1);
+    (rows == 2 ? k_batch_defect<2> : rows == 4 ? k_batch_defect<4> : k_batch_defect<8>)<<<
+        phase_grid(b, 2 * D + 1, 8), 32 * DEFECT_WARPS, 0, body>>>(b.plan, 2 * D + 1, b.defect_rows[1]);
   k_batch_check<<<1, 1024, 0, body>>>(b.plan, h);
   cudaGraph_t done = nullptr;
   err = cudaStreamEndCapture(body, &done);

@@ -79,3 +79,26 @@ def test_tail_frames(o32, nx, ny, side, coarsest, sweeps, pre, post):
     exp, _, rr32 = o32.mg_solve(nx, ny, p0, div, label, 0.02, 2, 1e-30, pre, post, sweeps, coarsest)
     same(exp, p, "%dx%d" % (nx, ny))
     assert used.value == 2 and abs(rr.value - rr32) <= 1e-9 * rr32
+
+
+@pytest.mark.parametrize("mixed", [1, 2])
+@pytest.mark.parametrize("nx,ny", [(3, 2), (29, 8), (30, 9), (61, 33), (130, 66), (517, 389), (724, 500), (1100, 1060)])
+def test_defect_pass_rows(o32, nx, ny, mixed):
+    """The defect-correction passes where their blocks' columns and rows end
+    and at sizes that take each number of rows a warp: the refined pressure
+    of two cycles, bit for bit."""
+    label, div, _ = problem(nx, ny)
+    prm = native.default_params(mg_pre=1, mg_post=1, mg_coarse_sweeps=4, mg_coarsest=4, mixed=mixed)
+    eng = native.Engine(nx, ny, params=prm)
+    try:
+        p, used, rr = np.zeros(nx * ny), native.ctypes.c_int(), native.ctypes.c_double()
+        eng.call("fl_mg_solve_mixed", ptr(p), ptr(div), ptr(label), 0.02, 2, 1e-30, native.ctypes.byref(used),
+                 native.ctypes.byref(rr))
+    finally:
+        eng.close()
+    solve = o32.mg_solve_mixed if mixed == 1 else o32.mg_solve_df
+    exp, used32, rr32 = solve(nx, ny, np.zeros(nx * ny), div, label, 0.02, 2, 1e-30, 1, 1, 4, 4)
+    assert used.value == used32
+    assert np.array_equal(np.asarray(exp, np.float64), p)
+    # sums of the same squares in another order, float64 or double-float
+    assert abs(rr.value - rr32) <= 1e-9 * rr32
