@@ -20,8 +20,9 @@
 namespace fl {
 
 // advect.ts:41-55
+template <class S>
 __device__ __forceinline__ void backtrace(const float* __restrict__ uc, const float* __restrict__ vc, int nx, int ny,
-                                          const Spacing& h, float x, float y, float u0, float v0, float dt, float& bx,
+                                          const S& h, float x, float y, float u0, float v0, float dt, float& bx,
                                           float& by) {
   float midX = x - 0.5f * dt * u0;
   float midY = y - 0.5f * dt * v0;
@@ -29,92 +30,112 @@ __device__ __forceinline__ void backtrace(const float* __restrict__ uc, const fl
   by = y - dt * sample_v(vc, nx, ny, h, midX, midY);
 }
 
-// MODE 0: forward pass (advectFaces with src = carrier), writes `out`.
-// MODE 1: MacCormack correction: `hat` is the forward result, `out` receives
-//         clamp(hat + 0.5*(in - reverse(hat))) (advect.ts:177-210).
-template <int MODE>
-__global__ void __launch_bounds__(256) k_advect_velocity(int nx, int ny, Spacing h, const float* __restrict__ u_in,
-                                                         const float* __restrict__ v_in,
-                                                         const float* __restrict__ u_hat,
-                                                         const float* __restrict__ v_hat, float* __restrict__ u_out,
-                                                         float* __restrict__ v_out,
-                                                         const uint8_t* __restrict__ label,
-                                                         const StepScalars* __restrict__ sc, float2* __restrict__ bt_u,
-                                                         float2* __restrict__ bt_v) {
+// The carrier at a face's own position, where the face holds only one of its
+// components: with h a power of two (x / h exact) an interior face's four
+// neighbours of the other kind with weights 1/2, otherwise the general sample.
+__device__ __forceinline__ float v_at_u_face(const float* __restrict__ v, int nx, int ny, const SpacingPow2&, int i,
+                                             int j, float, float) {
+  return sample(v, Stencil{i - 1 + j * nx, 0.5f, 0.5f}, nx);
+}
+__device__ __forceinline__ float v_at_u_face(const float* __restrict__ v, int nx, int ny, const SpacingAny& h, int,
+                                             int, float x, float y) {
+  return sample_v(v, nx, ny, h, x, y);
+}
+__device__ __forceinline__ float u_at_v_face(const float* __restrict__ u, int nx, int ny, const SpacingPow2&, int i,
+                                             int j, float, float) {
+  return sample(u, Stencil{i + (j - 1) * (nx + 1), 0.5f, 0.5f}, nx + 1);
+}
+__device__ __forceinline__ float u_at_v_face(const float* __restrict__ u, int nx, int ny, const SpacingAny& h, int,
+                                             int, float x, float y) {
+  return sample_u(u, nx, ny, h, x, y);
+}
+
+// MODE 0: forward pass (advectFaces with src = carrier), writes `out`; with
+//         `at` (MacCormack) also the offset of the backtraced point's stencil,
+//         as an integer in the correction's output.
+// MODE 1: MacCormack correction: `hat` is the forward result, `out` holds the
+//         stencil offsets and receives clamp(hat + 0.5*(in - reverse(hat)))
+//         (advect.ts:177-210).
+// Bound by instruction issue (70% active). Both launches of a MacCormack step
+// in a graph: 1024^2 32.2 us, 256^2 6.2; with the samplers' floor, index and
+// division as conversion and division instructions, the two faces one after
+// the other and backtraced positions handed over in buffers of their own 47.1
+// and 9.6 (20.4 M warp instructions a correction against 16.4 M).
+template <int MODE, class S>
+__device__ __forceinline__ void advect_faces(int nx, int ny, const S& h, const float* __restrict__ u_in,
+                                             const float* __restrict__ v_in, const float* u_hat, const float* v_hat,
+                                             float* u_out, float* v_out, const uint8_t* __restrict__ label,
+                                             const StepScalars* __restrict__ sc, float* u_at, float* v_at) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const float dt = sc->dt;
-  if (i <= nx && j < ny) {
-    const int k = i + j * (nx + 1);
-    if (solid_or_outside(label, nx, ny, i - 1, j) || solid_or_outside(label, nx, ny, i, j)) {
-      u_out[k] = u_in[k];
-    } else {
-      const float x = (float)i * h.h;
-      const float y = ((float)j + 0.5f) * h.h;
-      const float u0 = u_in[k];
-      const float v0 = sample_v(v_in, nx, ny, h, x, y);
-      float bx, by;
-      if (MODE == 0) {
-        backtrace(u_in, v_in, nx, ny, h, x, y, u0, v0, dt, bx, by);
-        if (bt_u != nullptr) bt_u[k] = make_float2(bx, by);
-        u_out[k] = sample_u(u_in, nx, ny, h, bx, by);
-      } else {
-        backtrace(u_in, v_in, nx, ny, h, x, y, u0, v0, -dt, bx, by);
-        const float ubar = sample_u(u_hat, nx, ny, h, bx, by);
-        const float corrected = u_hat[k] + 0.5f * (u_in[k] - ubar);
-        if (bt_u != nullptr) {
-          const float2 b = bt_u[k];
-          bx = b.x;
-          by = b.y;
-        } else {
-          backtrace(u_in, v_in, nx, ny, h, x, y, u0, v0, dt, bx, by);
-        }
-        u_out[k] = clamp_stencil_u(u_in, nx, ny, h, bx, by, corrected);
-      }
-    }
+  const float dt = MODE == 0 ? sc->dt : -sc->dt;
+  // Both faces go through the arithmetic together, without branches, so that
+  // their chains of gathers overlap; a face that is not advected (beside a
+  // solid cell, or outside the grid) stands in for one that is in range.
+  const bool u_in_grid = i <= nx && j < ny, v_in_grid = i < nx && j <= ny;
+  const bool u_fixed = solid_or_outside(label, nx, ny, i - 1, j) || solid_or_outside(label, nx, ny, i, j);
+  const bool v_fixed = solid_or_outside(label, nx, ny, i, j - 1) || solid_or_outside(label, nx, ny, i, j);
+  const int iu = u_fixed ? 1 : i, ju = u_fixed ? 0 : j, iv = v_fixed ? 0 : i, jv = v_fixed ? 1 : j;
+  const int ku = iu + ju * (nx + 1), kv = iv + jv * nx;
+  const float xu = (float)iu * h.h, yu = ((float)ju + 0.5f) * h.h;
+  const float xv = ((float)iv + 0.5f) * h.h, yv = (float)jv * h.h;
+  const float uu = u_in[ku], vv = v_in[kv];
+  const float vu = v_at_u_face(v_in, nx, ny, h, iu, ju, xu, yu);
+  const float uv = u_at_v_face(u_in, nx, ny, h, iv, jv, xv, yv);
+  float bxu, byu, bxv, byv;
+  backtrace(u_in, v_in, nx, ny, h, xu, yu, uu, vu, dt, bxu, byu);
+  backtrace(u_in, v_in, nx, ny, h, xv, yv, uv, vv, dt, bxv, byv);
+  const Stencil pu = stencil_u(nx, ny, h, bxu, byu), pv = stencil_v(nx, ny, h, bxv, byv);
+  // the correction's launch starts while the forward pass drains: only what
+  // that wrote (hat, the offsets in out) is read after the wait
+  if (MODE == 1) dep_wait();
+  float ru, rv;
+  if (MODE == 0) {
+    ru = sample(u_in, pu, nx + 1);
+    rv = sample(v_in, pv, nx);
+  } else {
+    const int au = u_fixed ? 0 : __float_as_int(u_out[ku]), av = v_fixed ? 0 : __float_as_int(v_out[kv]);
+    ru = clamp_at(u_in, au, nx + 1, u_hat[ku] + 0.5f * (uu - sample_fresh(u_hat, pu, nx + 1)));
+    rv = clamp_at(v_in, av, nx, v_hat[kv] + 0.5f * (vv - sample_fresh(v_hat, pv, nx)));
   }
-  if (i < nx && j <= ny) {
+  if (u_in_grid) {
+    const int k = i + j * (nx + 1);
+    if (MODE == 0 && u_at != nullptr) u_at[k] = __int_as_float(pu.k);
+    u_out[k] = u_fixed ? u_in[k] : ru;
+  }
+  if (v_in_grid) {
     const int k = i + j * nx;
-    if (solid_or_outside(label, nx, ny, i, j - 1) || solid_or_outside(label, nx, ny, i, j)) {
-      v_out[k] = v_in[k];
-    } else {
-      const float x = ((float)i + 0.5f) * h.h;
-      const float y = (float)j * h.h;
-      const float u0 = sample_u(u_in, nx, ny, h, x, y);
-      const float v0 = v_in[k];
-      float bx, by;
-      if (MODE == 0) {
-        backtrace(u_in, v_in, nx, ny, h, x, y, u0, v0, dt, bx, by);
-        if (bt_v != nullptr) bt_v[k] = make_float2(bx, by);
-        v_out[k] = sample_v(v_in, nx, ny, h, bx, by);
-      } else {
-        backtrace(u_in, v_in, nx, ny, h, x, y, u0, v0, -dt, bx, by);
-        const float vbar = sample_v(v_hat, nx, ny, h, bx, by);
-        const float corrected = v_hat[k] + 0.5f * (v_in[k] - vbar);
-        if (bt_v != nullptr) {
-          const float2 b = bt_v[k];
-          bx = b.x;
-          by = b.y;
-        } else {
-          backtrace(u_in, v_in, nx, ny, h, x, y, u0, v0, dt, bx, by);
-        }
-        v_out[k] = clamp_stencil_v(v_in, nx, ny, h, bx, by, corrected);
-      }
-    }
+    if (MODE == 0 && v_at != nullptr) v_at[k] = __int_as_float(pv.k);
+    v_out[k] = v_fixed ? v_in[k] : rv;
   }
 }
 
+template <int MODE>
+__global__ void __launch_bounds__(256) k_advect_velocity(int nx, int ny, Spacing h, const float* __restrict__ u_in,
+                                                         const float* __restrict__ v_in, const float* u_hat,
+                                                         const float* v_hat, float* u_out, float* v_out,
+                                                         const uint8_t* __restrict__ label,
+                                                         const StepScalars* __restrict__ sc, float* u_at,
+                                                         float* v_at) {
+  if (MODE == 0) dep_trigger();
+  if (h.pow2)
+    advect_faces<MODE>(nx, ny, SpacingPow2(h), u_in, v_in, u_hat, v_hat, u_out, v_out, label, sc, u_at, v_at);
+  else
+    advect_faces<MODE>(nx, ny, SpacingAny(h), u_in, v_in, u_hat, v_hat, u_out, v_out, label, sc, u_at, v_at);
+}
+
 // Dye. MODE 0 forward (advect.ts:241-270), MODE 1 correction (advect.ts:
-// 294-311). TAIL applies decay then the inlet patch (simulation.ts:569-581,
-// dye.ts:158-175) to the value this thread writes.
-template <int MODE, bool TAIL>
-__global__ void __launch_bounds__(256) k_advect_dye(int nx, int ny, Spacing h, int dnx, int dny, Spacing dh,
-                                                    const float* __restrict__ u, const float* __restrict__ v,
-                                                    const float* __restrict__ q_in, const float* __restrict__ q_hat,
-                                                    float* __restrict__ q_out, const uint8_t* __restrict__ label,
-                                                    const StepScalars* __restrict__ sc,
-                                                    const float* __restrict__ patch, int pi0, int pj0, int pnx,
-                                                    int pny, float2* __restrict__ bt) {
+// 294-311); the backtraced point's stencil offset passes from one to the other
+// in `at`, the first plane of the correction's output. TAIL applies decay then
+// the inlet patch (simulation.ts:569-581, dye.ts:158-175) to the value this
+// thread writes.
+template <int MODE, bool TAIL, class S>
+__device__ __forceinline__ void advect_cells(int nx, int ny, const S& h, int dnx, int dny, const S& dh,
+                                             const float* __restrict__ u, const float* __restrict__ v,
+                                             const float* __restrict__ q_in, const float* q_hat, float* q_out,
+                                             const uint8_t* __restrict__ label, const StepScalars* __restrict__ sc,
+                                             const float* __restrict__ patch, int pi0, int pj0, int pnx, int pny,
+                                             float* at) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= dnx || j >= dny) return;
@@ -129,32 +150,27 @@ __global__ void __launch_bounds__(256) k_advect_dye(int nx, int ny, Spacing h, i
   if (solid_or_outside(label, nx, ny, li, lj)) {
 #pragma unroll
     for (int c = 0; c < DYE_CHANNELS; c++) q[c] = q_in[k + c * cells];
+    if (MODE == 1) dep_wait();
   } else {
     const float x = ((float)i + 0.5f) * dh.h;
     const float y = ((float)j + 0.5f) * dh.h;
     const float u0 = sample_u(u, nx, ny, h, x, y);
     const float v0 = sample_v(v, nx, ny, h, x, y);
     float bx, by;
+    backtrace(u, v, nx, ny, h, x, y, u0, v0, MODE == 0 ? dt : -dt, bx, by);
+    const Stencil p = stencil_p(dnx, dny, dh, bx, by);
     if (MODE == 0) {
-      backtrace(u, v, nx, ny, h, x, y, u0, v0, dt, bx, by);
-      if (bt != nullptr) bt[k] = make_float2(bx, by);
+      if (at != nullptr) at[k] = __int_as_float(p.k);
 #pragma unroll
-      for (int c = 0; c < DYE_CHANNELS; c++) q[c] = sample_p(q_in + c * cells, dnx, dny, dh, bx, by);
+      for (int c = 0; c < DYE_CHANNELS; c++) q[c] = sample(q_in + c * cells, p, dnx);
     } else {
-      float rbx, rby;
-      backtrace(u, v, nx, ny, h, x, y, u0, v0, -dt, rbx, rby);
-      if (bt != nullptr) {
-        const float2 b = bt[k];
-        bx = b.x;
-        by = b.y;
-      } else {
-        backtrace(u, v, nx, ny, h, x, y, u0, v0, dt, bx, by);
-      }
+      dep_wait();  // hat and the offset in q_out are the forward pass's, whose end this launch need not await
+      const int ck = __float_as_int(q_out[k]);
 #pragma unroll
       for (int c = 0; c < DYE_CHANNELS; c++) {
-        const float qbar = sample_p(q_hat + c * cells, dnx, dny, dh, rbx, rby);
-        const float corrected = q_hat[k + c * cells] + 0.5f * (q_in[k + c * cells] - qbar);
-        q[c] = clamp_stencil_p(q_in + c * cells, dnx, dny, dh, bx, by, corrected);
+        const float corrected =
+            q_hat[k + c * cells] + 0.5f * (q_in[k + c * cells] - sample_fresh(q_hat + c * cells, p, dnx));
+        q[c] = clamp_at(q_in + c * cells, ck, dnx, corrected);
       }
     }
   }
@@ -181,19 +197,35 @@ __global__ void __launch_bounds__(256) k_advect_dye(int nx, int ny, Spacing h, i
   for (int c = 0; c < DYE_CHANNELS; c++) q_out[k + c * cells] = q[c];
 }
 
+template <int MODE, bool TAIL>
+__global__ void __launch_bounds__(256) k_advect_dye(int nx, int ny, Spacing h, int dnx, int dny, Spacing dh,
+                                                    const float* __restrict__ u, const float* __restrict__ v,
+                                                    const float* __restrict__ q_in, const float* q_hat, float* q_out,
+                                                    const uint8_t* __restrict__ label,
+                                                    const StepScalars* __restrict__ sc,
+                                                    const float* __restrict__ patch, int pi0, int pj0, int pnx,
+                                                    int pny, float* at) {
+  if (MODE == 0) dep_trigger();
+  if (h.pow2 && dh.pow2)
+    advect_cells<MODE, TAIL>(nx, ny, SpacingPow2(h), dnx, dny, SpacingPow2(dh), u, v, q_in, q_hat, q_out, label, sc,
+                             patch, pi0, pj0, pnx, pny, at);
+  else
+    advect_cells<MODE, TAIL>(nx, ny, SpacingAny(h), dnx, dny, SpacingAny(dh), u, v, q_in, q_hat, q_out, label, sc,
+                             patch, pi0, pj0, pnx, pny, at);
+}
+
 void launch_advect_velocity(cudaStream_t s, int nx, int ny, float h, int mac, const float* u_in, const float* v_in,
                             float* u_hat, float* v_hat, float* u_out, float* v_out, const uint8_t* label,
-                            const StepScalars* sc, float2* bt_u, float2* bt_v) {
+                            const StepScalars* sc) {
   const Spacing hs = make_spacing(h);
   dim3 blk(32, 8);
   dim3 grd((nx + 1 + blk.x - 1) / blk.x, (ny + 1 + blk.y - 1) / blk.y);
   if (mac) {
-    // the correction reuses the forward pass's backtrace positions when
-    // there is room for them (bt_u, bt_v; identical to recomputing them)
-    k_advect_velocity<0><<<grd, blk, 0, s>>>(nx, ny, hs, u_in, v_in, nullptr, nullptr, u_hat, v_hat, label, sc, bt_u,
-                                             bt_v);
-    k_advect_velocity<1><<<grd, blk, 0, s>>>(nx, ny, hs, u_in, v_in, u_hat, v_hat, u_out, v_out, label, sc, bt_u,
-                                             bt_v);
+    // the forward pass leaves its stencils' offsets in the correction's output
+    k_advect_velocity<0><<<grd, blk, 0, s>>>(nx, ny, hs, u_in, v_in, nullptr, nullptr, u_hat, v_hat, label, sc, u_out,
+                                             v_out);
+    launch_dependent(true, k_advect_velocity<1>, grd, blk, s, nx, ny, hs, u_in, v_in, u_hat, v_hat, u_out, v_out, label,
+                     sc, nullptr, nullptr);
   } else {
     k_advect_velocity<0><<<grd, blk, 0, s>>>(nx, ny, hs, u_in, v_in, nullptr, nullptr, u_out, v_out, label, sc,
                                              nullptr, nullptr);
@@ -209,20 +241,15 @@ cudaError_t preload_advect_kernels() {
 
 void launch_advect_dye(cudaStream_t s, int nx, int ny, float h, int dnx, int dny, float dh, int mac, const float* u,
                        const float* v, const float* q_in, float* q_hat, float* q_out, const uint8_t* label,
-                       const StepScalars* sc, bool tail, const float* patch, int pi0, int pj0, int pnx, int pny,
-                       float2* bt) {
+                       const StepScalars* sc, bool tail, const float* patch, int pi0, int pj0, int pnx, int pny) {
   const Spacing hs = make_spacing(h), ds = make_spacing(dh);
   dim3 blk(32, 8);
   dim3 grd((dnx + blk.x - 1) / blk.x, (dny + blk.y - 1) / blk.y);
   if (mac) {
     k_advect_dye<0, false><<<grd, blk, 0, s>>>(nx, ny, hs, dnx, dny, ds, u, v, q_in, nullptr, q_hat, label, sc, nullptr,
-                                               0, 0, 0, 0, bt);
-    if (tail)
-      k_advect_dye<1, true><<<grd, blk, 0, s>>>(nx, ny, hs, dnx, dny, ds, u, v, q_in, q_hat, q_out, label, sc, patch,
-                                                pi0, pj0, pnx, pny, bt);
-    else
-      k_advect_dye<1, false><<<grd, blk, 0, s>>>(nx, ny, hs, dnx, dny, ds, u, v, q_in, q_hat, q_out, label, sc,
-                                                 nullptr, 0, 0, 0, 0, bt);
+                                               0, 0, 0, 0, q_out);
+    launch_dependent(true, tail ? k_advect_dye<1, true> : k_advect_dye<1, false>, grd, blk, s, nx, ny, hs, dnx, dny, ds,
+                     u, v, q_in, q_hat, q_out, label, sc, tail ? patch : nullptr, pi0, pj0, pnx, pny, nullptr);
   } else {
     if (tail)
       k_advect_dye<0, true><<<grd, blk, 0, s>>>(nx, ny, hs, dnx, dny, ds, u, v, q_in, nullptr, q_out, label, sc, patch,

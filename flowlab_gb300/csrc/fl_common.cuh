@@ -127,7 +127,39 @@ __host__ inline Spacing make_spacing(float h) {
   return s;
 }
 
-__device__ __forceinline__ float over(float x, const Spacing& s) { return s.pow2 ? x * s.inv : x / s.h; }
+static __device__ __noinline__ float div_slow(float x, float h) { return x / h; }
+
+// A Spacing known to be a power of two (kernels that sample much branch on it
+// once and compile their body for both).
+struct SpacingPow2 {
+  float h;
+  float inv;
+  __device__ __forceinline__ explicit SpacingPow2(const Spacing& s) : h(s.h), inv(s.inv) {}
+};
+struct SpacingAny {
+  float h;
+  float inv;
+  __device__ __forceinline__ explicit SpacingAny(const Spacing& s) : h(s.h), inv(s.inv) {}
+};
+
+// x / h. For a general h the quotient by the correctly rounded reciprocal,
+// corrected twice: the first correction brings it within a unit in the last
+// place, the second one rounds it correctly (Markstein: q' = RN(q + r RN(1/h))
+// with the exact remainder r of such a q is RN(x / h)), in 5 operations without
+// a branch. Tiny, huge, infinite and NaN x, where a remainder could underflow
+// or overflow, take the division.
+__device__ __forceinline__ float over(float x, const SpacingPow2& s) { return x * s.inv; }
+__device__ __forceinline__ float over(float x, const SpacingAny& s) {
+  if ((__float_as_uint(x) & 0x7fffffffu) - 0x20000000u >= 0x40000000u) return div_slow(x, s.h);
+  float q = __fmul_rn(x, s.inv);
+  float r = __fmaf_rn(-s.h, q, x);
+  q = __fmaf_rn(r, s.inv, q);
+  r = __fmaf_rn(-s.h, q, x);
+  return __fmaf_rn(r, s.inv, q);
+}
+__device__ __forceinline__ float over(float x, const Spacing& s) {
+  return s.pow2 ? over(x, SpacingPow2(s)) : over(x, SpacingAny(s));
+}
 
 struct AxisF {
   int i0;
@@ -140,14 +172,28 @@ struct AxisF {
 __device__ __forceinline__ float smin(float a, float b) { return (b < a) ? b : a; }
 __device__ __forceinline__ float smax(float a, float b) { return (a < b) ? b : a; }
 
+// one instruction each, a NaN operand gives NaN (as smin / smax do when it is their first)
+__device__ __forceinline__ float min_nan(float a, float b) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 // grid.ts:173-177 clampedAxis: position clamped to [0, count-1], index to
-// count-2.
+// count-2. The floor of c (0 <= c < 2^23) and its index come from c + 2^23
+// rounded down, whose last place is 1: no conversion instruction, of which an
+// SM issues 16 lanes a clock. A NaN position gives an index in range and f NaN.
 __device__ __forceinline__ AxisF clamped_axis(float pos, int count) {
-  float c = smin(smax(pos, 0.0f), (float)(count - 1));
-  int i0 = min((int)floorf(c), count - 2);
+  const float c = min_nan(max_nan(pos, 0.0f), (float)(count - 1));
+  const float t = fminf(__fadd_rd(c, 8388608.0f), 8388608.0f + (float)(count - 2));
   AxisF a;
-  a.i0 = i0;
-  a.f = c - (float)i0;
+  a.i0 = (int)(__float_as_uint(t) - 0x4b000000u);
+  a.f = c - (t - 8388608.0f);
   return a;
 }
 
@@ -163,31 +209,60 @@ __device__ __forceinline__ float ldg(const float* p) { return __ldg(p); }
 // The samplers index with 32-bit offsets: a sampled field holds fewer than
 // 2^31 values (the engine's grid and dye-grid limits guarantee it).
 
+// A sampled point of a field: the offset of its stencil's first value (in rows
+// of s values) and the two weights.
+struct Stencil {
+  int k;
+  float fx, fy;
+};
+
+__device__ __forceinline__ float sample(const float* __restrict__ f, const Stencil& p, int s) {
+  const float* q = f + p.k;
+  return bilerp(ldg(q), ldg(q + 1), ldg(q + s), ldg(q + s + 1), p.fx, p.fy);
+}
+
+// The same of a field that the launch before this one may have written
+// (dep_wait): ordinary loads, which stay behind the wait.
+__device__ __forceinline__ float sample_fresh(const float* f, const Stencil& p, int s) {
+  const float* q = f + p.k;
+  return bilerp(q[0], q[1], q[s], q[s + 1], p.fx, p.fy);
+}
+
+__device__ __forceinline__ Stencil stencil_at(float px, float py, int nx, int ny) {
+  const AxisF a = clamped_axis(px, nx), b = clamped_axis(py, ny);
+  Stencil p;
+  p.k = a.i0 + b.i0 * nx;
+  p.fx = a.f;
+  p.fy = b.f;
+  return p;
+}
+
 // grid.ts:197-208 sampleU: u[i,j] at (i*h, (j+0.5)*h), (nx+1) x ny values.
-__device__ __forceinline__ float sample_u(const float* __restrict__ u, int nx, int ny, const Spacing& h, float x, float y) {
-  AxisF a = clamped_axis(over(x, h), nx + 1);
-  AxisF b = clamped_axis(over(y, h) - 0.5f, ny);
-  const int s = nx + 1;
-  const int k = a.i0 + b.i0 * s;
-  return bilerp(ldg(u + k), ldg(u + k + 1), ldg(u + k + s), ldg(u + k + s + 1), a.f, b.f);
+template <class S>
+__device__ __forceinline__ Stencil stencil_u(int nx, int ny, const S& h, float x, float y) {
+  return stencil_at(over(x, h), over(y, h) - 0.5f, nx + 1, ny);
 }
-
 // grid.ts:214-225 sampleV: v[i,j] at ((i+0.5)*h, j*h), nx x (ny+1) values.
-__device__ __forceinline__ float sample_v(const float* __restrict__ v, int nx, int ny, const Spacing& h, float x, float y) {
-  AxisF a = clamped_axis(over(x, h) - 0.5f, nx);
-  AxisF b = clamped_axis(over(y, h), ny + 1);
-  const int s = nx;
-  const int k = a.i0 + b.i0 * s;
-  return bilerp(ldg(v + k), ldg(v + k + 1), ldg(v + k + s), ldg(v + k + s + 1), a.f, b.f);
+template <class S>
+__device__ __forceinline__ Stencil stencil_v(int nx, int ny, const S& h, float x, float y) {
+  return stencil_at(over(x, h) - 0.5f, over(y, h), nx, ny + 1);
 }
-
 // grid.ts:239-250 sampleP on a cell-centred field of nx x ny.
-__device__ __forceinline__ float sample_p(const float* __restrict__ q, int nx, int ny, const Spacing& h, float x, float y) {
-  AxisF a = clamped_axis(over(x, h) - 0.5f, nx);
-  AxisF b = clamped_axis(over(y, h) - 0.5f, ny);
-  const int s = nx;
-  const int k = a.i0 + b.i0 * s;
-  return bilerp(ldg(q + k), ldg(q + k + 1), ldg(q + k + s), ldg(q + k + s + 1), a.f, b.f);
+template <class S>
+__device__ __forceinline__ Stencil stencil_p(int nx, int ny, const S& h, float x, float y) {
+  return stencil_at(over(x, h) - 0.5f, over(y, h) - 0.5f, nx, ny);
+}
+template <class S>
+__device__ __forceinline__ float sample_u(const float* __restrict__ u, int nx, int ny, const S& h, float x, float y) {
+  return sample(u, stencil_u(nx, ny, h, x, y), nx + 1);
+}
+template <class S>
+__device__ __forceinline__ float sample_v(const float* __restrict__ v, int nx, int ny, const S& h, float x, float y) {
+  return sample(v, stencil_v(nx, ny, h, x, y), nx);
+}
+template <class S>
+__device__ __forceinline__ float sample_p(const float* __restrict__ q, int nx, int ny, const S& h, float x, float y) {
+  return sample(q, stencil_p(nx, ny, h, x, y), nx);
 }
 
 // grid.ts:268-270
@@ -197,30 +272,10 @@ __device__ __forceinline__ float clamp_to_range(float q, float a, float b, float
   return smin(smax(q, lo), hi);
 }
 
-// grid.ts:273-315 clampToStencil{U,V,P}
-__device__ __forceinline__ float clamp_stencil_u(const float* __restrict__ u, int nx, int ny, const Spacing& h, float x, float y,
-                                                 float q) {
-  int i0 = clamped_axis(over(x, h), nx + 1).i0;
-  int j0 = clamped_axis(over(y, h) - 0.5f, ny).i0;
-  const int s = nx + 1;
-  const int k = i0 + j0 * s;
-  return clamp_to_range(q, ldg(u + k), ldg(u + k + 1), ldg(u + k + s), ldg(u + k + s + 1));
-}
-__device__ __forceinline__ float clamp_stencil_v(const float* __restrict__ v, int nx, int ny, const Spacing& h, float x, float y,
-                                                 float q) {
-  int i0 = clamped_axis(over(x, h) - 0.5f, nx).i0;
-  int j0 = clamped_axis(over(y, h), ny + 1).i0;
-  const int s = nx;
-  const int k = i0 + j0 * s;
-  return clamp_to_range(q, ldg(v + k), ldg(v + k + 1), ldg(v + k + s), ldg(v + k + s + 1));
-}
-__device__ __forceinline__ float clamp_stencil_p(const float* __restrict__ q, int nx, int ny, const Spacing& h, float x, float y,
-                                                 float val) {
-  int i0 = clamped_axis(over(x, h) - 0.5f, nx).i0;
-  int j0 = clamped_axis(over(y, h) - 0.5f, ny).i0;
-  const int s = nx;
-  const int k = i0 + j0 * s;
-  return clamp_to_range(val, ldg(q + k), ldg(q + k + 1), ldg(q + k + s), ldg(q + k + s + 1));
+// grid.ts:273-315 clampToStencil{U,V,P}: q limited to the four values at k,
+// the offset of the stencil's first value in rows of s.
+__device__ __forceinline__ float clamp_at(const float* __restrict__ f, int k, int s, float q) {
+  return clamp_to_range(q, ldg(f + k), ldg(f + k + 1), ldg(f + k + s), ldg(f + k + s + 1));
 }
 
 // grid.ts:159-161 isSolidOrOutside on the velocity grid's labels.
