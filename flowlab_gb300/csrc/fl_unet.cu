@@ -235,29 +235,96 @@ __global__ void __launch_bounds__(256) k_conv3_wgrad(const __nv_bfloat16* __rest
     for (int pix = 0; pix < CT * CT; pix++) s = __fmaf_rn(gs[co][pix], xs[ci][pix / CT + ky][pix % CT + kx], s);
     atomicAdd(&dw[((long)(co0 + co) * 9 + tap) * Cin + c0 + ci], s);
   }
-  if (blockIdx.z == 0 && threadIdx.x < CO_T && co0 + threadIdx.x < Cout) {
+  if (db != nullptr && blockIdx.z == 0 && threadIdx.x < CO_T && co0 + threadIdx.x < Cout) {
     float s = 0.0f;
     for (int pix = 0; pix < CT * CT; pix++) s += gs[threadIdx.x][pix];
     atomicAdd(&db[co0 + threadIdx.x], s);
   }
 }
 
-// db[c] += sum over pixels of g[p][c]: thread t of a block handles channel
-// t % C over every (blockDim / C)-th pixel of the block's share (coalesced
-// rows); the block's partials meet in shared memory, one atomic per channel.
-__global__ void __launch_bounds__(256) k_bias_grad(const float* __restrict__ g, long P, int C, float* __restrict__ db) {
+// An output gradient's bf16 copy and its bias gradient, db[c] += sum over
+// pixels of g[p][c], from one read of it (bound by memory; as two passes, the
+// second with 152 blocks reading a word a lane, they took 7.7 + 19.2 us a layer
+// on average for 4 x 256^2, this one 10.4). A thread takes groups of 8
+// channels, always the same ones: the grid's threads are a multiple of the
+// groups a pixel.
+__global__ void __launch_bounds__(256) k_grad_bf16(const float* __restrict__ g, long P, int C,
+                                                   __nv_bfloat16* __restrict__ out, float* __restrict__ db) {
   __shared__ float sdb[256];
   for (int c = threadIdx.x; c < C; c += blockDim.x) sdb[c] = 0.0f;
   __syncthreads();
-  const int per = blockDim.x / C;  // pixels in flight per block
-  if ((int)threadIdx.x < per * C) {
-    const int c = threadIdx.x % C, j = threadIdx.x / C;
-    float s = 0.0f;
-    for (long p = (long)blockIdx.x * per + j; p < P; p += (long)gridDim.x * per) s += g[p * C + c];
-    atomicAdd(&sdb[c], s);
+  const int G = C / 8;
+  const long n = P * G, stride = (long)gridDim.x * blockDim.x / G * G, t0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  float s[8] = {};
+  if (t0 < stride) {
+#pragma unroll 4
+    for (long e = t0; e < n; e += stride) {
+      const float4 a = reinterpret_cast<const float4*>(g)[2 * e], b = reinterpret_cast<const float4*>(g)[2 * e + 1];
+      const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      __align__(16) __nv_bfloat16 o[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        o[k] = __float2bfloat16_rn(v[k]);
+        s[k] += v[k];
+      }
+      reinterpret_cast<uint4*>(out)[e] = *reinterpret_cast<const uint4*>(o);
+    }
+    const int c = 8 * (int)(t0 % G);
+#pragma unroll
+    for (int k = 0; k < 8; k++) atomicAdd(&sdb[c + k], s[k]);
   }
   __syncthreads();
   for (int c = threadIdx.x; c < C; c += blockDim.x) atomicAdd(&db[c], sdb[c]);
+}
+
+// The input layer's weight gradient (3 channels in, 32 out): lane = output
+// channel, a warp's 27 sums a lane in registers over its share of a tile's
+// pixels (g a coalesced 128-byte row a pixel, the inputs broadcast from shared
+// memory), the block's warps then meet in shared memory: one atomic a weight
+// and block. 4 x 256^2: 101 us by the general kernel, whose chunks of 8 inputs
+// are 5/8 empty here, 32 us by this one.
+__global__ void __launch_bounds__(256) k_wgrad_in3(const __nv_bfloat16* __restrict__ x, const float* __restrict__ g,
+                                                   int H, int W, int B, float* __restrict__ dw) {
+  constexpr int CI = 3, CO = 32, TW = 32, TH = 16;  // pixel tile
+  __shared__ float xs[TH + 2][(TW + 2) * CI + 2];
+  __shared__ float sw[9 * CI][CO];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int e = threadIdx.x; e < 9 * CI * CO; e += 256) (&sw[0][0])[e] = 0.0f;
+  float acc[9 * CI] = {};
+  const int tx = (W + TW - 1) / TW, ty = (H + TH - 1) / TH, tiles = tx * ty * B;
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const int X0 = t % tx * TW, Y0 = t / tx % ty * TH;
+    const long img = (long)(t / (tx * ty)) * H * W;
+    __syncthreads();
+    for (int e = threadIdx.x; e < (TH + 2) * (TW + 2) * CI; e += 256) {
+      const int q = e % ((TW + 2) * CI), ly = e / ((TW + 2) * CI);
+      const int gx = X0 + q / CI - 1, gy = Y0 + ly - 1;
+      xs[ly][q] = gx >= 0 && gy >= 0 && gx < W && gy < H ? __bfloat162float(x[(img + (long)gy * W + gx) * CI + q % CI]) : 0.0f;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int r = w; r < TH; r += 8) {
+      if (Y0 + r >= H) break;
+      const int cols = min(TW, W - X0);
+      const float* gr = g + (img + (long)(Y0 + r) * W + X0) * CO + lane;
+#pragma unroll 4
+      for (int c = 0; c < cols; c++) {
+        const float gv = gr[c * CO];
+#pragma unroll
+        for (int ky = 0; ky < 3; ky++)
+#pragma unroll
+          for (int k = 0; k < 3 * CI; k++)  // the three taps' inputs lie side by side
+            acc[ky * 3 * CI + k] = __fmaf_rn(gv, xs[r + ky][c * CI + k], acc[ky * 3 * CI + k]);
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 9 * CI; k++) atomicAdd(&sw[k][lane], acc[k]);
+  __syncthreads();
+  for (int e = threadIdx.x; e < 9 * CI * CO; e += 256) {
+    const int co = e / (9 * CI), k = e % (9 * CI);
+    atomicAdd(&dw[e], sw[k][co]);
+  }
 }
 
 // 2x2 average pooling, bf16 -> bf16 (the mean in float32). One thread per
@@ -307,45 +374,67 @@ __global__ void k_up_concat(const __nv_bfloat16* __restrict__ u, int Cu, const _
   }
 }
 
+// c[p] = u[p/2] (nearest upsampling); one thread per pixel and group of 8
+// channels. The convolution that follows reads the skip where it is
+// (unet_tc_conv_fwd's second input): writing the concatenation took 100 us of a
+// 1024^2 forward pass, the upsampled part alone 58.
+__global__ void k_up(const __nv_bfloat16* __restrict__ u, int C, int B, int H, int W, __nv_bfloat16* __restrict__ c) {
+  const int cg = C / 8, n = B * H * W * cg;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+    const int g = e % cg, p = e / cg;
+    const int i = p % W, r = p / W, j = r % H, b = r / H;
+    reinterpret_cast<uint4*>(c)[e] =
+        *reinterpret_cast<const uint4*>(u + (((long)b * (H / 2) + j / 2) * (W / 2) + i / 2) * C + 8 * g);
+  }
+}
+
 // Backward of up_concat: g_u[q] = (sum of dc over q's 4 children, first Cu
-// channels) * (act_u[q] > 0); skip[p] = dc[p][Cu:].
+// channels) * (act_u[q] > 0); skip[p] = dc[p][Cu:]. One thread per pixel and
+// group of 4 channels (Cu, Cs multiples of 4; fewer than 2^31 groups). Bound by
+// memory; a channel a thread took 93 us of a 4 x 256^2 training step, this 40.
+__device__ __forceinline__ float4 relu_mask4(float4 s, const __nv_bfloat16* act) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(act);
+  const __nv_bfloat16* a = reinterpret_cast<const __nv_bfloat16*>(&raw);
+  return make_float4(__bfloat162float(a[0]) > 0.0f ? s.x : 0.0f, __bfloat162float(a[1]) > 0.0f ? s.y : 0.0f,
+                     __bfloat162float(a[2]) > 0.0f ? s.z : 0.0f, __bfloat162float(a[3]) > 0.0f ? s.w : 0.0f);
+}
+
 __global__ void k_up_split_bwd(const float* __restrict__ dc, int Cu, int Cs, int B, int H, int W,
                                const __nv_bfloat16* __restrict__ act_u, float* __restrict__ g_u,
                                float* __restrict__ skip) {
-  const int C = Cu + Cs;
-  const int h = H / 2, w = W / 2;
-  const long nu = (long)B * h * w * Cu;
-  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < nu; e += (long)gridDim.x * blockDim.x) {
-    const int ch = (int)(e % Cu);
-    long r = e / Cu;
-    const int i = (int)(r % w);
-    r /= w;
-    const int j = (int)(r % h), b = (int)(r / h);
-    const long p = ((long)b * H + 2 * j) * W + 2 * i;
-    const float s = (dc[p * C + ch] + dc[(p + 1) * C + ch]) + (dc[(p + W) * C + ch] + dc[(p + W + 1) * C + ch]);
-    g_u[e] = __bfloat162float(act_u[e]) > 0.0f ? s : 0.0f;
+  const int C = Cu + Cs, h = H / 2, w = W / 2, gu = Cu / 4, gs = Cs / 4;
+  const int nu = B * h * w * gu, ns = B * H * W * gs;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nu; e += gridDim.x * blockDim.x) {
+    const int ch = 4 * (e % gu), q = e / gu;
+    const int i = q % w, r = q / w, j = r % h, b = r / h;
+    const float* d = dc + (((long)b * H + 2 * j) * W + 2 * i) * C + ch;
+    const float4 d00 = *reinterpret_cast<const float4*>(d), d01 = *reinterpret_cast<const float4*>(d + C);
+    const float4 d10 = *reinterpret_cast<const float4*>(d + (long)W * C);
+    const float4 d11 = *reinterpret_cast<const float4*>(d + (long)W * C + C);
+    const float4 s = make_float4((d00.x + d01.x) + (d10.x + d11.x), (d00.y + d01.y) + (d10.y + d11.y),
+                                 (d00.z + d01.z) + (d10.z + d11.z), (d00.w + d01.w) + (d10.w + d11.w));
+    *reinterpret_cast<float4*>(g_u + (long)q * Cu + ch) = relu_mask4(s, act_u + (long)q * Cu + ch);
   }
-  const long ns = (long)B * H * W * Cs;
-  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < ns; e += (long)gridDim.x * blockDim.x) {
-    const int ch = (int)(e % Cs);
-    const long p = e / Cs;
-    skip[e] = dc[p * C + Cu + ch];
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ns; e += gridDim.x * blockDim.x) {
+    const int ch = 4 * (e % gs), p = e / gs;
+    *reinterpret_cast<float4*>(skip + (long)p * Cs + ch) = *reinterpret_cast<const float4*>(dc + (long)p * C + Cu + ch);
   }
 }
 
 // g_s[p] = (skip[p] + dpool[p/2] / 4) * (act_s[p] > 0): the gradient of a
-// skip activation that also fed the pooling.
+// skip activation that also fed the pooling. One thread per pixel and group
+// of 4 channels (a channel a thread: 84 us of a 4 x 256^2 training step, this 28).
 __global__ void k_pool_bwd_mask(const float* __restrict__ skip, const float* __restrict__ dpool, int B, int H, int W,
                                 int C, const __nv_bfloat16* __restrict__ act, float* __restrict__ g) {
-  const long n = (long)B * H * W * C;
-  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
-    const int c = (int)(e % C);
-    const long p = e / C;
-    const int i = (int)(p % W);
-    const long r = p / W;
-    const int j = (int)(r % H), b = (int)(r / H);
-    const float d = skip[e] + 0.25f * dpool[(((long)b * (H / 2) + j / 2) * (W / 2) + i / 2) * C + c];
-    g[e] = __bfloat162float(act[e]) > 0.0f ? d : 0.0f;
+  const int cg = C / 4, n = B * H * W * cg;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+    const int ch = 4 * (e % cg), p = e / cg;
+    const int i = p % W, r = p / W, j = r % H, b = r / H;
+    const long k = (long)p * C + ch;
+    const float4 s = *reinterpret_cast<const float4*>(skip + k);
+    const float4 d = *reinterpret_cast<const float4*>(dpool + (((long)b * (H / 2) + j / 2) * (W / 2) + i / 2) * C + ch);
+    *reinterpret_cast<float4*>(g + k) = relu_mask4(
+        make_float4(s.x + 0.25f * d.x, s.y + 0.25f * d.y, s.z + 0.25f * d.z, s.w + 0.25f * d.w), act + k);
   }
 }
 
@@ -480,7 +569,7 @@ int Unet::alloc(long max_pixels, std::string* err) {
   bool ok = A((void**)&theta, nparam * 4, "weights") && A((void**)&m, nparam * 4, "adam m") &&
             A((void**)&v, nparam * 4, "adam v") && A((void**)&grad, nparam * 4, "gradient") &&
             A((void**)&theta16, nparam * 2, "bf16 weights") && A((void**)&wimg, nparam * 2, "weight images") &&
-            A((void**)&wimg_flip, 9L * 224 * 96 * 2, "flipped weight image") &&
+            A((void**)&wimg_flip, nparam * 2, "flipped weight images") &&
             A((void**)&gbf, max_pixels * 32L * 2, "bf16 gradient") && A((void**)&wflip, 9L * 224 * 96 * 2, "flipped weights") &&
             A((void**)&loss_dev, sizeof(double), "loss");
   if (!ok) return FL_ENOMEM;
@@ -515,9 +604,14 @@ void Unet::release() {
   for (auto* a : act) cudaFree(a);
 }
 
+// Tiles of a data gradient's output channels (at most 128 each).
+static int dgrad_tiles(int cin) { return (cin + 127) / 128; }
+
 void Unet::conv_fwd(cudaStream_t s, int l, const __nv_bfloat16* x, int B, int H, int W, __nv_bfloat16* y) {
   const UnetLayer& L = kUnetLayers[l];
-  if (unet_tc_conv_fwd(s, x, B, H, W, L.cin, theta16 + woff[l], wimg + woff[l], theta + boff[l], L.cout, y)) return;
+  if (unet_tc_conv_fwd(s, UnetInput{x, nullptr, L.cin}, B, H, W, L.cin, theta16 + woff[l], wimg + woff[l],
+                       theta + boff[l], L.cout, y))
+    return;
   if (L.cin == 3 && L.cout == 32 && L.k == 3) {
     dim3 g((unsigned)(((W + CT - 1) / CT) * ((H + CT - 1) / CT)), (unsigned)B);
     k_conv3_in3<<<g, CT * CT, 0, s>>>(x, H, W, theta16 + woff[l], theta + boff[l], y);
@@ -528,38 +622,76 @@ void Unet::conv_fwd(cudaStream_t s, int l, const __nv_bfloat16* x, int B, int H,
                                                         nullptr, nullptr);
 }
 
+// A decoder's first layer: u (Cu channels, half the size) upsampled, then the
+// skip (Cs channels), into y; c is room for the layer's input. The tensor-core
+// halo form reads the two parts where they are, so c holds the upsampled
+// channels alone; the other forms take the whole concatenation.
+void Unet::conv_up_fwd(cudaStream_t s, int l, const __nv_bfloat16* u, int Cu, const __nv_bfloat16* skip, int Cs, int B,
+                       int H, int W, __nv_bfloat16* c, __nv_bfloat16* y) {
+  const UnetLayer& L = kUnetLayers[l];
+  const long P = (long)B * H * W;
+  split[l] = unet_tc_two_inputs();
+  if (split[l]) {
+    k_up<<<grid_for(P * Cu / 8), 256, 0, s>>>(u, Cu, B, H, W, c);
+    if (unet_tc_conv_fwd(s, UnetInput{c, skip, Cu}, B, H, W, L.cin, theta16 + woff[l], wimg + woff[l], theta + boff[l],
+                         L.cout, y))
+      return;
+    split[l] = false;
+  }
+  k_up_concat<<<grid_for(P * L.cin), 256, 0, s>>>(u, Cu, skip, Cs, B, H, W, c);
+  conv_fwd(s, l, c, B, H, W, y);
+}
+
+// conv_bwd of a decoder's first layer, without the data gradient's ReLU mask.
+void Unet::conv_up_bwd(cudaStream_t s, int l, const __nv_bfloat16* u, int Cu, const __nv_bfloat16* skip, int Cs,
+                       __nv_bfloat16* c, const float* g, int B, int H, int W, float* gx) {
+  if (split[l] && !unet_tc_two_inputs()) {  // the forms changed since the forward pass
+    k_up_concat<<<grid_for((long)B * H * W * (Cu + Cs)), 256, 0, s>>>(u, Cu, skip, Cs, B, H, W, c);
+    split[l] = false;
+  }
+  conv_bwd(s, l, split[l] ? UnetInput{c, skip, Cu} : UnetInput{c, nullptr, Cu + Cs}, g, B, H, W, gx, nullptr);
+}
+
 // Weight gradient of layer l from its input x and pre-activation gradient g,
 // then (when gx is set) the data gradient into gx, masked by act_x > 0 when
 // act_x is set.
-void Unet::conv_bwd(cudaStream_t s, int l, const __nv_bfloat16* x, const float* g, int B, int H, int W, float* gx,
+void Unet::conv_bwd(cudaStream_t s, int l, const UnetInput& in, const float* g, int B, int H, int W, float* gx,
                     const __nv_bfloat16* act_x) {
+  const __nv_bfloat16* x = in.x;
   const UnetLayer& L = kUnetLayers[l];
   const long P = (long)B * H * W;
   // tensor cores take the output gradient in bf16
   const bool tc = unet_tc_enabled() && L.cout % 32 == 0;
-  if (tc) k_to_bf16<<<grid_for(P * L.cout), 256, 0, s>>>(g, P * L.cout, gbf);
-  if (tc && L.cin % 32 == 0 && unet_tc_conv_wgrad(s, x, gbf, B, H, W, L.cin, L.cout, grad + woff[l])) {
-    k_bias_grad<<<152, 256, 0, s>>>(g, P, L.cout, grad + boff[l]);
-  } else {
+  bool done = false;
+  if (tc) {
+    // (few blocks: each ends in an atomic per channel on the same words)
+    k_grad_bf16<<<std::min(grid_for(P * L.cout / 8), 608u), 256, 0, s>>>(g, P, L.cout, gbf, grad + boff[l]);
+    if (L.cin == 3 && L.cout == 32) {
+      k_wgrad_in3<<<304, 256, 0, s>>>(x, g, H, W, B, grad + woff[l]);
+      done = true;
+    } else {
+      done = L.cin % 32 == 0 && unet_tc_conv_wgrad(s, in, gbf, B, H, W, L.cin, L.cout, grad + woff[l]);
+    }
+  }
+  if (!done) {
     dim3 gw((unsigned)(((W + CT - 1) / CT) * ((H + CT - 1) / CT)), (unsigned)(B * ((L.cout + CO_T - 1) / CO_T)),
             (unsigned)((L.cin + CK - 1) / CK));
-    k_conv3_wgrad<<<gw, 256, 0, s>>>(x, g, H, W, L.cin, L.cout, grad + woff[l], grad + boff[l]);
+    k_conv3_wgrad<<<gw, 256, 0, s>>>(x, g, H, W, L.cin, L.cout, grad + woff[l], tc ? nullptr : grad + boff[l]);
   }
   if (gx == nullptr) return;
-  k_flip_weights<<<grid_for(9L * L.cin * L.cout), 256, 0, s>>>(theta16 + woff[l], L.cin, L.cout, wflip);
   if (tc) {
-    // the data gradient in tiles of at most 128 input channels (each tile's
-    // weight image built here)
-    const int tiles = (L.cin + 127) / 128, nt = L.cin / tiles;
+    // the data gradient in tiles of at most 128 input channels, each with its
+    // own weight image (refresh_weight_images)
+    const int tiles = dgrad_tiles(L.cin), nt = L.cin / tiles;
     bool ok = nt * tiles == L.cin && nt % 16 == 0;
     for (int t = 0; ok && t < tiles; t++) {
       const int n0 = t * nt;
-      unet_tc_weight_image(s, wflip + (long)n0 * 9 * L.cout, L.cout, nt, wimg_flip);
-      ok = unet_tc_conv_dgrad(s, gbf, B, H, W, L.cout, wimg_flip, nt, gx + n0, L.cin,
+      ok = unet_tc_conv_dgrad(s, gbf, B, H, W, L.cout, wimg_flip + woff[l] + (long)n0 * 9 * L.cout, nt, gx + n0, L.cin,
                               act_x != nullptr ? act_x + n0 : nullptr);
     }
     if (ok) return;
   }
+  k_flip_weights<<<grid_for(9L * L.cin * L.cout), 256, 0, s>>>(theta16 + woff[l], L.cin, L.cout, wflip);
   dim3 gd((unsigned)(((W + CT - 1) / CT) * ((H + CT - 1) / CT)), (unsigned)(B * ((L.cin + CO_T - 1) / CO_T)));
   k_conv3<float, EPI_GRAD><<<gd, CT * CT, 0, s>>>(g, H, W, L.cout, wflip, nullptr, L.cin, nullptr, gx, act_x);
 }
@@ -585,14 +717,11 @@ void Unet::forward(cudaStream_t s, int B, int H, int W) {
   k_pool<<<grid_for(P / 64 * 96), 256, 0, s>>>(act[A_S2], B, H2, W2, 96, act[A_P2]);
   conv_fwd(s, 6, act[A_P2], B, H3, W3, act[A_MA]);
   conv_fwd(s, 7, act[A_MA], B, H3, W3, act[A_M]);
-  k_up_concat<<<grid_for(P / 16 * 224), 256, 0, s>>>(act[A_M], 128, act[A_S2], 96, B, H2, W2, act[A_C2]);
-  conv_fwd(s, 8, act[A_C2], B, H2, W2, act[A_D2A]);
+  conv_up_fwd(s, 8, act[A_M], 128, act[A_S2], 96, B, H2, W2, act[A_C2], act[A_D2A]);
   conv_fwd(s, 9, act[A_D2A], B, H2, W2, act[A_D2]);
-  k_up_concat<<<grid_for(P / 4 * 160), 256, 0, s>>>(act[A_D2], 96, act[A_S1], 64, B, H1, W1, act[A_C1]);
-  conv_fwd(s, 10, act[A_C1], B, H1, W1, act[A_D1A]);
+  conv_up_fwd(s, 10, act[A_D2], 96, act[A_S1], 64, B, H1, W1, act[A_C1], act[A_D1A]);
   conv_fwd(s, 11, act[A_D1A], B, H1, W1, act[A_D1]);
-  k_up_concat<<<grid_for(P * 96), 256, 0, s>>>(act[A_D1], 64, act[A_S0], 32, B, H, W, act[A_C0]);
-  conv_fwd(s, 12, act[A_C0], B, H, W, act[A_D0A]);
+  conv_up_fwd(s, 12, act[A_D1], 64, act[A_S0], 32, B, H, W, act[A_C0], act[A_D0A]);
   conv_fwd(s, 13, act[A_D0A], B, H, W, act[A_D0]);
   k_head<<<grid_for(P), 256, 0, s>>>(act[A_D0], 32, P, theta16 + woff[14], theta + boff[14], out);
 }
@@ -600,31 +729,32 @@ void Unet::forward(cudaStream_t s, int B, int H, int W) {
 void Unet::backward(cudaStream_t s, int B, int H, int W) {
   const long P = (long)B * H * W;
   const int H1 = H / 2, W1 = W / 2, H2 = H / 4, W2 = W / 4, H3 = H / 8, W3 = W / 8;
+  auto one = [&](const __nv_bfloat16* x, int l) { return UnetInput{x, nullptr, kUnetLayers[l].cin}; };
   float* g0 = gbuf[0];
   float* g1 = gbuf[1];
   cudaMemsetAsync(grad, 0, nparam * 4, s);
-  k_head_bwd<<<grid_for(P), 256, 0, s>>>(act[A_D0], 32, P, theta16 + woff[14], dout, g0, grad + woff[14],
+  k_head_bwd<<<std::min(grid_for(P), 608u), 256, 0, s>>>(act[A_D0], 32, P, theta16 + woff[14], dout, g0, grad + woff[14],
                                         grad + boff[14]);
-  conv_bwd(s, 13, act[A_D0A], g0, B, H, W, g1, act[A_D0A]);           // dec0b
-  conv_bwd(s, 12, act[A_C0], g1, B, H, W, g0, nullptr);               // dec0a -> dc0 (96 ch)
+  conv_bwd(s, 13, one(act[A_D0A], 13), g0, B, H, W, g1, act[A_D0A]);           // dec0b
+  conv_up_bwd(s, 12, act[A_D1], 64, act[A_S0], 32, act[A_C0], g1, B, H, W, g0);       // dec0a -> dc0 (96 ch)
   k_up_split_bwd<<<grid_for(P / 4 * 64), 256, 0, s>>>(g0, 64, 32, B, H, W, act[A_D1], g1, gskip[0]);
-  conv_bwd(s, 11, act[A_D1A], g1, B, H1, W1, g0, act[A_D1A]);         // dec1b
-  conv_bwd(s, 10, act[A_C1], g0, B, H1, W1, g1, nullptr);             // dec1a -> dc1 (160 ch)
+  conv_bwd(s, 11, one(act[A_D1A], 11), g1, B, H1, W1, g0, act[A_D1A]);         // dec1b
+  conv_up_bwd(s, 10, act[A_D2], 96, act[A_S1], 64, act[A_C1], g0, B, H1, W1, g1);     // dec1a -> dc1 (160 ch)
   k_up_split_bwd<<<grid_for(P / 16 * 96), 256, 0, s>>>(g1, 96, 64, B, H1, W1, act[A_D2], g0, gskip[1]);
-  conv_bwd(s, 9, act[A_D2A], g0, B, H2, W2, g1, act[A_D2A]);          // dec2b
-  conv_bwd(s, 8, act[A_C2], g1, B, H2, W2, g0, nullptr);              // dec2a -> dc2 (224 ch)
+  conv_bwd(s, 9, one(act[A_D2A], 9), g0, B, H2, W2, g1, act[A_D2A]);          // dec2b
+  conv_up_bwd(s, 8, act[A_M], 128, act[A_S2], 96, act[A_C2], g1, B, H2, W2, g0);      // dec2a -> dc2 (224 ch)
   k_up_split_bwd<<<grid_for(P / 64 * 128), 256, 0, s>>>(g0, 128, 96, B, H2, W2, act[A_M], g1, gskip[2]);
-  conv_bwd(s, 7, act[A_MA], g1, B, H3, W3, g0, act[A_MA]);            // midb
-  conv_bwd(s, 6, act[A_P2], g0, B, H3, W3, gpool, nullptr);           // mida -> dp2 (96 ch, 1/64)
+  conv_bwd(s, 7, one(act[A_MA], 7), g1, B, H3, W3, g0, act[A_MA]);            // midb
+  conv_bwd(s, 6, one(act[A_P2], 6), g0, B, H3, W3, gpool, nullptr);           // mida -> dp2 (96 ch, 1/64)
   k_pool_bwd_mask<<<grid_for(P / 16 * 96), 256, 0, s>>>(gskip[2], gpool, B, H2, W2, 96, act[A_S2], g1);
-  conv_bwd(s, 5, act[A_E2A], g1, B, H2, W2, g0, act[A_E2A]);          // enc2b
-  conv_bwd(s, 4, act[A_P1], g0, B, H2, W2, gpool, nullptr);           // enc2a -> dp1 (64 ch, 1/16)
+  conv_bwd(s, 5, one(act[A_E2A], 5), g1, B, H2, W2, g0, act[A_E2A]);          // enc2b
+  conv_bwd(s, 4, one(act[A_P1], 4), g0, B, H2, W2, gpool, nullptr);           // enc2a -> dp1 (64 ch, 1/16)
   k_pool_bwd_mask<<<grid_for(P / 4 * 64), 256, 0, s>>>(gskip[1], gpool, B, H1, W1, 64, act[A_S1], g1);
-  conv_bwd(s, 3, act[A_E1A], g1, B, H1, W1, g0, act[A_E1A]);          // enc1b
-  conv_bwd(s, 2, act[A_P0], g0, B, H1, W1, gpool, nullptr);           // enc1a -> dp0 (32 ch, 1/4)
+  conv_bwd(s, 3, one(act[A_E1A], 3), g1, B, H1, W1, g0, act[A_E1A]);          // enc1b
+  conv_bwd(s, 2, one(act[A_P0], 2), g0, B, H1, W1, gpool, nullptr);           // enc1a -> dp0 (32 ch, 1/4)
   k_pool_bwd_mask<<<grid_for(P * 32), 256, 0, s>>>(gskip[0], gpool, B, H, W, 32, act[A_S0], g1);
-  conv_bwd(s, 1, act[A_E0A], g1, B, H, W, g0, act[A_E0A]);            // enc0b
-  conv_bwd(s, 0, act[A_X0], g0, B, H, W, nullptr, nullptr);           // enc0a (weights only)
+  conv_bwd(s, 1, one(act[A_E0A], 1), g1, B, H, W, g0, act[A_E0A]);            // enc0b
+  conv_bwd(s, 0, one(act[A_X0], 0), g0, B, H, W, nullptr, nullptr);           // enc0a (weights only)
 }
 
 void Unet::loss(cudaStream_t s, long P, float inv_n) {
@@ -646,12 +776,21 @@ void Unet::refresh_bf16(cudaStream_t s) {
 }
 
 // The halo-form tensor-core convolutions read their weights as per-chunk
-// images (all 9 taps' B tiles of 32 input channels, contiguous).
+// images (all 9 taps' B tiles of 32 input channels, contiguous): every layer's
+// forward image and its data gradient's (the flipped weights, per tile of
+// input channels) in one launch, whenever the weights change.
 void Unet::refresh_weight_images(cudaStream_t s) {
+  UnetImages im{};
   for (int l = 0; l < UNET_LAYERS; l++) {
     const UnetLayer& L = kUnetLayers[l];
-    if (L.k == 3 && L.cin % 32 == 0) unet_tc_weight_image(s, theta16 + woff[l], L.cin, L.cout, wimg + woff[l]);
+    if (L.k != 3 || L.cin % 32 != 0) continue;
+    im.job[im.n++] = UnetImage{theta16 + woff[l], wimg + woff[l], L.cin, L.cout, L.cin, -1};
+    const int tiles = dgrad_tiles(L.cin), nt = L.cin / tiles;
+    for (int t = 0; t < tiles; t++)
+      im.job[im.n++] = UnetImage{theta16 + woff[l], wimg_flip + woff[l] + (long)t * nt * 9 * L.cout, L.cout, nt, L.cin,
+                                 t * nt};
   }
+  unet_tc_weight_images(s, im);
 }
 
 // ------------------------------------------------------------- warm start

@@ -20,6 +20,28 @@ extern const UnetLayer kUnetLayers[UNET_LAYERS];
 
 long long unet_num_params();
 
+// A convolution's input: the first `split` channels from x (split channels a
+// pixel), the others from x2 (null: all from x).
+struct UnetInput {
+  const __nv_bfloat16* x;
+  const __nv_bfloat16* x2;
+  int split;
+};
+
+// One weight image to build (unet_tc_weight_images): of the convolution of
+// `cin` channels to `n`, from the weights w of a layer of `wcin` input
+// channels; n0 < 0: that layer itself, else the data gradient's tile of its
+// input channels from n0 on.
+struct UnetImage {
+  const __nv_bfloat16* w;
+  __nv_bfloat16* img;
+  int cin, n, wcin, n0;
+};
+struct UnetImages {
+  int n;
+  UnetImage job[32];
+};
+
 struct Unet {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -33,7 +55,8 @@ struct Unet {
   __nv_bfloat16* theta16 = nullptr;  // bf16 copies used by the kernels
   __nv_bfloat16* wflip = nullptr;    // flipped/transposed weights of one layer
   __nv_bfloat16* wimg = nullptr;     // tensor-core weight images (offsets woff)
-  __nv_bfloat16* wimg_flip = nullptr;  // image of one output-channel tile of the flipped weights
+  __nv_bfloat16* wimg_flip = nullptr;  // images of the flipped weights' tiles (offsets woff)
+  bool split[UNET_LAYERS] = {};        // the layer's input is in two parts (conv_up_fwd)
   __nv_bfloat16* gbf = nullptr;        // bf16 copy of an output gradient (tensor-core data gradient)
   double* loss_dev = nullptr;
   __nv_bfloat16* act[ACT_COUNT] = {};
@@ -59,8 +82,12 @@ struct Unet {
   void refresh_bf16(cudaStream_t s);
   void refresh_weight_images(cudaStream_t s);
   void conv_fwd(cudaStream_t s, int l, const __nv_bfloat16* x, int B, int H, int W, __nv_bfloat16* y);
-  void conv_bwd(cudaStream_t s, int l, const __nv_bfloat16* x, const float* g, int B, int H, int W, float* gx,
+  void conv_bwd(cudaStream_t s, int l, const UnetInput& in, const float* g, int B, int H, int W, float* gx,
                 const __nv_bfloat16* act_x);
+  void conv_up_fwd(cudaStream_t s, int l, const __nv_bfloat16* u, int Cu, const __nv_bfloat16* skip, int Cs, int B,
+                   int H, int W, __nv_bfloat16* c, __nv_bfloat16* y);
+  void conv_up_bwd(cudaStream_t s, int l, const __nv_bfloat16* u, int Cu, const __nv_bfloat16* skip, int Cs,
+                   __nv_bfloat16* c, const float* g, int B, int H, int W, float* gx);
 };
 
 // Tensor-core (tcgen05) forward convolution with bias and ReLU; returns
@@ -68,10 +95,12 @@ struct Unet {
 // tensor-core path is switched off, in which case the caller runs the
 // CUDA-core kernel.
 // w: [Cout][3][3][Cin]; wimg: the same weights arranged by
-// unet_tc_weight_image (read by the halo form).
-bool unet_tc_conv_fwd(cudaStream_t s, const __nv_bfloat16* x, int B, int H, int W, int Cin, const __nv_bfloat16* w,
+// unet_tc_weight_images (read by the halo form, which alone takes an input in
+// two parts: unet_tc_two_inputs).
+bool unet_tc_conv_fwd(cudaStream_t s, const UnetInput& in, int B, int H, int W, int Cin, const __nv_bfloat16* w,
                       const __nv_bfloat16* wimg, const float* bias, int Cout, __nv_bfloat16* y);
-void unet_tc_weight_image(cudaStream_t s, const __nv_bfloat16* w, int Cin, int Cout, __nv_bfloat16* img);
+bool unet_tc_two_inputs();
+void unet_tc_weight_images(cudaStream_t s, const UnetImages& im);
 // Tensor-core data gradient of a 3x3 convolution over the output-channel
 // tile of N channels: gx = conv(g, W') (g bf16 with Cin channels, wimg the
 // image of W' rows of the tile), zeroed where mask <= 0 (mask optional);
@@ -81,7 +110,7 @@ void unet_tc_weight_image(cudaStream_t s, const __nv_bfloat16* w, int Cin, int C
 // sum over pixels of g[p][n] x[p + off(tap)][ci] (x and g bf16 NHWC; dw
 // float, accumulated with atomics). Cin and Cout multiples of 32. False
 // (nothing launched) when not covered or the tensor cores are off.
-bool unet_tc_conv_wgrad(cudaStream_t s, const __nv_bfloat16* x, const __nv_bfloat16* g, int B, int H, int W, int Cin,
+bool unet_tc_conv_wgrad(cudaStream_t s, const UnetInput& in, const __nv_bfloat16* g, int B, int H, int W, int Cin,
                         int Cout, float* dw);
 bool unet_tc_conv_dgrad(cudaStream_t s, const __nv_bfloat16* g, int B, int H, int W, int Cin, const __nv_bfloat16* wimg,
                         int N, float* gx, int ldg, const __nv_bfloat16* mask);

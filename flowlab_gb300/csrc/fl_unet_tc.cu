@@ -355,7 +355,8 @@ struct HaloOut {
 constexpr int WS_EPI_WARPS = 8;
 constexpr int WS_THREADS = 64 + 32 * WS_EPI_WARPS;
 
-__global__ void __launch_bounds__(WS_THREADS) k_conv3_halo_ws(const __grid_constant__ CUtensorMap xmap, int H,
+__global__ void __launch_bounds__(WS_THREADS) k_conv3_halo_ws(const __grid_constant__ CUtensorMap xmap,
+                                                              const __grid_constant__ CUtensorMap xmap2, int split, int H,
                                                               int W, int B, const __nv_bfloat16* __restrict__ wimg,
                                                               int N, int nchunks, int TR, int ns, int ncols,
                                                               int stacked, HaloOut out) {
@@ -416,7 +417,8 @@ __global__ void __launch_bounds__(WS_THREADS) k_conv3_halo_ws(const __grid_const
           mbar_expect_tx(fb, tx_bytes);
 #pragma unroll
           for (int g = 0; g < 4; g++)
-            tma_load_4d(smem_u32(st + g * plane), &xmap, c * 32 + 8 * g, bx * HALO_TW - 1, by * TR - 1, img, fb);
+            tma_load_4d(smem_u32(st + g * plane), c * 32 < split ? &xmap : &xmap2,
+                        (c * 32 < split ? c * 32 : c * 32 - split) + 8 * g, bx * HALO_TW - 1, by * TR - 1, img, fb);
           bulk_load(smem_u32(st + stage_a), wimg + (long)c * 9 * 32 * N, (uint32_t)stage_b, fb);
         }
       }
@@ -586,38 +588,48 @@ __global__ void __launch_bounds__(WS_THREADS) k_conv3_halo_ws(const __grid_const
   }
 }
 
-// Weight image of one layer for the halo form: per 32-channel chunk c, per
-// tap t, per 8-channel group g, per output channel n, 8 channels:
-// img[(((c * 9 + t) * 4 + g) * N + n) * 8 + j] = w[(n * 9 + t) * Cin + 32c + 8g + j]
+// Weight images for the halo form (one per blockIdx.y): per 32-channel chunk
+// c, per tap t, per 8-channel group g, per output channel n, 8 channels:
+// img[(((c * 9 + t) * 4 + g) * N + n) * 8 + j] = w(n, t, 32c + 8g + j)
 // — the shared-memory B tiles of all 9 taps of a chunk, contiguous.
 //
 // Stacked (3 N <= 256): per chunk c, per kx, per group g, the three ky taps'
 // rows stacked along N (row ky N + n), 8 channels:
-// img[((((c * 3 + kx) * 4 + g) * 3 + ky) * N + n) * 8 + j] = w[(n * 9 + 3 ky + kx) * Cin + 32c + 8g + j]
-__global__ void k_weight_image(const __nv_bfloat16* __restrict__ w, int Cin, int N, int stacked,
-                               __nv_bfloat16* __restrict__ img) {
-  const long total = 9L * Cin * N;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const int j = (int)(i & 7);
-    long q = i >> 3;
-    const int n = (int)(q % N);
+// img[((((c * 3 + kx) * 4 + g) * 3 + ky) * N + n) * 8 + j] = w(n, 3 ky + kx, 32c + 8g + j)
+//
+// w(n, t, k) is the layer's weight [n][t][k], or of its data gradient the
+// flipped one, [k][8 - t][n0 + n].
+bool halo_stacked(int N);
+struct HaloImages {
+  UnetImages im;
+  int stacked[32];
+};
+__global__ void __launch_bounds__(256) k_weight_images(const __grid_constant__ HaloImages a) {
+  const UnetImage& m = a.im.job[blockIdx.y];
+  const int N = m.n, stacked = a.stacked[blockIdx.y];
+  const int total = 9 * m.cin * N;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int j = i & 7;
+    int q = i >> 3;
+    const int n = q % N;
     q /= N;
     int t, g, c;
     if (stacked) {
-      const int ky = (int)(q % 3);
+      const int ky = q % 3;
       q /= 3;
-      g = (int)(q & 3);
+      g = q & 3;
       q >>= 2;
-      const int kx = (int)(q % 3);
-      c = (int)(q / 3);
+      const int kx = q % 3;
+      c = q / 3;
       t = 3 * ky + kx;
     } else {
-      g = (int)(q & 3);
+      g = q & 3;
       q >>= 2;
-      t = (int)(q % 9);
-      c = (int)(q / 9);
+      t = q % 9;
+      c = q / 9;
     }
-    img[i] = w[((long)n * 9 + t) * Cin + 32 * c + 8 * g + j];
+    const int k = 32 * c + 8 * g + j;
+    m.img[i] = m.n0 < 0 ? m.w[((long)n * 9 + t) * m.wcin + k] : m.w[((long)k * 9 + (8 - t)) * m.wcin + m.n0 + n];
   }
 }
 
@@ -653,6 +665,7 @@ constexpr int WG_SMEM = 2 * WG_STAGE + 128;
 constexpr int WG_THREADS = 192;
 
 __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad_tc(const __grid_constant__ CUtensorMap xmap,
+                                                               const __grid_constant__ CUtensorMap xmap2, int split,
                                                                const __grid_constant__ CUtensorMap gmap, int H, int W,
                                                                int B, int Cin, int tiles_per_cta,
                                                                float* __restrict__ dw) {
@@ -708,7 +721,8 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad_tc(const __grid_cons
         const uint32_t fb = smem_u32(&full[s]);
         mbar_expect_tx(fb, tx);
         for (int g = 0; g < cb / 8; g++)
-          tma_load_4d(smem_u32(st + g * WG_PL), &xmap, ci0 + 8 * g, bx * WG_TW - 1, y - 1, img, fb);
+          tma_load_4d(smem_u32(st + g * WG_PL), ci0 + 8 * g < split ? &xmap : &xmap2,
+                      ci0 + 8 * g < split ? ci0 + 8 * g : ci0 + 8 * g - split, bx * WG_TW - 1, y - 1, img, fb);
         for (int g = 0; g < WG_NB / 8; g++)
           tma_load_4d(smem_u32(st + WG_A + g * WG_GPL), &gmap, n0 + 8 * g, bx * WG_TW, y, img, fb);
       }
@@ -826,40 +840,56 @@ void unet_tc_setup() {
   cudaGetLastError();
 }
 
-void unet_tc_weight_image(cudaStream_t s, const __nv_bfloat16* w, int Cin, int Cout, __nv_bfloat16* img) {
-  const long total = 9L * Cin * Cout;
-  k_weight_image<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(w, Cin, Cout, halo_stacked(Cout) ? 1 : 0, img);
+void unet_tc_weight_images(cudaStream_t s, const UnetImages& im) {
+  HaloImages a{};
+  a.im = im;
+  for (int k = 0; k < im.n; k++) a.stacked[k] = halo_stacked(im.job[k].n) ? 1 : 0;
+  k_weight_images<<<dim3(64, (unsigned)im.n), 256, 0, s>>>(a);
 }
 
 void unet_tc_enable(bool on) { g_tc_on = on; }
 void unet_tc_form(int form) { g_tc_form = form; }
 bool unet_tc_enabled() { return g_tc_on; }
+bool unet_tc_two_inputs() { return g_tc_on && g_tc_form != 0 && g_halo_ok; }
 
 namespace {
 
-bool launch_halo(cudaStream_t s, const __nv_bfloat16* x, int B, int H, int W, int Cin, const __nv_bfloat16* wimg,
-                 int N, const HaloOut& out) {
+// x as a 4-D tensor (channels, columns, rows, images), boxes of 8 channels x
+// `cols` columns x `rows` rows; outside the image the box reads zeros.
+bool image_map(CUtensorMap* map, const __nv_bfloat16* x, int C, int W, int H, int B, int cols, int rows) {
+  const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
+  const cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
+  const cuuint32_t box[4] = {8, (cuuint32_t)cols, (cuuint32_t)rows, 1};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  return g_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(x), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The maps of an input's two parts (the second is the first again when there
+// is only one). A part boundary must be one of 32-channel chunks.
+bool input_maps(CUtensorMap* m, const UnetInput& in, int Cin, int W, int H, int B, int cols, int rows) {
+  if (in.x2 == nullptr ? in.split != Cin : in.split % KC != 0 || in.split <= 0 || in.split >= Cin) return false;
+  if (!image_map(&m[0], in.x, in.split, W, H, B, cols, rows)) return false;
+  if (in.x2 != nullptr) return image_map(&m[1], in.x2, Cin - in.split, W, H, B, cols, rows);
+  m[1] = m[0];
+  return true;
+}
+
+bool launch_halo(cudaStream_t s, const UnetInput& in, int B, int H, int W, int Cin, const __nv_bfloat16* wimg, int N,
+                 const HaloOut& out) {
   int tr, ns, ncols;
   const int nchunks = Cin / KC;
   if (!halo_ws_shape(N, &tr, &ns, &ncols)) return false;
-  // x as a 4-D tensor (channels, columns, rows, images), boxes of 8 channels
-  // x 130 columns x (tr + 2) rows; outside the image the box reads zeros
-  CUtensorMap map;
-  const cuuint64_t dims[4] = {(cuuint64_t)Cin, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
-  const cuuint64_t strides[3] = {(cuuint64_t)Cin * 2, (cuuint64_t)W * Cin * 2, (cuuint64_t)H * W * Cin * 2};
-  const cuuint32_t box[4] = {8, (cuuint32_t)HALO_W, (cuuint32_t)(tr + 2), 1};
-  const cuuint32_t estr[4] = {1, 1, 1, 1};
-  if (g_encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(x), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return false;
+  CUtensorMap map[2];
+  if (!input_maps(map, in, Cin, W, H, B, HALO_W, tr + 2)) return false;
   const int tiles_x = (W + HALO_TW - 1) / HALO_TW, tiles_y = (H + tr - 1) / tr;
   const long ntiles = (long)tiles_x * tiles_y * B;
   if (ntiles >= (1L << 31)) return false;
   const int grid = (int)(ntiles < g_num_sms ? ntiles : g_num_sms);
   const int smem = 2 * halo_stage_bytes(tr, N) + WS_BAR_BYTES;
   if (smem > HALO_SMEM_MAX) return false;
-  k_conv3_halo_ws<<<grid, WS_THREADS, smem, s>>>(map, H, W, B, wimg, N, nchunks, tr, ns, ncols,
+  k_conv3_halo_ws<<<grid, WS_THREADS, smem, s>>>(map[0], map[1], in.split, H, W, B, wimg, N, nchunks, tr, ns, ncols,
                                                   halo_stacked(N) ? 1 : 0, out);
   return true;
 }
@@ -873,34 +903,17 @@ bool unet_tc_conv_dgrad(cudaStream_t s, const __nv_bfloat16* g, int B, int H, in
   if ((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(wimg)) & 15) return false;
   if (reinterpret_cast<uintptr_t>(gx) & 15) return false;
   const HaloOut out{nullptr, gx, mask, nullptr, ldg};
-  return launch_halo(s, g, B, H, W, Cin, wimg, N, out);
+  return launch_halo(s, UnetInput{g, nullptr, Cin}, B, H, W, Cin, wimg, N, out);
 }
 
-bool unet_tc_conv_wgrad(cudaStream_t s, const __nv_bfloat16* x, const __nv_bfloat16* g, int B, int H, int W, int Cin,
+bool unet_tc_conv_wgrad(cudaStream_t s, const UnetInput& in, const __nv_bfloat16* g, int B, int H, int W, int Cin,
                         int Cout, float* dw) {
   if (!g_tc_on || g_tc_form == 0 || !g_halo_ok) return false;
   if (Cin % 32 != 0 || Cout % WG_NB != 0) return false;
-  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(g)) & 15) return false;
-  CUtensorMap xmap, gmap;
-  const cuuint32_t estr[4] = {1, 1, 1, 1};
-  {
-    const cuuint64_t dims[4] = {(cuuint64_t)Cin, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
-    const cuuint64_t strides[3] = {(cuuint64_t)Cin * 2, (cuuint64_t)W * Cin * 2, (cuuint64_t)H * W * Cin * 2};
-    const cuuint32_t box[4] = {8, (cuuint32_t)HALO_W, 3, 1};
-    if (g_encode(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(x), dims, strides, box, estr,
-                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return false;
-  }
-  {
-    const cuuint64_t dims[4] = {(cuuint64_t)Cout, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
-    const cuuint64_t strides[3] = {(cuuint64_t)Cout * 2, (cuuint64_t)W * Cout * 2, (cuuint64_t)H * W * Cout * 2};
-    const cuuint32_t box[4] = {8, (cuuint32_t)WG_TW, 1, 1};
-    if (g_encode(&gmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(g), dims, strides, box, estr,
-                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return false;
-  }
+  if ((reinterpret_cast<uintptr_t>(in.x) | reinterpret_cast<uintptr_t>(in.x2) | reinterpret_cast<uintptr_t>(g)) & 15)
+    return false;
+  CUtensorMap map[2], gmap;
+  if (!input_maps(map, in, Cin, W, H, B, HALO_W, 3) || !image_map(&gmap, g, Cout, W, H, B, WG_TW, 1)) return false;
   const int nblk = Cout / WG_NB, cblk = (Cin + WG_CB - 1) / WG_CB;
   const long ntiles = (long)((W + WG_TW - 1) / WG_TW) * H * B;
   long ctas = (g_num_sms + nblk * cblk - 1) / (nblk * cblk);
@@ -910,7 +923,7 @@ bool unet_tc_conv_wgrad(cudaStream_t s, const __nv_bfloat16* x, const __nv_bfloa
   ctas = (ntiles + per - 1) / per;
   if (per >= (1L << 30) || ctas >= 65535) return false;
   dim3 grid((unsigned)ctas, (unsigned)nblk, (unsigned)cblk);
-  k_conv3_wgrad_tc<<<grid, WG_THREADS, WG_SMEM, s>>>(xmap, gmap, H, W, B, Cin, (int)per, dw);
+  k_conv3_wgrad_tc<<<grid, WG_THREADS, WG_SMEM, s>>>(map[0], map[1], in.split, gmap, H, W, B, Cin, (int)per, dw);
   return true;
 }
 
@@ -928,18 +941,20 @@ int unet_tc_take_error() {
   return v;
 }
 
-bool unet_tc_conv_fwd(cudaStream_t s, const __nv_bfloat16* x, int B, int H, int W, int Cin, const __nv_bfloat16* w,
+bool unet_tc_conv_fwd(cudaStream_t s, const UnetInput& in, int B, int H, int W, int Cin, const __nv_bfloat16* w,
                       const __nv_bfloat16* wimg, const float* bias, int Cout, __nv_bfloat16* y) {
   if (!g_tc_on) return false;
   if (Cin % KC != 0 || Cout % 16 != 0 || Cout < 16 || Cout > 128) return false;
   // 16-byte aligned rows of x, w and y
-  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y) |
+  const __nv_bfloat16* x = in.x;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(in.x2) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y) |
        reinterpret_cast<uintptr_t>(wimg)) & 15)
     return false;
   if (g_tc_form != 0 && g_halo_ok) {
     const HaloOut out{y, nullptr, nullptr, bias, Cout};
-    if (launch_halo(s, x, B, H, W, Cin, wimg, Cout, out)) return true;
+    if (launch_halo(s, in, B, H, W, Cin, wimg, Cout, out)) return true;
   }
+  if (in.x2 != nullptr) return false;
   if (!g_attr_set) return false;  // unet_tc_setup not called on this device
   int ncols = 32;
   while (ncols < Cout) ncols <<= 1;
