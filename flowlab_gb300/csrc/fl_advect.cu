@@ -88,7 +88,10 @@ __device__ __forceinline__ void advect_faces(int nx, int ny, const S& h, const f
   const Stencil pu = stencil_u(nx, ny, h, bxu, byu), pv = stencil_v(nx, ny, h, bxv, byv);
   // the correction's launch starts while the forward pass drains: only what
   // that wrote (hat, the offsets in out) is read after the wait
-  if (MODE == 1) dep_wait();
+  if (MODE == 1) {
+    dep_wait();
+    dep_trigger();
+  }
   float ru, rv;
   if (MODE == 0) {
     ru = sample(u_in, pu, nx + 1);
@@ -131,8 +134,8 @@ __global__ void __launch_bounds__(256) k_advect_velocity(int nx, int ny, Spacing
 // thread writes.
 template <int MODE, bool TAIL, class S>
 __device__ __forceinline__ void advect_cells(int nx, int ny, const S& h, int dnx, int dny, const S& dh,
-                                             const float* __restrict__ u, const float* __restrict__ v,
-                                             const float* __restrict__ q_in, const float* q_hat, float* q_out,
+                                             const float* u, const float* v, const float* __restrict__ q_in,
+                                             const float* q_hat, float* q_out,
                                              const uint8_t* __restrict__ label, const StepScalars* __restrict__ sc,
                                              const float* __restrict__ patch, int pi0, int pj0, int pnx, int pny,
                                              float* at) {
@@ -150,7 +153,10 @@ __device__ __forceinline__ void advect_cells(int nx, int ny, const S& h, int dnx
   if (solid_or_outside(label, nx, ny, li, lj)) {
 #pragma unroll
     for (int c = 0; c < DYE_CHANNELS; c++) q[c] = q_in[k + c * cells];
-    if (MODE == 1) dep_wait();
+    if (MODE == 1) {
+      dep_wait();
+      dep_trigger();
+    }
   } else {
     const float x = ((float)i + 0.5f) * dh.h;
     const float y = ((float)j + 0.5f) * dh.h;
@@ -165,6 +171,7 @@ __device__ __forceinline__ void advect_cells(int nx, int ny, const S& h, int dnx
       for (int c = 0; c < DYE_CHANNELS; c++) q[c] = sample(q_in + c * cells, p, dnx);
     } else {
       dep_wait();  // hat and the offset in q_out are the forward pass's, whose end this launch need not await
+      dep_trigger();
       const int ck = __float_as_int(q_out[k]);
 #pragma unroll
       for (int c = 0; c < DYE_CHANNELS; c++) {
@@ -199,13 +206,16 @@ __device__ __forceinline__ void advect_cells(int nx, int ny, const S& h, int dnx
 
 template <int MODE, bool TAIL>
 __global__ void __launch_bounds__(256) k_advect_dye(int nx, int ny, Spacing h, int dnx, int dny, Spacing dh,
-                                                    const float* __restrict__ u, const float* __restrict__ v,
-                                                    const float* __restrict__ q_in, const float* q_hat, float* q_out,
+                                                    const float* u, const float* v, const float* __restrict__ q_in,
+                                                    const float* q_hat, float* q_out,
                                                     const uint8_t* __restrict__ label,
                                                     const StepScalars* __restrict__ sc,
                                                     const float* __restrict__ patch, int pi0, int pj0, int pnx,
                                                     int pny, float* at) {
-  if (MODE == 0) dep_trigger();
+  if (MODE == 0) {
+    dep_wait();  // u and v are the launch before's (ordinary loads: not restrict)
+    dep_trigger();
+  }
   if (h.pow2 && dh.pow2)
     advect_cells<MODE, TAIL>(nx, ny, SpacingPow2(h), dnx, dny, SpacingPow2(dh), u, v, q_in, q_hat, q_out, label, sc,
                              patch, pi0, pj0, pnx, pny, at);
@@ -241,22 +251,19 @@ cudaError_t preload_advect_kernels() {
 
 void launch_advect_dye(cudaStream_t s, int nx, int ny, float h, int dnx, int dny, float dh, int mac, const float* u,
                        const float* v, const float* q_in, float* q_hat, float* q_out, const uint8_t* label,
-                       const StepScalars* sc, bool tail, const float* patch, int pi0, int pj0, int pnx, int pny) {
+                       const StepScalars* sc, bool tail, const float* patch, int pi0, int pj0, int pnx, int pny,
+                       bool early) {
   const Spacing hs = make_spacing(h), ds = make_spacing(dh);
   dim3 blk(32, 8);
   dim3 grd((dnx + blk.x - 1) / blk.x, (dny + blk.y - 1) / blk.y);
   if (mac) {
-    k_advect_dye<0, false><<<grd, blk, 0, s>>>(nx, ny, hs, dnx, dny, ds, u, v, q_in, nullptr, q_hat, label, sc, nullptr,
-                                               0, 0, 0, 0, q_out);
+    launch_dependent(early, k_advect_dye<0, false>, grd, blk, s, nx, ny, hs, dnx, dny, ds, u, v, q_in, nullptr, q_hat,
+                     label, sc, nullptr, 0, 0, 0, 0, q_out);
     launch_dependent(true, tail ? k_advect_dye<1, true> : k_advect_dye<1, false>, grd, blk, s, nx, ny, hs, dnx, dny, ds,
                      u, v, q_in, q_hat, q_out, label, sc, tail ? patch : nullptr, pi0, pj0, pnx, pny, nullptr);
   } else {
-    if (tail)
-      k_advect_dye<0, true><<<grd, blk, 0, s>>>(nx, ny, hs, dnx, dny, ds, u, v, q_in, nullptr, q_out, label, sc, patch,
-                                                pi0, pj0, pnx, pny, nullptr);
-    else
-      k_advect_dye<0, false><<<grd, blk, 0, s>>>(nx, ny, hs, dnx, dny, ds, u, v, q_in, nullptr, q_out, label, sc,
-                                                 nullptr, 0, 0, 0, 0, nullptr);
+    launch_dependent(early, tail ? k_advect_dye<0, true> : k_advect_dye<0, false>, grd, blk, s, nx, ny, hs, dnx, dny, ds,
+                     u, v, q_in, nullptr, q_out, label, sc, tail ? patch : nullptr, pi0, pj0, pnx, pny, nullptr);
   }
 }
 

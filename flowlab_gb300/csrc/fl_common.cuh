@@ -291,7 +291,9 @@ __device__ __forceinline__ bool solid_cell(const uint8_t* __restrict__ label, in
 // (fl_internal.h) may start while the kernel before it drains. dep_wait blocks
 // until that kernel has completed and its results are visible (at once in a
 // kernel launched otherwise); before it, a kernel reads only what kernels
-// further back wrote. dep_trigger, after it, lets the next kernel start
+// further back wrote, and what that kernel wrote it reads with ordinary loads
+// behind the wait: through parameters that are not __restrict__, whose loads the
+// compiler may move above it. dep_trigger, after it, lets the next kernel start
 // likewise: so whoever runs ahead of its dep_wait has only its immediate
 // predecessor still running.
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

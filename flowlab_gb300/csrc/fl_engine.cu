@@ -392,7 +392,11 @@ void wait_codes(Engine* e, cudaStream_t s) {
 }
 
 // advect u,v -> [stir] -> [confinement] -> body forces -> divergence
-void enqueue_pre(Engine* e, cudaStream_t s, int par, bool stir) {
+// host: fl_step_host's step, which waits for the fields that arrive meanwhile
+// and marks where its results are final (event nodes when captured; a step on
+// resident fields is kernels alone, each of which may start while the one
+// before it drains).
+void enqueue_pre(Engine* e, cudaStream_t s, int par, bool stir, bool host) {
   Level& L0 = e->levels[0];
   const int mac = e->prm.scheme == FL_MACCORMACK;
   const double N = (double)e->cells(), F = (double)(e->ufaces() + e->vfaces()), D = (double)e->dye_cells();
@@ -407,29 +411,32 @@ void enqueue_pre(Engine* e, cudaStream_t s, int par, bool stir) {
   if (stir) launch_stir(s, e->nx, e->ny, e->h, u, v, L0.label, e->stir);
   const bool conf = e->prm.confinement != 0;
   const bool beta_on = e->prm.beta != 0, alpha_on = e->prm.alpha != 0;
+  const bool early = capturing(s);  // the launch before is a kernel of this graph
   tok = prof_begin(*e, FL_PH_BODY_FORCES);
   double fbytes = 0;
   int flaunch = 0;
   if (conf) {
-    launch_vort_confine(s, e->nx, e->ny, e->h, u, v, L0.label, (float)e->prm.confinement, e->fx, e->fy);
+    launch_vort_confine(s, e->nx, e->ny, e->h, u, v, L0.label, (float)e->prm.confinement, e->fx, e->fy, early);
     fbytes += 4 * F + N + 8 * N;
     flaunch += 1;
   }
-  if (beta_on || alpha_on) wait_dye(e, s);
+  if (host && (beta_on || alpha_on)) wait_dye(e, s);
   if (beta_on || alpha_on || conf) {
     launch_forces(s, e->nx, e->ny, e->h, e->dnx, e->dny, e->dh, u, v, e->dye[par], L0.label, beta_on, alpha_on, conf,
-                  e->fx, e->fy, e->sc);
+                  e->fx, e->fy, e->sc, early && !(host && (beta_on || alpha_on)));
     fbytes += 8 * F + N + (beta_on ? 4 * D : 0) + (alpha_on ? 4 * D : 0) + (conf ? 8 * N : 0);
     flaunch += 1;
   }
   prof_end(*e, tok, fbytes, flaunch);
-  launch_fill32(s, e->acc, 4 * sizeof(double) / 4, 0u);  // b_sq, res_sq, n_fluid, n_res
+  launch_fill32(s, e->acc, 4 * sizeof(double) / 4, 0u, early);  // b_sq, res_sq, n_fluid, n_res
   tok = prof_begin(*e, FL_PH_DIVERGENCE);
   launch_divergence(s, e->nx, e->ny, e->h, u, v, L0.b, e->prm.solver == FL_SOLVER_MG, L0.label, e->sc, e->acc,
-                    step_mixed(e) ? e->b_lo : nullptr);
+                    step_mixed(e) ? e->b_lo : nullptr, early);
   prof_end(*e, tok, 4 * F + N + 4 * N, 1);
-  wait_p(e, s);
-  wait_codes(e, s);
+  if (host) {
+    wait_p(e, s);
+    wait_codes(e, s);
+  }
   if (e->prm.warm_extrapolate && e->prm.solver == FL_SOLVER_MG) {
     const bool mixed = e->prm.mixed != 0;
     launch_extrapolate(s, e->cells(), L0.label, L0.x[0], e->pprev32, mixed ? e->p64[0] : nullptr,
@@ -515,7 +522,9 @@ void enqueue_rb_fixed(Engine* e, cudaStream_t s) {
 }
 
 // subtract gradient + outflow -> dye (advect, decay, inlet) -> CFL
-cudaError_t enqueue_post(Engine* e, cudaStream_t s, int par, bool device_dt) {
+// joined: the stream has just joined another (the first launch is an ordinary one).
+cudaError_t enqueue_post(Engine* e, cudaStream_t s, int par, bool device_dt, bool host, bool joined = false) {
+  const bool early = capturing(s);  // every launch but a joined first follows a kernel of this graph
   Level& L0 = e->levels[0];
   const int mac = e->prm.scheme == FL_MACCORMACK;
   const double N = (double)e->cells(), F = (double)(e->ufaces() + e->vfaces()), D = (double)e->dye_cells();
@@ -524,25 +533,27 @@ cudaError_t enqueue_post(Engine* e, cudaStream_t s, int par, bool device_dt) {
   float* v = e->v[1 - par];
   int tok = prof_begin(*e, FL_PH_PROJECT);
   launch_subtract_outflow(s, e->nx, e->ny, L0.x[0], u, v, L0.label, e->sc, true, true, mixed ? e->p64[0] : nullptr,
-                          mixed ? e->p64[1] : nullptr, e->ctl, refined_df(e), mixed ? e->p32_final : nullptr);
+                          mixed ? e->p64[1] : nullptr, e->ctl, refined_df(e), mixed ? e->p32_final : nullptr, early && !joined);
   prof_end(*e, tok, (mixed ? 8 + 4 : 4) * N + 4 * F + N + 4 * F, 1);
   // velocity and pressure are final: fl_step_host reads them back from here
   // on while the dye advection runs
-  cudaEventRecordWithFlags(e->ev_proj, s, capturing(s) ? cudaEventRecordExternal : 0);
-  wait_dye(e, s);
+  if (host) {
+    cudaEventRecordWithFlags(e->ev_proj, s, capturing(s) ? cudaEventRecordExternal : 0);
+    wait_dye(e, s);
+  }
   tok = prof_begin(*e, FL_PH_ADVECT_DYE);
   launch_advect_dye(s, e->nx, e->ny, e->h, e->dnx, e->dny, e->dh, mac, u, v, e->dye[par], e->dye_hat, e->dye[1 - par],
-                    L0.label, e->sc, true, e->patch, e->pi0, e->pj0, e->pnx, e->pny);
+                    L0.label, e->sc, true, e->patch, e->pi0, e->pj0, e->pnx, e->pny, early && !host);
   // forward: u,v + 3 planes + label in, 3 planes out (MacCormack: + stencil
   // offsets out); correction adds the hat planes and the offsets
   prof_end(*e, tok, mac ? (4 * F + 28 * D + N) + (4 * F + 40 * D + N) : 4 * F + 24 * D + N, mac ? 2 : 1);
   // the dye is final: fl_step_host reads it back from here on
-  cudaEventRecordWithFlags(e->ev_dye_done, s, capturing(s) ? cudaEventRecordExternal : 0);
+  if (host) cudaEventRecordWithFlags(e->ev_dye_done, s, capturing(s) ? cudaEventRecordExternal : 0);
   tok = prof_begin(*e, FL_PH_CFL);
   if (e->prm.residual_every > 0) {
     // with the residual diagnostic (simulation.ts:539-540) on its cadence
     launch_cfl_residual(s, e->nx, e->ny, e->h, u, v, e->div_post, L0.label, e->prm.residual_every, e->diag, e->acc,
-                        e->sc, e->time_dev, &e->prm, device_dt, device_dt);
+                        e->sc, e->time_dev, &e->prm, device_dt, device_dt, early && !host);
     // u, v in; on diagnostic steps labels in and the divergence out
     prof_end(*e, tok, 4 * F + N + 4 * N, 1);
   } else {
@@ -624,7 +635,7 @@ int step_eager(Engine* e, bool device_dt) {
     e->labels_dirty = false;
   }
   if (e->pending.size() > 8192) prof_drain(*e);
-  enqueue_pre(e, s, par, e->stir_pending);
+  enqueue_pre(e, s, par, e->stir_pending, true);
   e->stir_pending = false;
   TRY(check_launch(e, "advect / forces / divergence"));
   e->stats_on_device = solve_on_device(e);
@@ -646,7 +657,7 @@ int step_eager(Engine* e, bool device_dt) {
       TRY(rb_solve_device(e, hs.scale, e->prm.pressure_iters, (float)e->prm.omega, e->prm.tol, div_rms, &iters));
     e->last_iters = iters;
   }
-  TRY(cuda_status(e, enqueue_post(e, s, par, device_dt), "project / dye / CFL"));
+  TRY(cuda_status(e, enqueue_post(e, s, par, device_dt, true), "project / dye / CFL"));
   TRY(check_launch(e, "project / dye / CFL"));
   e->cur = 1 - par;
   e->steps++;
@@ -659,6 +670,10 @@ void destroy_step_graphs(Engine* e) {
     g = nullptr;
   }
   for (auto& g : e->graph_up) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
+  for (auto& g : e->graph_host) {
     if (g) cudaGraphExecDestroy(g);
     g = nullptr;
   }
@@ -679,14 +694,14 @@ void destroy_graphs(Engine* e) {
 // body is captured from e->stream2.
 // cfl_first: led by the clock reset and the CFL scalars of the current
 // velocity (the work an upload otherwise enqueues after its copies).
-cudaError_t capture_step(Engine* e, int par, bool cfl_first) {
+cudaError_t capture_step(Engine* e, int par, bool cfl_first, bool host) {
   cudaStream_t s = e->stream;
   cudaError_t err = cudaSuccess;
   if (cfl_first) {
     launch_fill32(s, e->time_dev, 2, 0u);
     launch_max_speed(s, e->nx, e->ny, e->u[par], e->v[par], e->acc, e->sc, e->time_dev, &e->prm, e->h, true, false);
   }
-  enqueue_pre(e, s, par, false);
+  enqueue_pre(e, s, par, false, host);
   if (e->prm.solver == FL_SOLVER_MG) {
     cudaStreamCaptureStatus cst;
     cudaGraph_t cap = nullptr;
@@ -724,16 +739,16 @@ cudaError_t capture_step(Engine* e, int par, bool cfl_first) {
   } else {
     enqueue_rb_fixed(e, s);
   }
-  if (err == cudaSuccess) err = enqueue_post(e, s, par, true);
+  if (err == cudaSuccess) err = enqueue_post(e, s, par, true, host);
   return err;
 }
 
 // Captures the whole step for buffer parity `par` into an executable graph.
-int build_graph(Engine* e, int par, cudaGraphExec_t* out, bool cfl_first = false) {
+int build_graph(Engine* e, int par, cudaGraphExec_t* out, bool cfl_first, bool host) {
   cudaStream_t s = e->stream;
   cudaError_t err = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
   if (err != cudaSuccess) return cuda_status(e, err, "begin capture");
-  err = capture_step(e, par, cfl_first);
+  err = capture_step(e, par, cfl_first, host);
   cudaGraph_t graph = nullptr;
   cudaError_t end = cudaStreamEndCapture(s, &graph);
   if (err == cudaSuccess) err = end;
@@ -753,14 +768,15 @@ bool graph_eligible(const Engine* e) {
 
 // cfl_first: the step right after fl_step_host's upload, which left the
 // clock reset and the CFL scalars to the step's graph.
-int step_graph(Engine* e, bool cfl_first = false) {
+// host: fl_step_host's step (built on first use).
+int step_graph(Engine* e, bool cfl_first = false, bool host = false) {
   if (!e->graphs_valid) {
     destroy_step_graphs(e);
-    for (int par = 0; par < 2; par++) TRY(build_graph(e, par, &e->graph[par]));
+    for (int par = 0; par < 2; par++) TRY(build_graph(e, par, &e->graph[par], false, false));
     e->graphs_valid = true;
   }
-  cudaGraphExec_t& g = cfl_first ? e->graph_up[e->cur] : e->graph[e->cur];
-  if (!g) TRY(build_graph(e, e->cur, &g, true));
+  cudaGraphExec_t& g = cfl_first ? e->graph_up[e->cur] : host ? e->graph_host[e->cur] : e->graph[e->cur];
+  if (!g) TRY(build_graph(e, e->cur, &g, cfl_first, host));
   TRY(cuda_status(e, cudaGraphLaunch(g, e->stream), "graph launch"));
   e->cur = 1 - e->cur;
   e->steps++;
@@ -1271,7 +1287,7 @@ int fl_step_host(fl_engine* h, int dtype, const void* u, const void* v, const vo
     TRY(cuda_status(e, cudaEventRecord(e->ev_dye, e->stream2), "step"));
   }
   if (graph_eligible(e)) {
-    TRY(step_graph(e, cfl_first));
+    TRY(step_graph(e, cfl_first, true));
   } else {
     if (cfl_first) {
       launch_fill32(e->stream, e->time_dev, 2, 0u);
@@ -1853,7 +1869,7 @@ int batch_capture(fl_batch* b, int flip, cudaGraphExec_t* out) {
   for (int k : b->order) {
     Engine* e = &b->engines[k]->e;
     cudaStreamWaitEvent(e->stream, b->start, 0);
-    enqueue_pre(e, e->stream, e->cur ^ flip, false);
+    enqueue_pre(e, e->stream, e->cur ^ flip, false, false);
     cudaEventRecord(b->events[k], e->stream);
     cudaStreamWaitEvent(s, b->events[k], 0);
   }
@@ -1862,7 +1878,7 @@ int batch_capture(fl_batch* b, int flip, cudaGraphExec_t* out) {
   for (int k : b->order) {
     Engine* e = &b->engines[k]->e;
     cudaStreamWaitEvent(e->stream, b->mid, 0);
-    const cudaError_t pe = enqueue_post(e, e->stream, e->cur ^ flip, true);
+    const cudaError_t pe = enqueue_post(e, e->stream, e->cur ^ flip, true, false, true);
     if (err == cudaSuccess) err = pe;
     cudaEventRecord(b->joins[k], e->stream);
     cudaStreamWaitEvent(s, b->joins[k], 0);

@@ -83,6 +83,9 @@ struct Engine {
   // kernel launches and a graph launch while the dye is still arriving,
   // which delays separately launched kernels (built on first use)
   cudaGraphExec_t graph_up[2] = {nullptr, nullptr};
+  // fl_step_host's steps without an upload (built on first use): graph, with
+  // the events at which the results are read back
+  cudaGraphExec_t graph_host[2] = {nullptr, nullptr};
   // the device-side work of fl_upload_fields after its copies (float32 p)
   cudaGraphExec_t upload_graph = nullptr;
   // fl_step_host's pressure arrives on the second stream (ev_p marks it and
@@ -186,7 +189,9 @@ void set_global_error(const char* fmt, ...);
 // (dep_wait, fl_common.cuh): only where that is a kernel, in the stream or the
 // captured graph, and only for kernels that call dep_wait. early = false: an
 // ordinary launch. Measured, V-cycles in a graph: 256^2 24.7 -> 20.5 us,
-// 1024^2 45.5 -> 40.9, 2048^2 82 -> 74.
+// 1024^2 45.5 -> 40.9, 2048^2 82 -> 74; the step's other kernels (which wait at
+// once), with graphs free of event nodes, 8 steps: Karman 128^2 1370 -> 1197,
+// plume 256^2 3742 -> 3528, 1024^2 3976 -> 3876.
 template <class... P, class... A>
 inline cudaError_t launch_dependent(bool early, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s,
                                     const A&... args) {
@@ -204,13 +209,16 @@ inline cudaError_t launch_dependent(bool early, void (*kernel)(P...), dim3 grid,
 
 // ------------------------------------------------------------- launchers
 
+// early (here and below): launch_dependent's
+
 // fl_advect.cu
 void launch_advect_velocity(cudaStream_t s, int nx, int ny, float h, int mac, const float* u_in, const float* v_in,
                             float* u_hat, float* v_hat, float* u_out, float* v_out, const uint8_t* label,
                             const StepScalars* sc);
 void launch_advect_dye(cudaStream_t s, int nx, int ny, float h, int dnx, int dny, float dh, int mac, const float* u,
                        const float* v, const float* q_in, float* q_hat, float* q_out, const uint8_t* label,
-                       const StepScalars* sc, bool tail, const float* patch, int pi0, int pj0, int pnx, int pny);
+                       const StepScalars* sc, bool tail, const float* patch, int pi0, int pj0, int pnx, int pny,
+                       bool early = false);
 // Loads the velocity-advection kernels (so that later launches need no module load).
 cudaError_t preload_advect_kernels();
 
@@ -218,16 +226,16 @@ cudaError_t preload_advect_kernels();
 void launch_vorticity(cudaStream_t s, int nx, int ny, float h, const float* u, const float* v, float* w);
 // vorticity + confinement force in one pass (the same values as the two launches)
 void launch_vort_confine(cudaStream_t s, int nx, int ny, float h, const float* u, const float* v,
-                         const uint8_t* label, float eps, float* fx, float* fy);
+                         const uint8_t* label, float eps, float* fx, float* fy, bool early = false);
 void launch_confinement_force(cudaStream_t s, int nx, int ny, float h, const float* w, const uint8_t* label,
                               float eps, float* fx, float* fy);
 void launch_forces(cudaStream_t s, int nx, int ny, float h, int dnx, int dny, float dh, float* u, float* v,
                    const float* dye, const uint8_t* label, bool beta_on, bool alpha_on, bool conf_on,
-                   const float* fx, const float* fy, const StepScalars* sc);
+                   const float* fx, const float* fy, const StepScalars* sc, bool early = false);
 // out_lo (optional): the exact rounding error of each b = (-scale) * div (b + out_lo is the product)
 void launch_divergence(cudaStream_t s, int nx, int ny, float h, const float* u, const float* v, float* out,
                        bool as_rhs, const uint8_t* label, const StepScalars* sc, StepAccum* acc,
-                       float* out_lo = nullptr);
+                       float* out_lo = nullptr, bool early = false);
 // The batched pressure solve of fl_batch (fl_multigrid.cu): the plan over
 // the engines' buffers, or null with the reason when some engine does not
 // qualify; the solve enqueued on a capturing stream (cycle body captured
@@ -238,19 +246,21 @@ void batch_solve_destroy(BatchSolve* b);
 cudaError_t batch_solve_enqueue(const BatchSolve& b, cudaStream_t s, cudaStream_t body);
 
 // Word fills and copies as kernels (not copy-engine nodes) in the graphs.
-void launch_fill32(cudaStream_t s, void* p, long words, uint32_t v);
+void launch_fill32(cudaStream_t s, void* p, long words, uint32_t v, bool early = false);
 void launch_copy32(cudaStream_t s, const void* src, void* dst, long words);
 // The end-of-step CFL scan with the residual diagnostic folded in (every
 // residual_every steps: the post-step divergence and its statistics); the
 // step's dt joins the clock and the next step's scalars are written.
 void launch_cfl_residual(cudaStream_t s, int nx, int ny, float h, const float* u, const float* v, float* div_out,
                          const uint8_t* label, int every, DiagAccum* d, StepAccum* acc, StepScalars* sc_next,
-                         double* time_dev, const fl_params* prm, bool write_scalars, bool add_time);
+                         double* time_dev, const fl_params* prm, bool write_scalars, bool add_time,
+                         bool early = false);
 // p64a/p64b: the refined pressure (float64, or double-float pairs when df)
 void launch_subtract_outflow(cudaStream_t s, int nx, int ny, const float* p, float* u, float* v,
                              const uint8_t* label, const StepScalars* sc, bool subtract, bool outflow,
                              const double* p64a = nullptr, const double* p64b = nullptr,
-                             const SolveCtl* ctl = nullptr, bool df = false, float* p32_out = nullptr);
+                             const SolveCtl* ctl = nullptr, bool df = false, float* p32_out = nullptr,
+                             bool early = false);
 void launch_max_speed(cudaStream_t s, int nx, int ny, const float* u, const float* v, StepAccum* acc,
                       StepScalars* sc_next, double* time_dev, const fl_params* prm, float h, bool write_scalars,
                       bool add_time);

@@ -1291,6 +1291,7 @@ __global__ void k_solve_check(StepAccum* acc, SolveCtl* ctl, int use_cond, cudaG
 // or the current float64 buffer).
 __global__ void k_zero_if(const SolveCtl* __restrict__ ctl, float* __restrict__ p32, double* __restrict__ p64a,
                           double* __restrict__ p64b, long n) {
+  dep_trigger();  // an ordinary launch: what precedes it is complete
   if (!ctl->zero_p) return;
   double* p64 = p64a ? (ctl->par ? p64b : p64a) : nullptr;
   for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {

@@ -62,9 +62,11 @@ __global__ void k_confinement_force(int nx, int ny, Spacing h1, Spacing h2, cons
 // force of its own cells from it. u and v are only read here; the forces
 // are applied by k_forces afterwards.
 __global__ void __launch_bounds__(256) k_vort_confine(int nx, int ny, Spacing h, Spacing h1, Spacing h2,
-                                                      const float* __restrict__ u, const float* __restrict__ v,
+                                                      const float* u, const float* v,
                                                       const uint8_t* __restrict__ label, float epsh,
                                                       float* __restrict__ fx, float* __restrict__ fy) {
+  dep_wait();
+  dep_trigger();
   constexpr int TX = 32, TY = 8;
   __shared__ float ws[TY + 2][TX + 2];
   const int X0 = blockIdx.x * TX, Y0 = blockIdx.y * TY;
@@ -108,11 +110,13 @@ __global__ void __launch_bounds__(256) k_vort_confine(int nx, int ny, Spacing h,
 // confinement face average. One thread per (u face, v face) pair, in place:
 // every write depends only on the thread's own face.
 __global__ void __launch_bounds__(256) k_forces(int nx, int ny, float h, int dnx, int dny, Spacing dh,
-                                                float* __restrict__ u, float* __restrict__ v,
+                                                float* u, float* v,
                                                 const float* __restrict__ dye, const uint8_t* __restrict__ label,
                                                 int beta_on, int alpha_on, int conf_on,
-                                                const float* __restrict__ fx, const float* __restrict__ fy,
+                                                const float* fx, const float* fy,
                                                 const StepScalars* __restrict__ sc) {
+  dep_wait();
+  dep_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   if (conf_on && i >= 1 && i < nx && j < ny) {
@@ -139,11 +143,13 @@ __global__ void __launch_bounds__(256) k_forces(int nx, int ny, float h, int dnx
 // divergence.ts:17-25. as_rhs: write b = (-scale)*div (pressureMultigrid.ts:
 // 311) instead of div. Also accumulates the sum of squares of what it writes
 // and the count over FLUID cells (pressure.ts:177-186's fluidDivRms).
-__global__ void __launch_bounds__(256) k_divergence(int nx, int ny, float h, const float* __restrict__ u,
-                                                    const float* __restrict__ v, float* __restrict__ out, int as_rhs,
+__global__ void __launch_bounds__(256) k_divergence(int nx, int ny, float h, const float* u,
+                                                    const float* v, float* __restrict__ out, int as_rhs,
                                                     const uint8_t* __restrict__ label,
                                                     const StepScalars* __restrict__ sc, StepAccum* acc,
                                                     float* __restrict__ out_lo) {
+  dep_wait();
+  dep_trigger();
   __shared__ double red[32];
   __shared__ unsigned long long redn[32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -222,13 +228,15 @@ __device__ __forceinline__ float projected_v(const float* __restrict__ p, const 
   return val;
 }
 
-__global__ void __launch_bounds__(256) k_subtract_outflow(int nx, int ny, const float* __restrict__ p,
-                                                          const double* __restrict__ p64a,
-                                                          const double* __restrict__ p64b,
-                                                          const SolveCtl* __restrict__ ctl, float* __restrict__ u,
-                                                          float* __restrict__ v, const uint8_t* __restrict__ label,
+__global__ void __launch_bounds__(256) k_subtract_outflow(int nx, int ny, const float* p,
+                                                          const double* p64a,
+                                                          const double* p64b,
+                                                          const SolveCtl* ctl, float* u,
+                                                          float* v, const uint8_t* __restrict__ label,
                                                           const StepScalars* __restrict__ sc, int subtract,
                                                           int outflow, int df, float* __restrict__ p32_out) {
+  dep_wait();
+  dep_trigger();
   // the float64 pressure, when there is one, is the buffer ctl->par names
   const double* p64 = p64a ? (ctl->par ? p64b : p64a) : nullptr;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -479,37 +487,38 @@ void launch_confinement_force(cudaStream_t s, int nx, int ny, float h, const flo
 }
 
 void launch_vort_confine(cudaStream_t s, int nx, int ny, float h, const float* u, const float* v,
-                         const uint8_t* label, float eps, float* fx, float* fy) {
+                         const uint8_t* label, float eps, float* fx, float* fy, bool early) {
   dim3 b(32, 8);
-  k_vort_confine<<<grid2(nx, ny, b), b, 0, s>>>(nx, ny, make_spacing(h), make_spacing(1.0f * h),
-                                                make_spacing(2.0f * h), u, v, label, eps * h, fx, fy);
+  launch_dependent(early, k_vort_confine, grid2(nx, ny, b), b, s, nx, ny, make_spacing(h), make_spacing(1.0f * h),
+                   make_spacing(2.0f * h), u, v, label, eps * h, fx, fy);
 }
 
 void launch_forces(cudaStream_t s, int nx, int ny, float h, int dnx, int dny, float dh, float* u, float* v,
                    const float* dye, const uint8_t* label, bool beta_on, bool alpha_on, bool conf_on,
-                   const float* fx, const float* fy, const StepScalars* sc) {
+                   const float* fx, const float* fy, const StepScalars* sc, bool early) {
   dim3 b(32, 8);
-  k_forces<<<grid2(nx + 1, ny + 1, b), b, 0, s>>>(nx, ny, h, dnx, dny, make_spacing(dh), u, v, dye, label, beta_on, alpha_on,
-                                                  conf_on, fx, fy, sc);
+  launch_dependent(early, k_forces, grid2(nx + 1, ny + 1, b), b, s, nx, ny, h, dnx, dny, make_spacing(dh), u, v, dye, label,
+                   beta_on, alpha_on, conf_on, fx, fy, sc);
 }
 
 void launch_divergence(cudaStream_t s, int nx, int ny, float h, const float* u, const float* v, float* out,
-                       bool as_rhs, const uint8_t* label, const StepScalars* sc, StepAccum* acc, float* out_lo) {
+                       bool as_rhs, const uint8_t* label, const StepScalars* sc, StepAccum* acc, float* out_lo,
+                       bool early) {
   dim3 b(32, 8);
   dim3 g = grid2(nx, ny, b);
   // about four blocks per SM, rows strided: every block ends in same-word
   // atomics, which serialise
   g.y = std::min(g.y, std::max(1u, 608u / g.x));
-  k_divergence<<<g, b, 0, s>>>(nx, ny, h, u, v, out, as_rhs, label, sc, acc, out_lo);
+  launch_dependent(early, k_divergence, g, b, s, nx, ny, h, u, v, out, as_rhs, label, sc, acc, out_lo);
 }
 
 void launch_subtract_outflow(cudaStream_t s, int nx, int ny, const float* p, float* u, float* v,
                              const uint8_t* label, const StepScalars* sc, bool subtract, bool outflow,
                              const double* p64a, const double* p64b, const SolveCtl* ctl, bool df,
-                             float* p32_out) {
+                             float* p32_out, bool early) {
   dim3 b(32, 8);
-  k_subtract_outflow<<<grid2(nx + 1, ny + 1, b), b, 0, s>>>(nx, ny, p, p64a, p64b, ctl, u, v, label, sc, subtract,
-                                                            outflow, df, p32_out);
+  launch_dependent(early, k_subtract_outflow, grid2(nx + 1, ny + 1, b), b, s, nx, ny, p, p64a, p64b, ctl, u, v, label, sc,
+                   subtract, outflow, df, p32_out);
 }
 
 void launch_scale_rhs(cudaStream_t s, long n, const float* div, float* b, float neg_scale, const uint8_t* label,
@@ -529,13 +538,15 @@ void launch_scale_rhs(cudaStream_t s, long n, const float* div, float* b, float 
 // sums its square and max over FLUID cells (viz/fieldView.ts:44-60). The
 // last block finishes the CFL scalars, publishes the diagnostic's sums and
 // counts the step.
-__global__ void __launch_bounds__(256) k_cfl_residual(int nx, int ny, float h, const float* __restrict__ u,
-                                                      const float* __restrict__ v, float* __restrict__ div_out,
+__global__ void __launch_bounds__(256) k_cfl_residual(int nx, int ny, float h, const float* u,
+                                                      const float* v, float* __restrict__ div_out,
                                                       const uint8_t* __restrict__ label, int every, DiagAccum* d,
                                                       StepAccum* acc, StepScalars* sc_next, double* time_dev,
                                                       float cfl, float dt_max, float rho, double d0, double d1,
                                                       double d2, float beta, float alpha, int write_scalars,
                                                       int add_time) {
+  dep_wait();
+  dep_trigger();
   __shared__ double red[32];
   __shared__ unsigned long long redn[32];
   __shared__ float redm[32];
@@ -613,23 +624,24 @@ __global__ void __launch_bounds__(256) k_cfl_residual(int nx, int ny, float h, c
 
 void launch_cfl_residual(cudaStream_t s, int nx, int ny, float h, const float* u, const float* v, float* div_out,
                          const uint8_t* label, int every, DiagAccum* d, StepAccum* acc, StepScalars* sc_next,
-                         double* time_dev, const fl_params* prm, bool write_scalars, bool add_time) {
+                         double* time_dev, const fl_params* prm, bool write_scalars, bool add_time, bool early) {
   dim3 b(32, 8);
   dim3 g = grid2(nx, ny, b);
   // about four blocks per SM, rows strided: every block ends in same-word
   // atomics, which serialise
   g.y = std::min(g.y, std::max(1u, 608u / g.x));
-  k_cfl_residual<<<g, b, 0, s>>>(nx, ny, h, u, v, div_out, label, every, d, acc, sc_next, time_dev,
-                                 (float)prm->cfl_target, (float)prm->dt_max, (float)prm->rho, prm->dye_decay[0],
-                                 prm->dye_decay[1], prm->dye_decay[2], (float)prm->beta, (float)prm->alpha,
-                                 write_scalars, add_time);
+  launch_dependent(early, k_cfl_residual, g, b, s, nx, ny, h, u, v, div_out, label, every, d, acc, sc_next, time_dev,
+                   (float)prm->cfl_target, (float)prm->dt_max, (float)prm->rho, prm->dye_decay[0], prm->dye_decay[1],
+                   prm->dye_decay[2], (float)prm->beta, (float)prm->alpha, write_scalars, add_time);
 }
 
 // Fills and device-to-device copies inside the step and upload graphs run as
 // kernels: as memset or memcpy nodes they would queue on the copy engine
 // behind the host transfers of fl_step_host (measured: the upload graph took
 // 64 us behind the dye upload, 43 us without it).
-__global__ void __launch_bounds__(256) k_fill32(uint32_t* __restrict__ p, long n, uint32_t v) {
+__global__ void __launch_bounds__(256) k_fill32(uint32_t* p, long n, uint32_t v) {
+  dep_wait();
+  dep_trigger();
   for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) p[k] = v;
 }
 
@@ -637,9 +649,9 @@ __global__ void __launch_bounds__(256) k_copy32(const uint32_t* __restrict__ src
   for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) dst[k] = src[k];
 }
 
-void launch_fill32(cudaStream_t s, void* p, long words, uint32_t v) {
+void launch_fill32(cudaStream_t s, void* p, long words, uint32_t v, bool early) {
   const long blocks = std::max(1L, std::min((words + 255) / 256, 152L * 8));
-  k_fill32<<<(unsigned)blocks, 256, 0, s>>>(static_cast<uint32_t*>(p), words, v);
+  launch_dependent(early, k_fill32, dim3((unsigned)blocks), dim3(256), s, static_cast<uint32_t*>(p), words, v);
 }
 
 void launch_copy32(cudaStream_t s, const void* src, void* dst, long words) {
