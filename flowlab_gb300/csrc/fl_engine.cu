@@ -291,11 +291,11 @@ int down32(Engine* e, void* dst, const void* src, size_t bytes, const char* what
 int zero_solve_accum(Engine* e) {
   return cuda_status(e, cudaMemsetAsync(e->acc, 0, 4 * sizeof(double), e->stream), "accumulators");
 }
+// res_sq and n_res, in one operation (two rows of 8 bytes)
 int zero_residual_accum(Engine* e) {
-  StepAccum* a = e->acc;
-  cudaError_t err = cudaMemsetAsync(&a->res_sq, 0, sizeof(double), e->stream);
-  if (err == cudaSuccess) err = cudaMemsetAsync(&a->n_res, 0, sizeof(unsigned long long), e->stream);
-  return cuda_status(e, err, "residual accumulators");
+  constexpr size_t a = offsetof(StepAccum, res_sq), b = offsetof(StepAccum, n_res);
+  static_assert(b > a + 8, "rows apart");
+  return cuda_status(e, cudaMemset2DAsync((char*)e->acc + a, b - a, 0, 8, 2, e->stream), "residual accumulators");
 }
 int read_accum(Engine* e) {
   TRY(cuda_status(e, cudaMemcpyAsync(e->acc_host, e->acc, sizeof(StepAccum), cudaMemcpyDeviceToHost, e->stream), "read accumulators"));
@@ -307,15 +307,37 @@ double rms(double sq, unsigned long long n) { return n > 0 ? std::sqrt(sq / (dou
 // fluidDivRms of a host array (pressure.ts:177-186), used where the reference
 // evaluates it on the host before the device solve (pressureGpu.ts:228,
 // multigridGpu.ts:323).
+// Eight running sums where eight labels in a row are FLUID: one sum alone is a
+// chain of n dependent additions (640x480 on one Grace core: 189 -> 129 us).
 double host_fluid_div_rms(const float* div, const uint8_t* label, long n) {
-  double s = 0;
-  long c = 0;
-  for (long k = 0; k < n; k++) {
-    if (label[k] != FLUID) continue;
-    s += (double)div[k] * (double)div[k];
+  static_assert(FLUID == 0, "eight FLUID labels are a zero word");
+  double part[8] = {};
+  long c = 0, k = 0;
+  auto add = [&](int q) {
+    part[q] += (double)div[k + q] * (double)div[k + q];
     c++;
+  };
+  for (; k + 8 <= n; k += 8) {
+    uint64_t eight;
+    std::memcpy(&eight, label + k, 8);
+    if (eight == 0)
+      for (int q = 0; q < 8; q++) add(q);
+    else
+      for (int q = 0; q < 8; q++)
+        if (label[k + q] == FLUID) add(q);
   }
+  for (; k < n; k++)
+    if (label[k] == FLUID) add(0);
+  double s = 0;
+  for (double x : part) s += x;
   return c > 0 ? std::sqrt(s / (double)c) : 0.0;
+}
+
+// host_fluid_div_rms == 0 (a square of a float never underflows in double)
+bool host_fluid_div_zero(const float* div, const uint8_t* label, long n) {
+  for (long k = 0; k < n; k++)
+    if (label[k] == FLUID && div[k] != 0.0f) return false;
+  return true;
 }
 
 // ------------------------------------------------------------ the step
@@ -565,37 +587,49 @@ cudaError_t enqueue_post(Engine* e, cudaStream_t s, int par, bool device_dt, boo
 
 // Red-black SOR to a tolerance (pressureRedBlack.ts:88-113): checked every
 // 12 sweeps on the host, pairs grouped up to four per launch and never
-// across a check.
-int rb_solve_device(Engine* e, float scale, int iterations, float omega, double tol, double div_rms, int* used) {
+// across a check. host_div: div_rms is not known yet, and is summed from this
+// while the first sweeps run.
+int rb_solve_device(Engine* e, float scale, int iterations, float omega, double tol, double div_rms, int* used,
+                    const float* host_div = nullptr, const uint8_t* host_label = nullptr) {
   Level& L = e->levels[0];
   *used = iterations;
-  const double target = tol > 0 ? tol * div_rms : -1;
+  bool checks = tol > 0 && (host_div != nullptr || tol * div_rms >= 0);
+  auto rms_of_host = [&] {
+    if (host_div != nullptr) e->last_div_rms = div_rms = host_fluid_div_rms(host_div, host_label, e->cells());
+    host_div = nullptr;
+  };
   int k = 0;
   int src = 0;
   const int per = e->prm.rb_pairs > 0 ? e->prm.rb_pairs : 4;
   while (k < iterations) {
     int chunk = std::min(per, iterations - k);
-    if (target >= 0) chunk = std::min(chunk, 12 - (k % 12));
+    if (checks) chunk = std::min(chunk, 12 - (k % 12));
     const int tok = prof_begin(*e, FL_PH_RB_SWEEPS);
     launch_rb_sweeps(e->stream, L.nx, L.ny, L.x[src], L.x[1 - src], L.b, L.code, scale, omega, chunk, nullptr,
-                     k > 0 && !(target >= 0 && k % 12 == 0));
+                     k > 0 && !(checks && k % 12 == 0));
     prof_end(*e, tok, 13.0 * e->cells(), 1);
     TRY(check_launch(e, "red-black sweeps"));
     src = 1 - src;
     k += chunk;
-    if (target >= 0 && k % 12 == 0) {
+    if (checks && k % 12 == 0) {
+      rms_of_host();
+      if (!(tol * div_rms >= 0)) {  // NaN: no check ever passes
+        checks = false;
+        continue;
+      }
       TRY(zero_residual_accum(e));
       launch_rms_remaining(e->stream, L.nx, L.ny, L.x[src], L.b, L.code, scale, e->acc);
       TRY(check_launch(e, "residual"));
       TRY(read_accum(e));
       const double r = rms(e->acc_host->res_sq, e->acc_host->n_res);
       e->last_relres = div_rms > 0 ? r / div_rms : 0;
-      if (r <= target) {
+      if (r <= tol * div_rms) {
         *used = k;
         break;
       }
     }
   }
+  rms_of_host();
   if (src == 1)
     TRY(cuda_status(e, cudaMemcpyAsync(L.x[0], L.x[1], e->cells() * sizeof(float), cudaMemcpyDeviceToDevice, e->stream),
                     "p copy"));
@@ -1547,13 +1581,13 @@ int fl_rb_solve(fl_engine* h, float* p, const float* div, const uint8_t* label, 
   if (!p || !div || !label) return fail(e, FL_EINVAL, "null pointer");
   const long n = e->cells();
   // pressureRedBlack.ts:335-339 — zero divergence: p = 0, no sweeps.
-  const double div_rms = host_fluid_div_rms(div, label, n);
+  const bool zero = host_fluid_div_zero(div, label, n);
   e->stats_on_device = false;
-  e->last_div_rms = div_rms;
-  e->last_relres = div_rms == 0 ? 0.0 : -1.0;
+  e->last_div_rms = zero || iterations > 0 ? 0.0 : host_fluid_div_rms(div, label, n);
+  e->last_relres = zero ? 0.0 : -1.0;
   e->last_iters = 0;
   if (used) *used = 0;
-  if (div_rms == 0) {
+  if (zero) {
     std::memset(p, 0, n * sizeof(float));
     return FL_OK;
   }
@@ -1565,7 +1599,7 @@ int fl_rb_solve(fl_engine* h, float* p, const float* div, const uint8_t* label, 
   launch_build_codes(e->stream, L.nx, L.ny, L.label, L.code);
   e->codes_valid = false;
   int u = 0;
-  TRY(rb_solve_device(e, scale, iterations, omega, tol, div_rms, &u));
+  TRY(rb_solve_device(e, scale, iterations, omega, tol, 0.0, &u, div, label));
   e->last_iters = u;
   if (used) *used = u;
   TRY(down32(e, p, L.x[0], n * 4, "p"));
