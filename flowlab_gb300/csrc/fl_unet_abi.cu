@@ -174,8 +174,11 @@ int fl_unet_train_step(fl_unet* h, int B, int H, int W, const float* x, const fl
   Unet& u = h->u;
   cudaStream_t s = u.stream;
   const long P = (long)B * H * W;
-  double nmask = 0;
-  for (long k = 0; k < P; k++) nmask += mask[k];
+  // eight running sums: one alone is a chain of P additions (exact for 0 / 1 masks either way)
+  double part[8] = {};
+  for (long k = 0; k + 8 <= P; k += 8)  // P is a multiple of 64
+    for (int q = 0; q < 8; q++) part[q] += mask[k + q];
+  const double nmask = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
   if (!(nmask > 0)) return ufail(h, FL_EINVAL, "empty mask");
   UTRY(ucuda(h, cudaMemcpyAsync(u.input, x, P * 3 * 4, cudaMemcpyHostToDevice, s), "input"));
   UTRY(ucuda(h, cudaMemcpyAsync(u.target, target, P * 4, cudaMemcpyHostToDevice, s), "target"));
