@@ -522,14 +522,14 @@ void enqueue_solve_epilogue(Engine* e, cudaStream_t s, bool mixed) {
 }
 
 // Red-black SOR with a fixed budget (tol <= 0, the reference's browser
-// setting): sweep pairs grouped up to four per launch, scale read from the
+// setting): sweep pairs grouped by rb_launch_pairs, scale read from the
 // step's scalars on the device, result back in levels[0].x[0].
 void enqueue_rb_fixed(Engine* e, cudaStream_t s) {
   Level& L = e->levels[0];
   launch_solve_begin(s, e->acc, e->ctl, false, 0);
   int k = 0, src = 0;
   const int iters = e->prm.pressure_iters;
-  const int per = e->prm.rb_pairs > 0 ? e->prm.rb_pairs : 4;
+  const int per = e->prm.rb_pairs > 0 ? e->prm.rb_pairs : rb_launch_pairs(L.nx, L.ny, iters);
   while (k < iters) {
     const int chunk = std::min(per, iters - k);
     const int tok = prof_begin(*e, FL_PH_RB_SWEEPS);
@@ -586,7 +586,7 @@ cudaError_t enqueue_post(Engine* e, cudaStream_t s, int par, bool device_dt, boo
 }
 
 // Red-black SOR to a tolerance (pressureRedBlack.ts:88-113): checked every
-// 12 sweeps on the host, pairs grouped up to four per launch and never
+// 12 sweeps on the host, pairs grouped by rb_launch_pairs and never
 // across a check. host_div: div_rms is not known yet, and is summed from this
 // while the first sweeps run.
 int rb_solve_device(Engine* e, float scale, int iterations, float omega, double tol, double div_rms, int* used,
@@ -600,7 +600,8 @@ int rb_solve_device(Engine* e, float scale, int iterations, float omega, double 
   };
   int k = 0;
   int src = 0;
-  const int per = e->prm.rb_pairs > 0 ? e->prm.rb_pairs : 4;
+  const int per = e->prm.rb_pairs > 0 ? e->prm.rb_pairs
+                                      : rb_launch_pairs(L.nx, L.ny, checks ? std::min(12, iterations) : iterations);
   while (k < iterations) {
     int chunk = std::min(per, iterations - k);
     if (checks) chunk = std::min(chunk, 12 - (k % 12));

@@ -190,8 +190,8 @@ void set_global_error(const char* fmt, ...);
 // captured graph, and only for kernels that call dep_wait. early = false: an
 // ordinary launch. Measured, V-cycles in a graph: 256^2 24.7 -> 20.5 us,
 // 1024^2 45.5 -> 40.9, 2048^2 82 -> 74; the step's other kernels (which wait at
-// once), with graphs free of event nodes, 8 steps: Karman 128^2 1370 -> 1197,
-// plume 256^2 3742 -> 3528, 1024^2 3976 -> 3876.
+// once), with graphs free of event nodes: 16 Karman 128^2 steps 1370 -> 1197, 16
+// plume 256^2 steps 3742 -> 3528, 8 at 1024^2 3976 -> 3876.
 template <class... P, class... A>
 inline cudaError_t launch_dependent(bool early, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s,
                                     const A&... args) {
@@ -300,9 +300,12 @@ void launch_update_resid64(cudaStream_t s, int nx, int ny, double* p64a, double*
 void launch_solve_begin(cudaStream_t s, StepAccum* acc, SolveCtl* ctl, bool use_cond, cudaGraphConditionalHandle h);
 void launch_solve_check(cudaStream_t s, StepAccum* acc, SolveCtl* ctl, bool use_cond, cudaGraphConditionalHandle h);
 void launch_zero_if(cudaStream_t s, const SolveCtl* ctl, float* p32, double* p64a, double* p64b, long n);
-// early: the kernel before it on the stream is another of these launches
+// early: the kernel before it on the stream is another of these launches of
+// the same row (b, code and *scale_dev as they were)
 void launch_rb_sweeps(cudaStream_t s, int nx, int ny, const float* x_in, float* x_out, const float* b,
                       const uint8_t* code, float scale, float omega, int pairs, const float* scale_dev, bool early);
+// Sweep pairs a launch for `span` of them in a row (at most 10).
+int rb_launch_pairs(int nx, int ny, int span);
 void launch_rms_remaining(cudaStream_t s, int nx, int ny, const float* p, const float* div, const uint8_t* code,
                           float scale, StepAccum* acc);
 void launch_build_codes(cudaStream_t s, int nx, int ny, const uint8_t* label, uint8_t* code);

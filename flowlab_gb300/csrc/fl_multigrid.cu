@@ -20,6 +20,7 @@
 //   * Labels become one byte per cell of stencil links (fl_common.cuh), built
 //     per level when labels change (pressureMultigrid.ts:302-310 rebuilt them
 //     every solve; stepGpu.ts:498 only on change, as here).
+#include <cfloat>
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -226,39 +227,42 @@ __device__ __forceinline__ void smooth_tile(const SmoothArgs& a, int bx, int by,
           cd[r] = (cd[r] & (o ? 0x00ffu : 0xff00u)) | (unsigned)a.code[k + o] << (8 * o);
     }
   };
-  auto load_values = [&](int r) {
-    const int gj = row + r, k = col + gj * nx;
-    x[r][0] = x[r][1] = b[r][0] = b[r][1] = 0.0f;
+  auto load_row = [&](const float* f, float* v, int gj) {
+    const int k = col + gj * nx;
+    v[0] = v[1] = 0.0f;
     if ((unsigned)gj >= (unsigned)ny) return;
     if (pair) {
       if ((unsigned)col < (unsigned)nx) {
-        const float2 q = *reinterpret_cast<const float2*>(a.b + k);
-        b[r][0] = q.x;
-        b[r][1] = q.y;
-        if (!a.x_is_zero) {
-          const float2 p = *reinterpret_cast<const float2*>(a.xin + k);
-          x[r][0] = p.x;
-          x[r][1] = p.y;
-        }
+        const float2 q = *reinterpret_cast<const float2*>(f + k);
+        v[0] = q.x;
+        v[1] = q.y;
       }
     } else {
 #pragma unroll
       for (int o = 0; o < 2; o++)
-        if ((unsigned)(col + o) < (unsigned)nx) {
-          b[r][o] = a.b[k + o];
-          if (!a.x_is_zero) x[r][o] = a.xin[k + o];
-        }
+        if ((unsigned)(col + o) < (unsigned)nx) v[o] = f[k + o];
     }
+  };
+  auto load_b = [&](int r) { load_row(a.b, b[r], row + r); };
+  auto load_x = [&](int r) {
+    x[r][0] = x[r][1] = 0.0f;
+    if (!a.x_is_zero) load_row(a.xin, x[r], row + r);
   };
   // Before dep_wait: the codes (built long before), and on the way up b and x,
   // which this level's PRE launch and the finer one's wrote; only the coarse
-  // correction comes from the launch before. On the way down b does.
+  // correction comes from the launch before. On the way down b does. Of a row
+  // of SOR launches (the first is an ordinary one) only x does.
 #pragma unroll
   for (int r = 0; r < RW; r++) load_codes(r);
+  if (MODE != MODE_PRE) {
+#pragma unroll
+    for (int r = 0; r < RW; r++) load_b(r);
+  }
   if (MODE == MODE_POST) {
 #pragma unroll
-    for (int r = 0; r < RW; r++) load_values(r);
+    for (int r = 0; r < RW; r++) load_x(r);
   }
+  const float scale = MODE == MODE_PLAIN && a.scale_dev ? *a.scale_dev : a.scale;
   if (tid < 64) sh.lut[tid] = link_factors(tid);
   if (w == 0) {
     sh.edge[0][0][1][lane] = sh.edge[1][0][1][lane] = 0.0f;
@@ -266,9 +270,13 @@ __device__ __forceinline__ void smooth_tile(const SmoothArgs& a, int bx, int by,
   }
   dep_wait();
   dep_trigger();
+  if (MODE == MODE_PRE) {
+#pragma unroll
+    for (int r = 0; r < RW; r++) load_b(r);
+  }
   if (MODE != MODE_POST) {
 #pragma unroll
-    for (int r = 0; r < RW; r++) load_values(r);
+    for (int r = 0; r < RW; r++) load_x(r);
   }
   if constexpr (MODE == MODE_POST) {
     // pressureMultigrid.ts:192-207 — a fluid cell's x += 9/16, 3/16, 3/16,
@@ -328,7 +336,6 @@ __device__ __forceinline__ void smooth_tile(const SmoothArgs& a, int bx, int by,
         x[r][o] = (c & 3u) == SOLID ? 0.0f : x[r][o];
       }
   }
-  const float scale = MODE == MODE_PLAIN && a.scale_dev ? *a.scale_dev : a.scale;
   if constexpr (MODE == MODE_PLAIN) {
 #pragma unroll
     for (int r = 0; r < RW; r++) {
@@ -1396,9 +1403,7 @@ static void launch_smooth_mode(cudaStream_t s, const SmoothArgs& a, bool early) 
 static void launch_smooth(cudaStream_t s, SmoothArgs a, int pairs, int mode, bool early) {
   a.pairs = pairs;
   a.halo = smooth_halo(mode, pairs, a.x_is_zero, a.acc != nullptr);
-  if (mode == MODE_PLAIN)
-    launch_smooth_mode<MODE_PLAIN>(s, a, early);
-  else if (mode == MODE_PRE)
+  if (mode == MODE_PRE)
     launch_smooth_mode<MODE_PRE>(s, a, early);
   else
     launch_smooth_mode<MODE_POST>(s, a, early);
@@ -1420,6 +1425,51 @@ void launch_rb_halfsweep(cudaStream_t s, int nx, int ny, float* p, const float* 
   k_rb_halfsweep<<<g, bl, 0, s>>>(nx, ny, p, b, code, scale, omega, color);
 }
 
+// A row of SOR launches: the pairs a launch and the region shape, by the
+// estimated time of the row. One region an SM costs its set-up, load and store
+// plus its pairs, two an SM the same and nearly twice the pairs (a launch of
+// p pairs with obstacles, measured: 16 warps of 2 rows, 128^2, 64 regions of 6
+// pairs 3.2 us, 24 of 4 2.7; 192^2 120 of 6 3.3; 384^2 192 of 4 3.5, 288 of 5
+// 4.0; 16 of 4, 320x240 140 of 10 6.3; 384^2 144 of 8 5.9; 517x389 130 of 6 5.3;
+// 640x480 140 of 4 4.2 (16 of 2: 5.3), 300 of 8 8.6; 800x600 221 of 4 5.6, 300 of
+// 6 7.2). So more pairs pay while their regions, which shrink with the halo, fit
+// the SMs; with more than two regions an SM it is 8 warps of 8 rows and 4 pairs
+// (1024^2 484 regions 8.7; 2048^2 4 pairs 22.3, 5 28.2, 3 17.1).
+// A span is what runs between two residual tests, in launches of equal length.
+struct RbShape {
+  int nw, rw;
+  float us;  // a launch
+};
+static RbShape rb_shape(int nx, int ny, int pairs) {
+  constexpr long SMS = 152;
+  const int tx = 64 - 4 * pairs;
+  auto regions = [&](int ty) { return (long)((nx + tx - 1) / tx) * ((ny + ty - 1) / ty); };
+  const long four = regions(tx);
+  RbShape best{8, 8, 0.018f * four};
+  if (four <= 2 * SMS) best = {16, 4, four <= SMS ? 2.6f + 0.4f * pairs : 2.8f + 0.73f * pairs};
+  if (pairs <= 6) {  // a region of 32 rows
+    const long two = regions(32 - 4 * pairs);
+    const float us = two <= SMS ? 1.6f + 0.28f * pairs : 1.7f + 0.48f * pairs;
+    if (two <= 2 * SMS && us < best.us) best = {16, 2, us};
+  }
+  return best;
+}
+
+int rb_launch_pairs(int nx, int ny, int span) {
+  int best = std::min(span, 4);
+  float time = FLT_MAX;
+  for (int p = std::min(span, 4); p <= 10 && p <= span; p++) {
+    const int launches = (span + p - 1) / p, q = (span + launches - 1) / launches;
+    const RbShape sh = rb_shape(nx, ny, q);
+    if (sh.rw == 8 && q > 4) continue;
+    if (launches * sh.us < time) {
+      time = launches * sh.us;
+      best = q;
+    }
+  }
+  return best;
+}
+
 void launch_rb_sweeps(cudaStream_t s, int nx, int ny, const float* x_in, float* x_out, const float* b,
                       const uint8_t* code, float scale, float omega, int pairs, const float* scale_dev, bool early) {
   SmoothArgs a{};
@@ -1432,7 +1482,15 @@ void launch_rb_sweeps(cudaStream_t s, int nx, int ny, const float* x_in, float* 
   a.code = code;
   a.scale = scale;
   a.omega = omega;
-  launch_smooth(s, a, pairs, MODE_PLAIN, early);
+  a.pairs = pairs;
+  a.halo = smooth_halo(MODE_PLAIN, pairs, false, false);
+  const RbShape sh = rb_shape(nx, ny, pairs);
+  if (sh.rw == 2)
+    launch_smooth_nw<MODE_PLAIN, 16, 2>(s, a, early);
+  else if (sh.rw == 4)
+    launch_smooth_nw<MODE_PLAIN, 16, 4>(s, a, early);
+  else
+    launch_smooth_nw<MODE_PLAIN, 8, 8>(s, a, early);
 }
 
 template <bool UPDATE, int RW>

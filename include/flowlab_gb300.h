@@ -89,7 +89,7 @@ typedef struct fl_params {
   int mixed;             /* defect correction around the multigrid: 0 off; 1 float64 fine pressure and
                             residual; 2 the same with a double-float pressure (hi + lo, two floats,
                             ~48 significand bits) and residual, all float32 arithmetic */
-  int rb_pairs;          /* red-black sweep pairs per launch, 1..4 (0: 4): the temporal-blocking
+  int rb_pairs;          /* red-black sweep pairs per launch, 1..4 (0: by the grid's size): the temporal-blocking
                             depth, i.e. the tile/halo shape; results do not depend on it */
   int warm_extrapolate;  /* 1: the multigrid starts from 2 p(n) - p(n-1) on Fluid cells instead of
                             p(n) (no reference counterpart; pressureSolver.ts:28-30 uses p(n)) */
