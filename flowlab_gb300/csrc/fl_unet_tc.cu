@@ -639,29 +639,41 @@ bool halo_stacked(int N) { return 3 * N <= 256; }
 
 // ---------------------------------------------------------- weight gradient
 //
-// dW[n][tap][ci] = sum over pixels p of g[p][n] * x[p + off(tap)][ci] on the
-// tensor cores: D[ci][n] += A[ci][p] B[n][p] with K = pixels. Both tensors
-// are NHWC (channels innermost), so both operands are MN-major: a plane of
-// 16-byte pixel rows per 8 channels, exactly the halo planes of the forward
-// kernel (MN-major no-swizzle descriptors: LBO = 128 bytes between groups of
-// 8 pixel rows, SBO = the plane stride between groups of 8 channels). A tile
-// is 128 pixels of one image row: its g planes (4 x 8 output channels) and
-// the x halo (3 rows x 130 pixels x up to 128 input channels) arrive by TMA;
-// tap (ky, kx) reads the halo from row ky, column kx on, so one copy serves
-// all 9 taps. A CTA owns 32 output channels x up to 128 input channels (M =
-// 128; rows past Cin are computed from unused shared memory and dropped) and
-// a range of tiles; its 9 tap accumulators (288 TMEM columns) are added to
-// dW with atomics at the end. Warp 0 issues the copies (2-stage ring), warp 1
-// the MMAs, warps 2-5 the epilogue; every wait is bounded.
+// dW[n][ky][kx][ci] = sum over pixels p of g[p][n] * x[p + (ky - 1, kx - 1)][ci]
+// on the tensor cores: D[ci][n] += A[ci][p] B[n][p] with K = pixels. Both
+// tensors are NHWC (channels innermost), so both operands are MN-major: a
+// plane of 16-byte pixel rows per 8 channels, exactly the halo planes of the
+// forward kernel (MN-major no-swizzle descriptors: LBO = 128 bytes between
+// groups of 8 pixel rows, SBO = the plane stride between groups of 8
+// channels).
+//
+// Bound by the tensor pipe's cost per MMA, ~85 cycles for every N up to 128: so
+// the three ky taps share one. A tile is 128 pixels of x row y (130 with the
+// halo, up to 128 input channels) and the same columns of g's rows y - 1, y,
+// y + 1 (32 output channels): x row y meets g row y + 1 - ky in tap ky. The 12
+// planes (8 channels x one row) lie channel group by channel group, row by row
+// 2 KB apart, which is one N = 96 operand; tap kx reads x from column kx on. Rows
+// and columns outside the image arrive as zeros. With g's row alone as the
+// operand (N = 32, 9 taps' MMAs a tile, 3 rows of x) the 13 launches of a
+// 4 x 256^2 training step took 441 us, with three 291 (262144 pixels, 96 -> 32
+// channels: 48.5 -> 31.3).
+//
+// A CTA owns 32 output channels x up to 128 input channels (M = 128; rows past
+// Cin are computed from unused shared memory and dropped) and a range of
+// tiles; its 3 accumulators (288 TMEM columns) are added to dW with atomics at
+// the end. Warp 0 issues the copies (3-stage ring), warp 1 the MMAs, warps 2-5
+// the epilogue; every wait is bounded.
 constexpr int WG_TW = 128;                                           // pixels per tile
-constexpr int WG_NB = 32;                                            // output channels per CTA (N)
+constexpr int WG_NB = 32;                                            // output channels per CTA
+constexpr int WG_N = 3 * WG_NB;                                      // N: they, for each ky
 constexpr int WG_CB = 128;                                           // input channels per CTA (M)
-constexpr int WG_PL = ((3 * HALO_W * 16 + 127) / 128) * 128;         // x plane: 3 halo rows
+constexpr int WG_PL = ((HALO_W * 16 + 127) / 128) * 128;             // x plane: one halo row
 constexpr int WG_A = (WG_CB / 8) * WG_PL;
-constexpr int WG_GPL = WG_TW * 16;                                   // g plane
-constexpr int WG_B = (WG_NB / 8) * WG_GPL;
+constexpr int WG_GPL = WG_TW * 16;                                   // g plane of one row
+constexpr int WG_B = (WG_N / 8) * WG_GPL;
 constexpr int WG_STAGE = WG_A + WG_B;
-constexpr int WG_SMEM = 2 * WG_STAGE + 128;
+constexpr int WG_RING = 3;
+constexpr int WG_SMEM = WG_RING * WG_STAGE + 128;
 constexpr int WG_THREADS = 192;
 
 __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad_tc(const __grid_constant__ CUtensorMap xmap,
@@ -670,9 +682,9 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad_tc(const __grid_cons
                                                                int B, int Cin, int tiles_per_cta,
                                                                float* __restrict__ dw) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + 2 * WG_STAGE);
-  uint64_t* empty = full + 2;
-  uint64_t* done = empty + 2;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + WG_RING * WG_STAGE);
+  uint64_t* empty = full + WG_RING;
+  uint64_t* done = empty + WG_RING;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n0 = blockIdx.y * WG_NB, ci0 = blockIdx.z * WG_CB;
@@ -691,7 +703,7 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad_tc(const __grid_cons
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 32) {
-    for (int q = 0; q < 2; q++) {
+    for (int q = 0; q < WG_RING; q++) {
       mbar_init(smem_u32(&full[q]), 1);
       mbar_init(smem_u32(&empty[q]), 1);
     }
@@ -707,12 +719,12 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad_tc(const __grid_cons
 
   if (warp == 0) {
     if (lane == 0) {
-      const uint32_t tx = (uint32_t)((cb / 8) * 3 * HALO_W * 16 + (WG_NB / 8) * WG_TW * 16);
+      const uint32_t tx = (uint32_t)((cb / 8) * HALO_W * 16 + WG_B);
       int q = 0;
       for (; q < mytiles; q++) {
         const long t = t0 + q;
         const int bx = (int)(t % tiles_x), y = (int)((t / tiles_x) % H), img = (int)(t / ((long)tiles_x * H));
-        const int s = q & 1, use = q >> 1;
+        const int s = q % WG_RING, use = q / WG_RING;
         if (use > 0 && !mbar_wait(smem_u32(&empty[s]), (uint32_t)((use - 1) & 1), lim)) {
           failed = true;
           break;
@@ -722,33 +734,32 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad_tc(const __grid_cons
         mbar_expect_tx(fb, tx);
         for (int g = 0; g < cb / 8; g++)
           tma_load_4d(smem_u32(st + g * WG_PL), ci0 + 8 * g < split ? &xmap : &xmap2,
-                      ci0 + 8 * g < split ? ci0 + 8 * g : ci0 + 8 * g - split, bx * WG_TW - 1, y - 1, img, fb);
+                      ci0 + 8 * g < split ? ci0 + 8 * g : ci0 + 8 * g - split, bx * WG_TW - 1, y, img, fb);
         for (int g = 0; g < WG_NB / 8; g++)
-          tma_load_4d(smem_u32(st + WG_A + g * WG_GPL), &gmap, n0 + 8 * g, bx * WG_TW, y, img, fb);
+          tma_load_4d(smem_u32(st + WG_A + 3 * g * WG_GPL), &gmap, n0 + 8 * g, bx * WG_TW, y - 1, img, fb);
       }
-      for (int k = 1; k <= 2 && k <= q; k++) {
+      for (int k = 1; k <= WG_RING && k <= q; k++) {
         const int qq = q - k;
-        if (!mbar_drain(smem_u32(&full[qq & 1]), (uint32_t)((qq >> 1) & 1))) failed = true;
+        if (!mbar_drain(smem_u32(&full[qq % WG_RING]), (uint32_t)((qq / WG_RING) & 1))) failed = true;
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      // M = 128, N = 32, both operands MN-major (bits 15 and 16)
-      const uint32_t idesc = instr_desc(WG_CB, WG_NB) | (1u << 15) | (1u << 16);
+      // M = 128, N = 96, both operands MN-major (bits 15 and 16)
+      const uint32_t idesc = instr_desc(WG_CB, WG_N) | (1u << 15) | (1u << 16);
       for (int q = 0; q < mytiles; q++) {
-        const int s = q & 1, use = q >> 1;
+        const int s = q % WG_RING, use = q / WG_RING;
         if (!mbar_wait(smem_u32(&full[s]), (uint32_t)(use & 1), lim)) {
           failed = true;
           break;
         }
         tc_fence_after();
         const uint32_t a0 = smem_u32(smem + s * WG_STAGE), b0 = a0 + (uint32_t)WG_A;
-        for (int tp = 0; tp < 9; tp++) {
-          const int ky = tp / 3, kx = tp % 3;
-          const uint32_t dacc = tmem + (uint32_t)(tp * WG_NB);
+        for (int kx = 0; kx < 3; kx++) {
+          const uint32_t dacc = tmem + (uint32_t)(kx * WG_N);
 #pragma unroll
           for (int k = 0; k < WG_TW / 16; k++) {
-            const uint64_t ad = smem_desc(a0 + 16u * (uint32_t)(ky * HALO_W + kx + 16 * k), 128, WG_PL);
+            const uint64_t ad = smem_desc(a0 + 16u * (uint32_t)(kx + 16 * k), 128, WG_PL);
             const uint64_t bd = smem_desc(b0 + 16u * (uint32_t)(16 * k), 128, WG_GPL);
             mma_bf16(dacc, ad, bd, idesc, (q > 0 || k > 0) ? 1u : 0u);
           }
@@ -765,18 +776,25 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad_tc(const __grid_cons
   if (failed) {
     if (tid == 0) atomicExch(&g_tc_error, 1);
   } else if (warp >= 2 && mytiles > 0) {
-    // TMEM lane = input channel ci0 + lane index; column = tap * 32 + output channel
+    // TMEM lane = input channel ci0 + lane index; column = kx * 96 + plane * 8 +
+    // j, plane = 3 (output channel / 8) + row, of g's rows y - 1, y, y + 1 = ky 2, 1, 0
     const int quarter = warp & 3;
     const int ci = ci0 + quarter * 32 + lane;
     const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
-    for (int tp = 0; tp < 9; tp++) {
-      float v[32];
-      tmem_ld16_nowait(lane_base + (uint32_t)(tp * WG_NB), v);
-      tmem_ld16_nowait(lane_base + (uint32_t)(tp * WG_NB + 16), v + 16);
-      tmem_wait_ld();
-      if (quarter * 32 + lane < cb) {
+    for (int kx = 0; kx < 3; kx++) {
+      for (int part = 0; part < 3; part++) {  // four planes each
+        float v[32];
+        tmem_ld16_nowait(lane_base + (uint32_t)(kx * WG_N + part * 32), v);
+        tmem_ld16_nowait(lane_base + (uint32_t)(kx * WG_N + part * 32 + 16), v + 16);
+        tmem_wait_ld();
+        if (quarter * 32 + lane < cb) {
 #pragma unroll
-        for (int j = 0; j < WG_NB; j++) atomicAdd(&dw[((long)(n0 + j) * 9 + tp) * Cin + ci], v[j]);
+          for (int q = 0; q < 4; q++) {
+            const int plane = 4 * part + q, n = n0 + plane / 3 * 8, tp = (2 - plane % 3) * 3 + kx;
+#pragma unroll
+            for (int j = 0; j < 8; j++) atomicAdd(&dw[((long)(n + j) * 9 + tp) * Cin + ci], v[8 * q + j]);
+          }
+        }
       }
     }
   }
@@ -913,7 +931,7 @@ bool unet_tc_conv_wgrad(cudaStream_t s, const UnetInput& in, const __nv_bfloat16
   if ((reinterpret_cast<uintptr_t>(in.x) | reinterpret_cast<uintptr_t>(in.x2) | reinterpret_cast<uintptr_t>(g)) & 15)
     return false;
   CUtensorMap map[2], gmap;
-  if (!input_maps(map, in, Cin, W, H, B, HALO_W, 3) || !image_map(&gmap, g, Cout, W, H, B, WG_TW, 1)) return false;
+  if (!input_maps(map, in, Cin, W, H, B, HALO_W, 1) || !image_map(&gmap, g, Cout, W, H, B, WG_TW, 3)) return false;
   const int nblk = Cout / WG_NB, cblk = (Cin + WG_CB - 1) / WG_CB;
   const long ntiles = (long)((W + WG_TW - 1) / WG_TW) * H * B;
   long ctas = (g_num_sms + nblk * cblk - 1) / (nblk * cblk);
