@@ -1860,8 +1860,14 @@ struct BatchSolve {
   std::pair<int, int> init_ph{0, 0}, zero_ph{0, 0};  // prologue defect pass, p = 0 fill: every scene
 };
 
+// Before a kernel's dep_wait: the lists are k_batch_check's, of the cycle
+// before. A block without items waits all the same (its kernel's end stands for
+// the end of all before it).
 __device__ __forceinline__ bool batch_item(const BatchPlan& P, int ph, int i, BatchItem& it) {
-  if (i >= P.act_total[ph]) return false;
+  if (i >= P.act_total[ph]) {
+    dep_wait();
+    return false;
+  }
   const int* pre = P.act_pre + (long)ph * (P.n + 1);
   int lo = 0, hi = P.act_n[ph] - 1;  // the last active scene whose prefix is <= i
   while (lo < hi) {
@@ -2006,6 +2012,7 @@ __global__ void __launch_bounds__(1024) k_batch_begin(BatchPlan plan, cudaGraphC
 // Every iterating scene's cycle test (the others keep their state), the
 // compacted lists of the next cycle.
 __global__ void __launch_bounds__(1024) k_batch_check(BatchPlan plan, cudaGraphConditionalHandle h) {
+  dep_wait();
   int any = 0;
   for (int k = threadIdx.x; k < plan.n; k += blockDim.x)
     if (plan.sc[k].ctl->cont) any |= solve_check(plan.sc[k].acc, plan.sc[k].ctl);
@@ -2208,12 +2215,13 @@ static unsigned phase_grid(const BatchSolve& b, int ph, int per_sm) {
 }
 
 template <int MODE>
-static void launch_batch_smooth(cudaStream_t s, const BatchSolve& b, int pairs, int ph) {
+static void launch_batch_smooth(cudaStream_t s, const BatchSolve& b, int pairs, int ph, bool& early) {
   if (b.max_items[ph] == 0) return;
   if (b.small[ph])
-    k_batch_smooth<MODE, 16, 2><<<phase_grid(b, ph, 2), 512, 0, s>>>(b.plan, ph, pairs);
+    launch_dependent(early, k_batch_smooth<MODE, 16, 2>, phase_grid(b, ph, 2), 512, s, b.plan, ph, pairs);
   else
-    k_batch_smooth<MODE, 8, 8><<<phase_grid(b, ph, 3), 256, 0, s>>>(b.plan, ph, pairs);
+    launch_dependent(early, k_batch_smooth<MODE, 8, 8>, phase_grid(b, ph, 3), 256, s, b.plan, ph, pairs);
+  early = true;
 }
 
 // The whole batched solve, enqueued on `s` while it is being captured: the
@@ -2247,17 +2255,19 @@ cudaError_t batch_solve_enqueue(const BatchSolve& b, cudaStream_t s, cudaStream_
     err = cudaStreamBeginCaptureToGraph(body, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                         cudaStreamCaptureModeThreadLocal);
   if (err != cudaSuccess) return err;
+  // each but the body's first may start while the one before it drains
+  // (launch_dependent): 12 uneven scenes up to 512^2, three steps 8.1 -> 7.5 ms
   const int D = b.depth;
-  for (int d = 0; d < D; d++) launch_batch_smooth<MODE_PRE>(body, b, b.pre, d);
-  if (b.tail_threads > 512)
-    k_batch_tail<64><<<phase_grid(b, D, 1), b.tail_threads, 0, body>>>(b.plan, D);
-  else
-    k_batch_tail<32><<<phase_grid(b, D, 1), b.tail_threads, 0, body>>>(b.plan, D);
-  for (int d = 0; d < D; d++) launch_batch_smooth<MODE_POST>(body, b, b.post, D + 1 + d);
+  bool early = false;
+  for (int d = 0; d < D; d++) launch_batch_smooth<MODE_PRE>(body, b, b.pre, d, early);
+  launch_dependent(early, b.tail_threads > 512 ? k_batch_tail<64> : k_batch_tail<32>, phase_grid(b, D, 1), b.tail_threads,
+                   body, b.plan, D);
+  early = true;
+  for (int d = 0; d < D; d++) launch_batch_smooth<MODE_POST>(body, b, b.post, D + 1 + d, early);
   if (b.max_items[2 * D + 1] > 0)
-    (rows == 2 ? k_batch_defect<2> : rows == 4 ? k_batch_defect<4> : k_batch_defect<8>)<<<
-        phase_grid(b, 2 * D + 1, 8), 32 * DEFECT_WARPS, 0, body>>>(b.plan, 2 * D + 1, b.defect_rows[1]);
-  k_batch_check<<<1, 1024, 0, body>>>(b.plan, h);
+    launch_dependent(early, rows == 2 ? k_batch_defect<2> : rows == 4 ? k_batch_defect<4> : k_batch_defect<8>,
+                     phase_grid(b, 2 * D + 1, 8), 32 * DEFECT_WARPS, body, b.plan, 2 * D + 1, b.defect_rows[1]);
+  launch_dependent(early, k_batch_check, 1, 1024, body, b.plan, h);
   cudaGraph_t done = nullptr;
   err = cudaStreamEndCapture(body, &done);
   if (err != cudaSuccess) return err;
