@@ -67,7 +67,7 @@ LIMITERS = {
     "mg_coarse": "latency: one CTA, a chain of dependent barrier phases",
     "mg_pre": "latency: small levels, few CTAs per launch",
     "mg_post": "latency: small levels, few CTAs per launch",
-    "mg_fine": "instruction issue: temporally blocked sweeps with halo recompute, working set in L2",
+    "mg_fine": "instruction issue and the region's latency: temporally blocked sweeps with halo recompute, working set in L2",
 }
 
 
