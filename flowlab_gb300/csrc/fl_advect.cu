@@ -19,15 +19,14 @@
 
 namespace fl {
 
-// advect.ts:41-55
-template <class S>
-__device__ __forceinline__ void backtrace(const float* __restrict__ uc, const float* __restrict__ vc, int nx, int ny,
-                                          const S& h, float x, float y, float u0, float v0, float dt, float& bx,
-                                          float& by) {
+// advect.ts:41-55 (FRESH: sample's)
+template <bool FRESH = false, class S>
+__device__ __forceinline__ void backtrace(const float* uc, const float* vc, int nx, int ny, const S& h, float x,
+                                          float y, float u0, float v0, float dt, float& bx, float& by) {
   float midX = x - 0.5f * dt * u0;
   float midY = y - 0.5f * dt * v0;
-  bx = x - dt * sample_u(uc, nx, ny, h, midX, midY);
-  by = y - dt * sample_v(vc, nx, ny, h, midX, midY);
+  bx = x - dt * sample_u<FRESH>(uc, nx, ny, h, midX, midY);
+  by = y - dt * sample_v<FRESH>(vc, nx, ny, h, midX, midY);
 }
 
 // The carrier at a face's own position, where the face holds only one of its
@@ -98,8 +97,8 @@ __device__ __forceinline__ void advect_faces(int nx, int ny, const S& h, const f
     rv = sample(v_in, pv, nx);
   } else {
     const int au = u_fixed ? 0 : __float_as_int(u_out[ku]), av = v_fixed ? 0 : __float_as_int(v_out[kv]);
-    ru = clamp_at(u_in, au, nx + 1, u_hat[ku] + 0.5f * (uu - sample_fresh(u_hat, pu, nx + 1)));
-    rv = clamp_at(v_in, av, nx, v_hat[kv] + 0.5f * (vv - sample_fresh(v_hat, pv, nx)));
+    ru = clamp_at(u_in, au, nx + 1, u_hat[ku] + 0.5f * (uu - sample<true>(u_hat, pu, nx + 1)));
+    rv = clamp_at(v_in, av, nx, v_hat[kv] + 0.5f * (vv - sample<true>(v_hat, pv, nx)));
   }
   if (u_in_grid) {
     const int k = i + j * (nx + 1);
@@ -160,10 +159,13 @@ __device__ __forceinline__ void advect_cells(int nx, int ny, const S& h, int dnx
   } else {
     const float x = ((float)i + 0.5f) * dh.h;
     const float y = ((float)j + 0.5f) * dh.h;
-    const float u0 = sample_u(u, nx, ny, h, x, y);
-    const float v0 = sample_v(v, nx, ny, h, x, y);
+    // u and v are the projection's, which the forward pass starts behind; the
+    // correction starts once every block of that pass has seen its end
+    constexpr bool FRESH = MODE == 0;
+    const float u0 = sample_u<FRESH>(u, nx, ny, h, x, y);
+    const float v0 = sample_v<FRESH>(v, nx, ny, h, x, y);
     float bx, by;
-    backtrace(u, v, nx, ny, h, x, y, u0, v0, MODE == 0 ? dt : -dt, bx, by);
+    backtrace<FRESH>(u, v, nx, ny, h, x, y, u0, v0, MODE == 0 ? dt : -dt, bx, by);
     const Stencil p = stencil_p(dnx, dny, dh, bx, by);
     if (MODE == 0) {
       if (at != nullptr) at[k] = __int_as_float(p.k);
@@ -176,7 +178,7 @@ __device__ __forceinline__ void advect_cells(int nx, int ny, const S& h, int dnx
 #pragma unroll
       for (int c = 0; c < DYE_CHANNELS; c++) {
         const float corrected =
-            q_hat[k + c * cells] + 0.5f * (q_in[k + c * cells] - sample_fresh(q_hat + c * cells, p, dnx));
+            q_hat[k + c * cells] + 0.5f * (q_in[k + c * cells] - sample<true>(q_hat + c * cells, p, dnx));
         q[c] = clamp_at(q_in + c * cells, ck, dnx, corrected);
       }
     }
@@ -213,7 +215,7 @@ __global__ void __launch_bounds__(256) k_advect_dye(int nx, int ny, Spacing h, i
                                                     const float* __restrict__ patch, int pi0, int pj0, int pnx,
                                                     int pny, float* at) {
   if (MODE == 0) {
-    dep_wait();  // u and v are the launch before's (ordinary loads: not restrict)
+    dep_wait();  // u and v are the launch before's
     dep_trigger();
   }
   if (h.pow2 && dh.pow2)

@@ -216,16 +216,14 @@ struct Stencil {
   float fx, fy;
 };
 
-__device__ __forceinline__ float sample(const float* __restrict__ f, const Stencil& p, int s) {
+// FRESH: the field may be what the launch before this one writes (dep_wait):
+// ordinary loads, which stay behind the wait. The read-only loads otherwise
+// taken are defined only for memory that nobody writes while the kernel lives.
+template <bool FRESH = false>
+__device__ __forceinline__ float sample(const float* f, const Stencil& p, int s) {
   const float* q = f + p.k;
+  if (FRESH) return bilerp(q[0], q[1], q[s], q[s + 1], p.fx, p.fy);
   return bilerp(ldg(q), ldg(q + 1), ldg(q + s), ldg(q + s + 1), p.fx, p.fy);
-}
-
-// The same of a field that the launch before this one may have written
-// (dep_wait): ordinary loads, which stay behind the wait.
-__device__ __forceinline__ float sample_fresh(const float* f, const Stencil& p, int s) {
-  const float* q = f + p.k;
-  return bilerp(q[0], q[1], q[s], q[s + 1], p.fx, p.fy);
 }
 
 __device__ __forceinline__ Stencil stencil_at(float px, float py, int nx, int ny) {
@@ -252,13 +250,13 @@ template <class S>
 __device__ __forceinline__ Stencil stencil_p(int nx, int ny, const S& h, float x, float y) {
   return stencil_at(over(x, h) - 0.5f, over(y, h) - 0.5f, nx, ny);
 }
-template <class S>
-__device__ __forceinline__ float sample_u(const float* __restrict__ u, int nx, int ny, const S& h, float x, float y) {
-  return sample(u, stencil_u(nx, ny, h, x, y), nx + 1);
+template <bool FRESH = false, class S>
+__device__ __forceinline__ float sample_u(const float* u, int nx, int ny, const S& h, float x, float y) {
+  return sample<FRESH>(u, stencil_u(nx, ny, h, x, y), nx + 1);
 }
-template <class S>
-__device__ __forceinline__ float sample_v(const float* __restrict__ v, int nx, int ny, const S& h, float x, float y) {
-  return sample(v, stencil_v(nx, ny, h, x, y), nx);
+template <bool FRESH = false, class S>
+__device__ __forceinline__ float sample_v(const float* v, int nx, int ny, const S& h, float x, float y) {
+  return sample<FRESH>(v, stencil_v(nx, ny, h, x, y), nx);
 }
 template <class S>
 __device__ __forceinline__ float sample_p(const float* __restrict__ q, int nx, int ny, const S& h, float x, float y) {
