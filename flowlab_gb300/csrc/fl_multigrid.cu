@@ -1456,9 +1456,9 @@ static RbShape rb_shape(int nx, int ny, int pairs) {
 }
 
 int rb_launch_pairs(int nx, int ny, int span) {
-  int best = std::min(span, 4);
+  int best = std::max(1, std::min(span, 4));  // (no sweeps at all: any)
   float time = FLT_MAX;
-  for (int p = std::min(span, 4); p <= 10 && p <= span; p++) {
+  for (int p = best; p <= 10 && p <= span; p++) {
     const int launches = (span + p - 1) / p, q = (span + launches - 1) / launches;
     const RbShape sh = rb_shape(nx, ny, q);
     if (sh.rw == 8 && q > 4) continue;
