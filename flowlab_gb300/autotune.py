@@ -12,8 +12,9 @@ What it chooses, per scene shape and solver:
                  budget on the scene's own right-hand sides (the reference's
                  browser setting, a fixed budget, makes accuracy the
                  objective); then the sweep pairs per launch (rb_pairs: the
-                 temporal-blocking depth, i.e. the tile/halo shape), whose
-                 results are identical, by time alone;
+                 temporal-blocking depth, i.e. the tile/halo shape; 0 the
+                 library's own choice by the grid), whose results are
+                 identical, by time alone;
   warm start     whether the learned warm start stays attached: only when
                  the warm-started step is measured faster than the plain
                  one on the scene itself (the network's forward pass must
@@ -36,7 +37,7 @@ from .native import f32, ptr
 
 MG_SPACE = {"mg_coarsest": (4, 8, 16, 32), "mg_coarse_sweeps": (8, 16, 32)}
 RB_OMEGAS = (1.5, 1.6, 1.7, 1.8, 1.85, 1.9, 1.95, 1.98)
-RB_PAIRS = (1, 2, 3, 4)
+RB_PAIRS = (0, 1, 2, 3, 4)  # 0: the library's choice by the grid, the only one beyond 4
 TAIL_SIDES = (16, 32, 64)
 
 
