@@ -645,18 +645,15 @@ void Unet::conv_up_fwd(cudaStream_t s, int l, const __nv_bfloat16* u, int Cu, co
 // conv_bwd of a decoder's first layer, without the data gradient's ReLU mask.
 void Unet::conv_up_bwd(cudaStream_t s, int l, const __nv_bfloat16* u, int Cu, const __nv_bfloat16* skip, int Cs,
                        __nv_bfloat16* c, const float* g, int B, int H, int W, float* gx) {
-  if (split[l] && !unet_tc_two_inputs()) {  // the forms changed since the forward pass
-    k_up_concat<<<grid_for((long)B * H * W * (Cu + Cs)), 256, 0, s>>>(u, Cu, skip, Cs, B, H, W, c);
-    split[l] = false;
-  }
-  conv_bwd(s, l, split[l] ? UnetInput{c, skip, Cu} : UnetInput{c, nullptr, Cu + Cs}, g, B, H, W, gx, nullptr);
+  conv_bwd(s, l, split[l] ? UnetInput{c, skip, Cu} : UnetInput{c, nullptr, Cu + Cs}, g, B, H, W, gx, nullptr, u, c);
 }
 
 // Weight gradient of layer l from its input x and pre-activation gradient g,
 // then (when gx is set) the data gradient into gx, masked by act_x > 0 when
-// act_x is set.
+// act_x is set. u, c: an input in two parts may be formed whole in c, from the
+// upsampled part's source u.
 void Unet::conv_bwd(cudaStream_t s, int l, const UnetInput& in, const float* g, int B, int H, int W, float* gx,
-                    const __nv_bfloat16* act_x) {
+                    const __nv_bfloat16* act_x, const __nv_bfloat16* u, __nv_bfloat16* c) {
   const __nv_bfloat16* x = in.x;
   const UnetLayer& L = kUnetLayers[l];
   const long P = (long)B * H * W;
@@ -674,6 +671,11 @@ void Unet::conv_bwd(cudaStream_t s, int l, const UnetInput& in, const float* g, 
     }
   }
   if (!done) {
+    if (in.x2 != nullptr) {  // only the tensor-core kernel reads two parts
+      k_up_concat<<<grid_for(P * L.cin), 256, 0, s>>>(u, in.split, in.x2, L.cin - in.split, B, H, W, c);
+      split[l] = false;
+      x = c;
+    }
     dim3 gw((unsigned)(((W + CT - 1) / CT) * ((H + CT - 1) / CT)), (unsigned)(B * ((L.cout + CO_T - 1) / CO_T)),
             (unsigned)((L.cin + CK - 1) / CK));
     k_conv3_wgrad<<<gw, 256, 0, s>>>(x, g, H, W, L.cin, L.cout, grad + woff[l], tc ? nullptr : grad + boff[l]);

@@ -83,7 +83,7 @@ struct Unet {
   void refresh_weight_images(cudaStream_t s);
   void conv_fwd(cudaStream_t s, int l, const __nv_bfloat16* x, int B, int H, int W, __nv_bfloat16* y);
   void conv_bwd(cudaStream_t s, int l, const UnetInput& in, const float* g, int B, int H, int W, float* gx,
-                const __nv_bfloat16* act_x);
+                const __nv_bfloat16* act_x, const __nv_bfloat16* u = nullptr, __nv_bfloat16* c = nullptr);
   void conv_up_fwd(cudaStream_t s, int l, const __nv_bfloat16* u, int Cu, const __nv_bfloat16* skip, int Cs, int B,
                    int H, int W, __nv_bfloat16* c, __nv_bfloat16* y);
   void conv_up_bwd(cudaStream_t s, int l, const __nv_bfloat16* u, int Cu, const __nv_bfloat16* skip, int Cs,
