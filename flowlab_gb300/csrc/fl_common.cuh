@@ -115,6 +115,7 @@ struct Spacing {
   float h;
   float inv;
   int pow2;
+  unsigned span;  // over(x, SpacingAny): the x of the corrected product
 };
 
 __host__ inline Spacing make_spacing(float h) {
@@ -123,7 +124,11 @@ __host__ inline Spacing make_spacing(float h) {
   Spacing s;
   s.h = h;
   s.inv = 1.0f / h;
-  s.pow2 = (m == 0.5f) ? 1 : 0;
+  // cell sizes far from 1 divide: quotients, reciprocals and positions of the
+  // others stay normal floats
+  const bool usual = h >= 0x1p-60f && h <= 0x1p60f;
+  s.pow2 = usual && m == 0.5f ? 1 : 0;
+  s.span = usual ? 0x40000000u : 0u;
   return s;
 }
 
@@ -139,18 +144,20 @@ struct SpacingPow2 {
 struct SpacingAny {
   float h;
   float inv;
-  __device__ __forceinline__ explicit SpacingAny(const Spacing& s) : h(s.h), inv(s.inv) {}
+  unsigned span;
+  __device__ __forceinline__ explicit SpacingAny(const Spacing& s) : h(s.h), inv(s.inv), span(s.span) {}
 };
 
 // x / h. For a general h the quotient by the correctly rounded reciprocal,
 // corrected twice: the first correction brings it within a unit in the last
 // place, the second one rounds it correctly (Markstein: q' = RN(q + r RN(1/h))
 // with the exact remainder r of such a q is RN(x / h)), in 5 operations without
-// a branch. Tiny, huge, infinite and NaN x, where a remainder could underflow
-// or overflow, take the division.
+// a branch. Tiny, huge, infinite and NaN x (outside 2^-63 <= |x| < 2^65), where
+// a remainder could underflow or overflow, take the division; with an unusual
+// cell size (make_spacing) every x does.
 __device__ __forceinline__ float over(float x, const SpacingPow2& s) { return x * s.inv; }
 __device__ __forceinline__ float over(float x, const SpacingAny& s) {
-  if ((__float_as_uint(x) & 0x7fffffffu) - 0x20000000u >= 0x40000000u) return div_slow(x, s.h);
+  if ((__float_as_uint(x) & 0x7fffffffu) - 0x20000000u >= s.span) return div_slow(x, s.h);
   float q = __fmul_rn(x, s.inv);
   float r = __fmaf_rn(-s.h, q, x);
   q = __fmaf_rn(r, s.inv, q);
