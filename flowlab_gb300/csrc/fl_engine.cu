@@ -712,7 +712,6 @@ void destroy_step_graphs(Engine* e) {
     if (g) cudaGraphExecDestroy(g);
     g = nullptr;
   }
-  e->graphs_valid = false;
   e->graph_gen++;
 }
 
@@ -803,15 +802,14 @@ bool graph_eligible(const Engine* e) {
 
 // cfl_first: the step right after fl_step_host's upload, which left the
 // clock reset and the CFL scalars to the step's graph.
-// host: fl_step_host's step (built on first use).
+// host: fl_step_host's step.
+// Graphs are built when a step of their kind first runs: both parities at once,
+// or the one that follows an upload.
 int step_graph(Engine* e, bool cfl_first = false, bool host = false) {
-  if (!e->graphs_valid) {
-    destroy_step_graphs(e);
-    for (int par = 0; par < 2; par++) TRY(build_graph(e, par, &e->graph[par], false, false));
-    e->graphs_valid = true;
-  }
-  cudaGraphExec_t& g = cfl_first ? e->graph_up[e->cur] : host ? e->graph_host[e->cur] : e->graph[e->cur];
-  if (!g) TRY(build_graph(e, e->cur, &g, cfl_first, host));
+  cudaGraphExec_t* pair = cfl_first ? e->graph_up : host ? e->graph_host : e->graph;
+  for (int par = 0; par < 2; par++)
+    if (!pair[par] && (par == e->cur || !cfl_first)) TRY(build_graph(e, par, &pair[par], cfl_first, host));
+  cudaGraphExec_t g = pair[e->cur];
   TRY(cuda_status(e, cudaGraphLaunch(g, e->stream), "graph launch"));
   e->cur = 1 - e->cur;
   e->steps++;

@@ -104,7 +104,6 @@ struct Engine {
   // they changed (label_flag: set when any cell differs)
   uint8_t* label_in = nullptr;
   int* label_flag = nullptr;
-  bool graphs_valid = false;
   // counts every destruction of the step graphs (parameters, patch, warm
   // start or levels changed): a batch rebuilds its own graphs when it moves
   unsigned long long graph_gen = 0;
