@@ -483,7 +483,7 @@ void enqueue_solve_prologue(Engine* e, cudaStream_t s, bool mixed, bool use_cond
     // the begin test runs in the pass's last block
     const int tok = prof_begin(*e, FL_PH_DEFECT64);
     launch_update_resid64(s, e->nx, e->ny, e->p64[0], e->p64[1], e->ctl, nullptr, L0.b, e->b_lo, L0.code, false,
-                          e->r32, e->acc, refined_df(e), 1, use_cond, h);
+                          e->r32, e->acc, refined_df(e), e->sms, 1, use_cond, h);
     // p64, b, code in; r32 out
     prof_end(*e, tok, 17.0 * e->cells(), 1);
     return;
@@ -503,7 +503,7 @@ void enqueue_solve_body(Engine* e, cudaStream_t s, bool mixed, bool use_cond, cu
     mg_vcycle_on(*e, e->r32, true, nullptr);
     const int tok = prof_begin(*e, FL_PH_DEFECT64);
     launch_update_resid64(s, e->nx, e->ny, e->p64[0], e->p64[1], e->ctl, L0.x[0], L0.b, e->b_lo, L0.code, true,
-                          e->r32, e->acc, refined_df(e), 2, use_cond, h);
+                          e->r32, e->acc, refined_df(e), e->sms, 2, use_cond, h);
     // p64, e, b, code in; p64 (other buffer), r32 out
     prof_end(*e, tok, 29.0 * e->cells(), 1);
     return;
@@ -529,12 +529,12 @@ void enqueue_rb_fixed(Engine* e, cudaStream_t s) {
   launch_solve_begin(s, e->acc, e->ctl, false, 0);
   int k = 0, src = 0;
   const int iters = e->prm.pressure_iters;
-  const int per = e->prm.rb_pairs > 0 ? e->prm.rb_pairs : rb_launch_pairs(L.nx, L.ny, iters);
+  const int per = e->prm.rb_pairs > 0 ? e->prm.rb_pairs : rb_launch_pairs(L.nx, L.ny, iters, e->sms);
   while (k < iters) {
     const int chunk = std::min(per, iters - k);
     const int tok = prof_begin(*e, FL_PH_RB_SWEEPS);
     launch_rb_sweeps(s, L.nx, L.ny, L.x[src], L.x[1 - src], L.b, L.code, 0.0f, (float)e->prm.omega, chunk,
-                     &e->sc->scale, k > 0);
+                     &e->sc->scale, k > 0, e->sms);
     prof_end(*e, tok, 13.0 * e->cells(), 1);
     src = 1 - src;
     k += chunk;
@@ -601,13 +601,13 @@ int rb_solve_device(Engine* e, float scale, int iterations, float omega, double 
   int k = 0;
   int src = 0;
   const int per = e->prm.rb_pairs > 0 ? e->prm.rb_pairs
-                                      : rb_launch_pairs(L.nx, L.ny, checks ? std::min(12, iterations) : iterations);
+                                      : rb_launch_pairs(L.nx, L.ny, checks ? std::min(12, iterations) : iterations, e->sms);
   while (k < iterations) {
     int chunk = std::min(per, iterations - k);
     if (checks) chunk = std::min(chunk, 12 - (k % 12));
     const int tok = prof_begin(*e, FL_PH_RB_SWEEPS);
     launch_rb_sweeps(e->stream, L.nx, L.ny, L.x[src], L.x[1 - src], L.b, L.code, scale, omega, chunk, nullptr,
-                     k > 0 && !(checks && k % 12 == 0));
+                     k > 0 && !(checks && k % 12 == 0), e->sms);
     prof_end(*e, tok, 13.0 * e->cells(), 1);
     TRY(check_launch(e, "red-black sweeps"));
     src = 1 - src;
@@ -884,11 +884,15 @@ int fl_create(int nx, int ny, double h, int dye_scale, const fl_params* params, 
     return fail(nullptr, FL_EDEVICE, "no CUDA device (%s)", err != cudaSuccess ? cudaGetErrorString(err) : "count 0");
   if (device < 0 || device >= ndev) return fail(nullptr, FL_EINVAL, "device %d of %d", device, ndev);
   if (cudaSetDevice(device) != cudaSuccess) return fail(nullptr, FL_EDEVICE, "cudaSetDevice(%d) failed", device);
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 1)
+    return fail(nullptr, FL_EDEVICE, "multiprocessor count of device %d", device);
 
   fl_engine* H = new (std::nothrow) fl_engine();
   if (!H) return fail(nullptr, FL_ENOMEM, "host allocation");
   Engine* e = &H->e;
   e->device = device;
+  e->sms = sms;
   e->nx = nx;
   e->ny = ny;
   e->dye_scale = dye_scale;

@@ -32,6 +32,7 @@ struct Level {
 
 struct Engine {
   int device = 0;
+  int sms = 1;  // the device's, which the launch shapes follow
   int nx = 0, ny = 0, dnx = 0, dny = 0, dye_scale = 1;
   float h = 0, dh = 0;
   fl_params prm{};
@@ -294,7 +295,7 @@ void mg_vcycle_on(Engine& e, const float* b0, bool zero_start, StepAccum* acc_fo
 // use_cond, sets the graph's conditional handle h.
 void launch_update_resid64(cudaStream_t s, int nx, int ny, double* p64a, double* p64b, SolveCtl* ctl,
                            const float* e, const float* b, const float* b_lo, const uint8_t* code, bool update,
-                           float* r32, StepAccum* acc, bool df, int test = 0, bool use_cond = false,
+                           float* r32, StepAccum* acc, bool df, int sms, int test = 0, bool use_cond = false,
                            cudaGraphConditionalHandle h = 0);
 void launch_solve_begin(cudaStream_t s, StepAccum* acc, SolveCtl* ctl, bool use_cond, cudaGraphConditionalHandle h);
 void launch_solve_check(cudaStream_t s, StepAccum* acc, SolveCtl* ctl, bool use_cond, cudaGraphConditionalHandle h);
@@ -302,9 +303,10 @@ void launch_zero_if(cudaStream_t s, const SolveCtl* ctl, float* p32, double* p64
 // early: the kernel before it on the stream is another of these launches of
 // the same row (b, code and *scale_dev as they were)
 void launch_rb_sweeps(cudaStream_t s, int nx, int ny, const float* x_in, float* x_out, const float* b,
-                      const uint8_t* code, float scale, float omega, int pairs, const float* scale_dev, bool early);
+                      const uint8_t* code, float scale, float omega, int pairs, const float* scale_dev, bool early,
+                      int sms);
 // Sweep pairs a launch for `span` of them in a row (at most 10).
-int rb_launch_pairs(int nx, int ny, int span);
+int rb_launch_pairs(int nx, int ny, int span, int sms);
 void launch_rms_remaining(cudaStream_t s, int nx, int ny, const float* p, const float* div, const uint8_t* code,
                           float scale, StepAccum* acc);
 void launch_build_codes(cudaStream_t s, int nx, int ny, const uint8_t* label, uint8_t* code);

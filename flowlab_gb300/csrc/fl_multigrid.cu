@@ -184,11 +184,11 @@ __device__ __forceinline__ float2 link_factors(int code) {
 // The shapes: 8 warps of 8 rows (a 64 x 64 region) spend the fewest
 // instructions a cell; 16 warps of 2 rows (64 x 32) have the shortest chain
 // of updates a warp, for levels whose 64 x 64 regions would leave SMs idle or
-// give a few of them a second one (SMOOTH_SMALL regions): PRE at 512^2 (100
-// regions) 4.2 against 3.2 us, 640^2 (169) 4.9 against 4.2, 704^2 (196) 4.9
+// give a few of them a second one (fewer than smooth_small, 176 on 152 SMs): PRE
+// at 512^2 (100 regions) 4.2 against 3.2 us, 640^2 (169) 4.9 against 4.2, 704^2 (196) 4.9
 // against 4.9, POST 5.4 against 5.8, 1024^2 (400) 6.1 against 7.7. 8 x 4 and
 // 16 x 4 lay between.
-constexpr long SMOOTH_SMALL = 176;
+static long smooth_small(int sms) { return 22L * sms / 19; }
 
 template <int NW, int RW>
 struct SmoothShared {
@@ -1392,21 +1392,21 @@ static void launch_smooth_nw(cudaStream_t s, const SmoothArgs& a, bool early) {
 }
 
 template <int MODE>
-static void launch_smooth_mode(cudaStream_t s, const SmoothArgs& a, bool early) {
+static void launch_smooth_mode(cudaStream_t s, const SmoothArgs& a, bool early, int sms) {
   const int t = 64 - 2 * a.halo;
-  if ((long)((a.nx + t - 1) / t) * ((a.ny + t - 1) / t) < SMOOTH_SMALL)
+  if ((long)((a.nx + t - 1) / t) * ((a.ny + t - 1) / t) < smooth_small(sms))
     launch_smooth_nw<MODE, 16, 2>(s, a, early);
   else
     launch_smooth_nw<MODE, 8, 8>(s, a, early);
 }
 
-static void launch_smooth(cudaStream_t s, SmoothArgs a, int pairs, int mode, bool early) {
+static void launch_smooth(cudaStream_t s, SmoothArgs a, int pairs, int mode, bool early, int sms) {
   a.pairs = pairs;
   a.halo = smooth_halo(mode, pairs, a.x_is_zero, a.acc != nullptr);
   if (mode == MODE_PRE)
-    launch_smooth_mode<MODE_PRE>(s, a, early);
+    launch_smooth_mode<MODE_PRE>(s, a, early, sms);
   else
-    launch_smooth_mode<MODE_POST>(s, a, early);
+    launch_smooth_mode<MODE_POST>(s, a, early, sms);
 }
 
 static void launch_level_codes(cudaStream_t s, int nx, int ny, const uint8_t* label, uint8_t* code, uint8_t* coarse,
@@ -1440,27 +1440,26 @@ struct RbShape {
   int nw, rw;
   float us;  // a launch
 };
-static RbShape rb_shape(int nx, int ny, int pairs) {
-  constexpr long SMS = 152;
+static RbShape rb_shape(int nx, int ny, int pairs, int sms) {
   const int tx = 64 - 4 * pairs;
   auto regions = [&](int ty) { return (long)((nx + tx - 1) / tx) * ((ny + ty - 1) / ty); };
   const long four = regions(tx);
-  RbShape best{8, 8, 0.018f * four};
-  if (four <= 2 * SMS) best = {16, 4, four <= SMS ? 2.6f + 0.4f * pairs : 2.8f + 0.73f * pairs};
+  RbShape best{8, 8, 2.736f / sms * four};
+  if (four <= 2L * sms) best = {16, 4, four <= sms ? 2.6f + 0.4f * pairs : 2.8f + 0.73f * pairs};
   if (pairs <= 6) {  // a region of 32 rows
     const long two = regions(32 - 4 * pairs);
-    const float us = two <= SMS ? 1.6f + 0.28f * pairs : 1.7f + 0.48f * pairs;
-    if (two <= 2 * SMS && us < best.us) best = {16, 2, us};
+    const float us = two <= sms ? 1.6f + 0.28f * pairs : 1.7f + 0.48f * pairs;
+    if (two <= 2L * sms && us < best.us) best = {16, 2, us};
   }
   return best;
 }
 
-int rb_launch_pairs(int nx, int ny, int span) {
+int rb_launch_pairs(int nx, int ny, int span, int sms) {
   int best = std::max(1, std::min(span, 4));  // (no sweeps at all: any)
   float time = FLT_MAX;
   for (int p = best; p <= 10 && p <= span; p++) {
     const int launches = (span + p - 1) / p, q = (span + launches - 1) / launches;
-    const RbShape sh = rb_shape(nx, ny, q);
+    const RbShape sh = rb_shape(nx, ny, q, sms);
     if (sh.rw == 8 && q > 4) continue;
     if (launches * sh.us < time) {
       time = launches * sh.us;
@@ -1471,7 +1470,8 @@ int rb_launch_pairs(int nx, int ny, int span) {
 }
 
 void launch_rb_sweeps(cudaStream_t s, int nx, int ny, const float* x_in, float* x_out, const float* b,
-                      const uint8_t* code, float scale, float omega, int pairs, const float* scale_dev, bool early) {
+                      const uint8_t* code, float scale, float omega, int pairs, const float* scale_dev, bool early,
+                      int sms) {
   SmoothArgs a{};
   a.scale_dev = scale_dev;
   a.nx = nx;
@@ -1484,7 +1484,7 @@ void launch_rb_sweeps(cudaStream_t s, int nx, int ny, const float* x_in, float* 
   a.omega = omega;
   a.pairs = pairs;
   a.halo = smooth_halo(MODE_PLAIN, pairs, false, false);
-  const RbShape sh = rb_shape(nx, ny, pairs);
+  const RbShape sh = rb_shape(nx, ny, pairs, sms);
   if (sh.rw == 2)
     launch_smooth_nw<MODE_PLAIN, 16, 2>(s, a, early);
   else if (sh.rw == 4)
@@ -1544,20 +1544,12 @@ static int defect_rows(bool df, int sms, Blocks blocks) {
   return 8;
 }
 
-// The device's SMs.
-static int sm_count() {
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    n = 0;
-  return n > 0 ? n : 1;
-}
-
 void launch_update_resid64(cudaStream_t s, int nx, int ny, double* p64a, double* p64b, SolveCtl* ctl,
                            const float* e, const float* b, const float* b_lo, const uint8_t* code, bool update,
-                           float* r32, StepAccum* acc, bool df, int test, bool use_cond,
+                           float* r32, StepAccum* acc, bool df, int sms, int test, bool use_cond,
                            cudaGraphConditionalHandle h) {
   const int uc = use_cond ? 1 : 0;
-  const int rows = defect_rows(df, sm_count(), [&](int r) { return defect_blocks(nx, ny, df, r); });
+  const int rows = defect_rows(df, sms, [&](int r) { return defect_blocks(nx, ny, df, r); });
   const int c = defect_cols(df), r = DEFECT_WARPS * rows;
   const dim3 g((nx + c - 1) / c, (ny + r - 1) / r), t(32 * DEFECT_WARPS);
   // the pass that updates follows the smoother that writes e
@@ -1749,7 +1741,7 @@ void mg_vcycle_on(Engine& e, const float* b0, bool zero_start, StepAccum* acc) {
     a.cnx = C.nx;
     a.cny = C.ny;
     a.x_is_zero = l > 0 || zero_start;
-    launch_smooth(s, a, e.prm.mg_pre, MODE_PRE, l > 0);
+    launch_smooth(s, a, e.prm.mg_pre, MODE_PRE, l > 0, e.sms);
     prof_end(e, tok, (l == 0 ? 13.0 : 9.0) * cells(l) + 4.0 * cells(l + 1), 1);
   }
   {
@@ -1780,7 +1772,7 @@ void mg_vcycle_on(Engine& e, const float* b0, bool zero_start, StepAccum* acc) {
     a.cnx = C.nx;
     a.cny = C.ny;
     a.acc = l == 0 ? acc : nullptr;
-    launch_smooth(s, a, e.prm.mg_post, MODE_POST, true);
+    launch_smooth(s, a, e.prm.mg_post, MODE_POST, true, e.sms);
     prof_end(e, tok, 13.0 * cells(l) + 4.0 * cells(l + 1), 1);
   }
 }
@@ -2125,7 +2117,7 @@ BatchSolve* batch_solve_create(const std::vector<Engine*>& es_in, std::string& w
       regions(k, l, halo, 64, &gx, &gy);
       total += (long)gx * gy;
     }
-    b->small[ph] = total < SMOOTH_SMALL;
+    b->small[ph] = total < smooth_small(b->sms);
   }
   auto smooth_items = [&](int ph, int k) {
     int halo, gx, gy;
