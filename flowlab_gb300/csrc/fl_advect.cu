@@ -55,11 +55,10 @@ __device__ __forceinline__ float u_at_v_face(const float* __restrict__ u, int nx
 // MODE 1: MacCormack correction: `hat` is the forward result, `out` holds the
 //         stencil offsets and receives clamp(hat + 0.5*(in - reverse(hat)))
 //         (advect.ts:177-210).
-// Bound by instruction issue (70% active). Both launches of a MacCormack step
-// in a graph: 1024^2 32.2 us, 256^2 6.2; with the samplers' floor, index and
-// division as conversion and division instructions, the two faces one after
-// the other and backtraced positions handed over in buffers of their own 47.1
-// and 9.6 (20.4 M warp instructions a correction against 16.4 M).
+// Bound by instruction issue (67% active) and the chains of gathers. Both
+// launches of a MacCormack step in a graph: 1024^2 32.2 us (47.1 with the
+// samplers' floor, index and division as conversion and division instructions
+// and the two faces one after the other), 256^2 6.2 (9.6).
 template <int MODE, class S>
 __device__ __forceinline__ void advect_faces(int nx, int ny, const S& h, const float* __restrict__ u_in,
                                              const float* __restrict__ v_in, const float* u_hat, const float* v_hat,

@@ -173,21 +173,18 @@ __device__ __forceinline__ float2 link_factors(int code) {
 //
 // Bound by instruction issue and, where a level has few regions, by the
 // latency of one region (load, 2 pairs half-sweeps of ~150 to 250 cycles,
-// residual). With x in shared memory instead (four loads, a store and a
-// barrier of 32 warps for every update, 4 cells a thread) the 1024^2 PRE
-// launch executed 8.9 M warp instructions, three quarters of them set-up.
-// Launches chained in a graph, before -> now: V(3,3) PRE from zero / POST at
-// 2048^2 44.3 / 45.8 -> 14.8 / 17.4 us, 1024^2 12.0 / 12.5 -> 5.8 / 6.2,
-// 512^2 4.5 / 4.7 -> 3.2 / 3.7, 256^2 3.4 / 3.5 -> 2.6 / 3.1, 64^2 2.9 / 3.1
-// -> 2.5 / 3.0; four SOR pairs at 1024^2 with obstacles 16.6 -> 8.9.
+// residual). Launches chained in a graph, with x in shared memory -> in
+// registers: V(3,3) PRE from zero / POST at 2048^2 44.3 / 45.8 -> 14.8 / 17.4
+// us, 1024^2 12.0 / 12.5 -> 5.8 / 6.2, 256^2 3.4 / 3.5 -> 2.6 / 3.1; four SOR
+// pairs at 1024^2 with obstacles 16.6 -> 8.9.
 //
 // The shapes: 8 warps of 8 rows (a 64 x 64 region) spend the fewest
 // instructions a cell; 16 warps of 2 rows (64 x 32) have the shortest chain
 // of updates a warp, for levels whose 64 x 64 regions would leave SMs idle or
-// give a few of them a second one (fewer than smooth_small, 176 on 152 SMs): PRE
-// at 512^2 (100 regions) 4.2 against 3.2 us, 640^2 (169) 4.9 against 4.2, 704^2 (196) 4.9
-// against 4.9, POST 5.4 against 5.8, 1024^2 (400) 6.1 against 7.7. 8 x 4 and
-// 16 x 4 lay between.
+// give a few of them a second one (fewer than smooth_small: 176 on 152 SMs).
+// PRE in the large and the small regions: 512^2 (100 regions) 4.2 against 3.2
+// us, 640^2 (169) 4.9 against 4.2, 704^2 (196) 4.9 against 4.9, 1024^2 (400) 6.1
+// against 7.7; POST at 704^2 5.4 against 5.8. 8 x 4 and 16 x 4 lay between.
 static long smooth_small(int sms) { return 22L * sms / 19; }
 
 template <int NW, int RW>
@@ -874,13 +871,12 @@ __global__ void __launch_bounds__(1024) k_tail_labels(TailLabels a, const int* o
 // squared norm of r accumulated: the finest level's part of a defect-
 // correction cycle (iterative refinement, solveMixed), in float64 or in
 // double-float pairs. A warp owns the interior columns of its lanes (the
-// first and last lane hold the halo) and RW rows; every load of its first rows is issued before any arithmetic,
-// all but e's before the launch waits for the smoother that writes e (e is not
-// restrict: its loads must not move above that wait). Each p'
-// is formed once a warp and handed to its neighbours in registers (the rows
-// above and below) and by shuffles (left and right).
-//
-// (the rows a warp: defect_rows).
+// first and last lane hold the halo) and its rows (defect_rows); every load of
+// its first rows is issued before any arithmetic, all but e's before the launch
+// waits for the smoother that writes e (e is not restrict: its loads must not
+// move above that wait). Each p' is formed once a warp and handed to its
+// neighbours in registers (the rows above and below) and by shuffles (left and
+// right).
 constexpr int DEFECT_WARPS = 4;
 // Columns a block owns.
 __host__ __device__ constexpr int defect_cols(bool df) { return df ? 60 : 30; }
@@ -1534,8 +1530,8 @@ static long defect_blocks(int nx, int ny, bool df, int rows) {
 // an SM): 256^2 2 rows 6.2 us, 4 rows 7.1, 8 rows 9.3; 724^2 12.6 / 10.6 /
 // 11.3; 2048^2 57 / 42 / 36.
 // (Each after the POST launch it follows, that launch's time taken off, with
-// the cycle test; 8 rows unrolled and 4 warps a block before: float64 17.9 us
-// at 256^2, 27 at 1024^2, 94 at 2048^2; double-float 9.2, 13.8 and 49.)
+// the cycle test. The form before, 8 rows on every grid: float64 17.9 us at
+// 256^2, 94 at 2048^2; double-float 9.2 and 49.)
 template <class Blocks>
 static int defect_rows(bool df, int sms, Blocks blocks) {
   if (!df) return blocks(2) <= 2L * sms ? 2 : blocks(4) <= 26L * sms ? 4 : 8;
@@ -1690,9 +1686,6 @@ void mg_build_codes_if(Engine& e, cudaStream_t s, int* flag) {
 // into it for the tolerance test.
 void mg_vcycle(Engine& e, StepAccum* acc) { mg_vcycle_on(e, e.levels[0].b, false, acc); }
 
-// One V-cycle with level 0's rhs `b0`; with `zero_start` the level-0 unknown
-// starts from 0 (the correction equation of the defect-correction loop)
-// instead of the warm start in levels[0].x[0].
 // The threads of a frame's warps, at least 64.
 static int tail_threads(int frame) { return std::min(1024, std::max(64, frame * frame / 2)); }
 
@@ -1718,6 +1711,9 @@ static CoarseArgs coarse_args(const Engine& e, const float* b0, bool zero_start,
   return a;
 }
 
+// One V-cycle with level 0's rhs `b0`; with `zero_start` the level-0 unknown
+// starts from 0 (the correction equation of the defect-correction loop)
+// instead of the warm start in levels[0].x[0].
 void mg_vcycle_on(Engine& e, const float* b0, bool zero_start, StepAccum* acc) {
   cudaStream_t s = e.stream;
   const int lc = e.coarse_level;
