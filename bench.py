@@ -74,7 +74,10 @@ LIMITERS = {
 def phase_bytes_per_cell(prm, size, tail_side=32):
     """Algorithmic bytes per fine cell per LAUNCH of each phase's kernels:
     every array a pass must read or write counted once, float32 4 B, labels
-    1 B. A red-black half-sweep reads p (4), the rhs of its colour (2) and
+    1 B; a smoother launch counts its half-sweeps as the separate passes that
+    they are in the reference, although it moves each array once (the engine's
+    own count stands beside it: engine_bytes_per_launch, engine_frac). A
+    red-black half-sweep reads p (4), the rhs of its colour (2) and
     the labels (1) and writes its colour (2): 9 B, 18 per sweep pair. A
     V(3,3) finest level is then 3 x 18 + 11 (residual and restriction) on
     the way down and 10 (prolongation) + 3 x 18 on the way up. MacCormack
@@ -689,6 +692,7 @@ def run_ours(args, world, rank, local, pg):
         us = 1000.0 * r["ms"] / r["launches"]
         t = {"ms_per_step": r["ms"] / nsteps_prof, "launches_per_step": r["launches"] / nsteps_prof,
              "avg_launch_us": us, "engine_bytes_per_launch": r["gbytes"] * 1e9 / r["launches"]}
+        t["engine_frac"] = t["engine_bytes_per_launch"] / (us * 1e-6) / 1e9 / peak
         if n in per_cell:
             b = per_cell[n] * cells
             t["algorithmic_bytes_per_launch"] = b
@@ -706,7 +710,7 @@ def run_ours(args, world, rank, local, pg):
                 "frac": d["frac"], "peak_source": peak_kind, "traffic": None,
                 "algorithmic_bytes_per_launch": d["algorithmic_bytes_per_launch"],
                 "avg_launch_us": d["avg_launch_us"],
-                "engine_bytes_per_launch": d["engine_bytes_per_launch"],
+                "engine_bytes_per_launch": d["engine_bytes_per_launch"], "engine_frac": d["engine_frac"],
                 "limiter": LIMITERS.get(dom, "instruction issue (working set resident in L2)")}
     # Launches in the timed region: the profiled steps give the launches per
     # V-cycle (smoothers, coarse tail, float64 update, cycle test) and per
